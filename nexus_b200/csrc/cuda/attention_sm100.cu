@@ -41,6 +41,7 @@ struct AttnDev {
   int hfirst;          // TMA coordinate order, see load_tile
   float scale;
   int items, nqb;      // fwd (persistent): number of work items = nqb * H * B, q blocks per (head, batch)
+  const int4* blocks;  // fwd over packed sequences: q blocks (first row of the sequence, its rows, q0 inside it, -), nqb of them
   float* merge_o;      // fwd: FP32 [B,Tq,H,D] running output of earlier key/value chunks (in/out), or null
   float* merge_lse;    // fwd: FP32 [B,H,Tq] running log-sum-exp (in/out)
   float out_scale;     // fwd: factor of the written output (`out` only)
@@ -147,9 +148,9 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* tm, u
 }
 
 // Per-row visible key range [lo, hi] (inclusive) under the causal / window / length masks.
-__device__ __forceinline__ void row_limits(const AttnDev& p, int q, int& lo, int& hi) {
-  const int off = p.Tk - p.Tq;
-  hi = p.Tk - 1;
+__device__ __forceinline__ void row_limits(const AttnDev& p, int Tq, int Tk, int q, int& lo, int& hi) {
+  const int off = Tk - Tq;
+  hi = Tk - 1;
   lo = 0;
   if (p.causal) hi = min(hi, q + off);
   if (p.window > 0) lo = max(lo, q + off - p.window + 1);
@@ -250,11 +251,11 @@ __device__ __forceinline__ float half_softmax_store(uint32_t taddr, uint8_t* sP,
 __device__ __forceinline__ void softmax_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 // first/last (exclusive) kv index that any row in [q0, q0+nq) can see
-__device__ __forceinline__ void kv_range(const AttnDev& p, int q0, int nq, int& lo, int& hi) {
-  const int off = p.Tk - p.Tq;
-  hi = p.Tk;
+__device__ __forceinline__ void kv_range(const AttnDev& p, int Tq, int Tk, int q0, int nq, int& lo, int& hi) {
+  const int off = Tk - Tq;
+  hi = Tk;
   lo = 0;
-  if (p.causal) hi = min(p.Tk, q0 + nq - 1 + off + 1);
+  if (p.causal) hi = min(Tk, q0 + nq - 1 + off + 1);
   if (p.window > 0) lo = max(0, q0 + off - p.window + 1);
   if (hi < 0) hi = 0;
 }
@@ -278,15 +279,51 @@ constexpr int kFwdThreads = 320;  // warps 0-7: softmax (row quarter = warp & 3,
 // Work item i of the persistent forward kernel -> (q block, head, batch).  Items are ordered by cost: under
 // a causal mask the late q blocks see the most keys, so they come first and the CTAs (which take items
 // i, i + grid, i + 2 grid, ...) finish together.
-__device__ __forceinline__ void fwd_item(const AttnDev& p, int item, int& qb, int& h, int& b) {
+//
+// kPacked: the rows hold sequences one after another and a table names their q blocks, the most keys first.  One launch
+// then serves all prompts of a step: 32 prompts of up to 512 tokens, 12 heads of 64, took one launch per prompt before
+// (about 10 us of device time and 30 us of host time each, and no more than a few dozen busy SMs).
+struct FwdItem {
+  int q0, h, b;
+  int row0, Tq, Tk;  // first row of the sequence (0 unless packed), its lengths
+};
+template <bool kPacked>
+__device__ __forceinline__ FwdItem fwd_item(const AttnDev& p, int item) {
+  FwdItem w;
+  if (kPacked) {
+    const int4 blk = __ldg(p.blocks + item / p.H);
+    w.h = item % p.H;
+    w.b = 0;
+    w.row0 = blk.x;
+    w.Tq = w.Tk = blk.y;
+    w.q0 = blk.z;
+    return w;
+  }
   const int per = p.H * p.B;
-  qb = p.nqb - 1 - item / per;
   const int rem = item % per;
-  h = rem % p.H;
-  b = rem / p.H;
+  w.q0 = (p.nqb - 1 - item / per) * 128;
+  w.h = rem % p.H;
+  w.b = rem / p.H;
+  w.row0 = 0;
+  w.Tq = p.Tq;
+  w.Tk = p.Tk;
+  return w;
 }
 
-template <int HD, int EXT>  // row math: 0 plain, 1 soft-capping / ALiBi / dropout, 2 soft-capping alone (builds of their own)
+// Packed sequences: the last key tile of one runs on into the next one's rows.  Their scores are masked, but the zero
+// probabilities still meet their values in P V, and zero times an infinity of a neighbour would poison this sequence: row r
+// of the V tile (HD / 64 slabs of [128][64]) is cleared where it lies past the end.  Each of the `parts` threads of a row
+// clears its share of every slab's 128 bytes.
+template <int HD>
+__device__ __forceinline__ void clear_past_end(uint8_t* tile, int r, int rows, int part, int parts) {
+  if (r < rows) return;
+#pragma unroll
+  for (int s = 0; s < HD / 64; ++s)
+    for (int c = part * (8 / parts); c < (part + 1) * (8 / parts); ++c)
+      *reinterpret_cast<uint4*>(tile + s * 128 * 128 + r * 128 + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+template <int HD, int EXT, bool kPacked>  // EXT, row math: 0 plain, 1 soft-capping / ALiBi / dropout, 2 soft-capping alone
 __global__ void __launch_bounds__(kFwdThreads, (HD == 64 ? 2 : 1))
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const AttnDev p) {
@@ -347,16 +384,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       int n_item = 0, n_kv = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x, ++n_item) {
-        int qb, h, b;
-        fwd_item(p, item, qb, h, b);
+        const FwdItem w = fwd_item<kPacked>(p, item);
+        const int q0 = w.q0, h = w.h, b = w.b;
         const int hk = h / (p.H / p.Hkv);
-        const int q0 = qb * 128;
         int kv_lo, kv_hi;
-        kv_range(p, q0, min(128, p.Tq - q0), kv_lo, kv_hi);
+        kv_range(p, w.Tq, w.Tk, q0, min(128, w.Tq - q0), kv_lo, kv_hi);
         const int jb = kv_lo / 128, je = (kv_hi + 127) / 128;
         // debug builds: the item's tile coordinates lie inside the tensors (a tile may run past the end, never start there)
-        if (!NX_INDEX_OK(q0 >= 0 && q0 < p.Tq && h >= 0 && h < p.H && hk < p.Hkv && b >= 0 && b < p.B && jb >= 0 &&
-                         (je == jb || (je - 1) * 128 < p.Tk), p.status)) {
+        if (!NX_INDEX_OK(q0 >= 0 && q0 < w.Tq && h >= 0 && h < p.H && hk < p.Hkv && b >= 0 && b < p.B && jb >= 0 &&
+                         (je == jb || (je - 1) * 128 < w.Tk) && w.row0 >= 0 && w.row0 + w.Tk <= p.Tk, p.status)) {
           *abort_flag = 1;
           break;
         }
@@ -365,7 +401,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           break;
         }
         mbar_arrive_expect_tx(q_full, C::kQBytes);
-        load_tile<HD>(sQ, &tm_q, q_full, 128, q0, h, b, p.hfirst);
+        load_tile<HD>(sQ, &tm_q, q_full, 128, w.row0 + q0, h, b, p.hfirst);
         for (int j = jb; j < je; ++j, ++n_kv) {
           const int s = n_kv & 1;
           if (!mbar_wait_bounded(&kv_empty[s], ((n_kv >> 1) & 1) ^ 1u, abort_flag)) {
@@ -374,8 +410,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             break;
           }
           mbar_arrive_expect_tx(&kv_full[s], 2 * C::kKVBytes);
-          load_tile<HD>(sK + s * C::kKVBytes, &tm_k, &kv_full[s], 128, j * 128, hk, b, p.hfirst);
-          load_tile<HD>(sV + s * C::kKVBytes, &tm_v, &kv_full[s], 128, j * 128, hk, b, p.hfirst);
+          load_tile<HD>(sK + s * C::kKVBytes, &tm_k, &kv_full[s], 128, w.row0 + j * 128, hk, b, p.hfirst);
+          load_tile<HD>(sV + s * C::kKVBytes, &tm_v, &kv_full[s], 128, w.row0 + j * 128, hk, b, p.hfirst);
         }
       }
     }
@@ -389,11 +425,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       int n_item = 0, n_kv = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x, ++n_item) {
-        int qb, h, b;
-        fwd_item(p, item, qb, h, b);
-        const int q0 = qb * 128;
+        const FwdItem w = fwd_item<kPacked>(p, item);
         int kv_lo, kv_hi;
-        kv_range(p, q0, min(128, p.Tq - q0), kv_lo, kv_hi);
+        kv_range(p, w.Tq, w.Tk, w.q0, min(128, w.Tq - w.q0), kv_lo, kv_hi);
         const int jb = kv_lo / 128, je = (kv_hi + 127) / 128;
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(q_full, n_item & 1, abort_flag))) {
           if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
@@ -448,16 +482,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     int n_kv = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
-      int qb, h, b;
-      fwd_item(p, item, qb, h, b);
-      const int q0 = qb * 128;
+      const FwdItem w = fwd_item<kPacked>(p, item);
+      const int q0 = w.q0, h = w.h, b = w.b;
       const int q = q0 + r;
       int kv_lo, kv_hi;
-      kv_range(p, q0, min(128, p.Tq - q0), kv_lo, kv_hi);
+      kv_range(p, w.Tq, w.Tk, q0, min(128, w.Tq - q0), kv_lo, kv_hi);
       const int jb = kv_lo / 128, je = (kv_hi + 127) / 128;
       float m_run = -INFINITY, l_run = 0.0f;  // l_run: partial sum over this thread's columns
       int row_lo, row_hi;
-      row_limits(p, q, row_lo, row_hi);
+      row_limits(p, w.Tq, w.Tk, q, row_lo, row_hi);
       const ScoreExt ext = EXT != 0 ? make_ext(p, h, b) : ScoreExt{};
       float o_acc[HH];
 #pragma unroll
@@ -471,8 +504,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         tc_fence_after_sync();
         // does this tile need per-element masking?  (uniform over the CTA by construction of the bounds)
-        const int off = p.Tk - p.Tq;
-        const bool need_mask = (k0 + 128 > p.Tk) || (p.causal && (k0 + 127 > q0 + off)) ||
+        const int off = w.Tk - w.Tq;
+        const bool need_mask = (k0 + 128 > w.Tk) || (p.causal && (k0 + 127 > q0 + off)) ||
                                (p.window > 0 && (k0 < q0 + 127 + off - p.window + 1));
         float mx, rs;
         const int qpos = q + off;
@@ -496,6 +529,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         else rs = half_softmax_store<false, EXT>(tmem_s + lane_addr, sP, r, c0, k0, row_lo, row_hi, sc, m_use, ext, qpos, off);
         l_run = l_run * alpha + rs;
         m_run = m_new;
+        if (kPacked && k0 + 128 > w.Tk) clear_past_end<HD>(sV + (n_kv & 1) * C::kKVBytes, r, w.Tk - k0, half, 2);
         fence_proxy_async_smem();  // generic-proxy writes of P -> visible to the tensor core's async proxy
         tc_fence_before_sync();
         __syncwarp();
@@ -527,7 +561,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       softmax_bar();
       if (half == 1) l_run = sX[r];
-      if (ok && q < p.Tq && p.merge_o != nullptr) {
+      if (!kPacked && ok && q < w.Tq && p.merge_o != nullptr) {
         // merge with the result of earlier key/value chunks: softmax over the union of the key sets
         const int64_t li = (static_cast<int64_t>(b) * p.H + h) * p.Tq + q;
         float* mo = p.merge_o + ((static_cast<int64_t>(b) * p.Tq + q) * p.H + h) * HD + half * HH;
@@ -556,10 +590,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         m_run = (den > 0.0f ? mm + logf(den) : -INFINITY) * kLog2e;
       }
       softmax_bar();  // every thread has read merge_lse / sX before they are written again
-      if (ok && q < p.Tq) {
+      if (ok && q < w.Tq) {
         const float inv = l_run > 0.0f ? p.out_scale / l_run : 0.0f;
         __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(b) * p.o_batch +
-                              static_cast<int64_t>(q) * p.o_row + static_cast<int64_t>(h) * p.o_head + half * HH;
+                              static_cast<int64_t>(w.row0 + q) * p.o_row + static_cast<int64_t>(h) * p.o_head + half * HH;
 #pragma unroll
         for (int g = 0; g < HH / 8; ++g) {
           uint4 w;
@@ -569,7 +603,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           w.w = pack_bf16x2(o_acc[8 * g + 6] * inv, o_acc[8 * g + 7] * inv);
           reinterpret_cast<uint4*>(orow)[g] = w;
         }
-        if (half == 0) {
+        if (!kPacked && half == 0) {
           const int64_t li = (static_cast<int64_t>(b) * p.H + h) * p.Tq + q;
           const float lse = l_run > 0.0f ? (m_run / kLog2e + logf(l_run)) : -INFINITY;
           if (p.lse) p.lse[li] = lse;
@@ -616,7 +650,7 @@ struct Fwd2Cfg {
   static constexpr int kSmem = 2 * kQBytes + kStages * 2 * kKVBytes + 256;
   static constexpr int kTmemCols = 512;
 };
-constexpr int kFwd2Threads = 320;  // warps 0-3: softmax A, 4-7: softmax B, 8: TMA, 9: MMA
+constexpr int kFwd2Threads = kFwdThreads;  // warps 0-3: softmax A, 4-7: softmax B, 8: TMA, 9: MMA
 
 // Work of one round of the persistent loop: CTA c takes item round * grid + c in even rounds and
 // round * grid + (grid - 1 - c) in odd ones, and the items are sorted by cost (late q blocks first under a causal
@@ -624,25 +658,38 @@ constexpr int kFwd2Threads = 320;  // warps 0-3: softmax A, 4-7: softmax B, 8: T
 struct PairWork {
   int q0, h, b;
   int jbA, jeA, jbB, jeB, jb, je;
+  int row0, Tq, Tk;  // as FwdItem
 };
+template <bool kPacked>
 __device__ __forceinline__ bool pair_work(const AttnDev& p, int round, PairWork& w) {
   const int G = static_cast<int>(gridDim.x), c = static_cast<int>(blockIdx.x);
   const int item = round * G + ((round & 1) ? (G - 1 - c) : c);
   if (item >= p.items) return false;
-  const int per = p.H * p.B;
-  const int qb = p.nqb - 1 - item / per;
-  const int rem = item % per;
-  w.h = rem % p.H;
-  w.b = rem / p.H;
-  w.q0 = qb * 256;
+  if (kPacked) {
+    const int4 blk = __ldg(p.blocks + item / p.H);
+    w.h = item % p.H;
+    w.b = 0;
+    w.row0 = blk.x;
+    w.Tq = w.Tk = blk.y;
+    w.q0 = blk.z;
+  } else {
+    const int per = p.H * p.B;
+    const int rem = item % per;
+    w.h = rem % p.H;
+    w.b = rem / p.H;
+    w.row0 = 0;
+    w.Tq = p.Tq;
+    w.Tk = p.Tk;
+    w.q0 = (p.nqb - 1 - item / per) * 256;
+  }
   int lo, hi;
-  kv_range(p, w.q0, min(128, p.Tq - w.q0), lo, hi);
+  kv_range(p, w.Tq, w.Tk, w.q0, min(128, w.Tq - w.q0), lo, hi);
   w.jbA = lo / 128;
   w.jeA = (hi + 127) / 128;
   if (w.jeA <= w.jbA) w.jbA = w.jeA = 0;
   w.jbB = w.jeB = 0;
-  if (w.q0 + 128 < p.Tq) {
-    kv_range(p, w.q0 + 128, min(128, p.Tq - w.q0 - 128), lo, hi);
+  if (w.q0 + 128 < w.Tq) {
+    kv_range(p, w.Tq, w.Tk, w.q0 + 128, min(128, w.Tq - w.q0 - 128), lo, hi);
     w.jbB = lo / 128;
     w.jeB = (hi + 127) / 128;
     if (w.jeB <= w.jbB) w.jbB = w.jeB = 0;
@@ -654,7 +701,7 @@ __device__ __forceinline__ bool pair_work(const AttnDev& p, int round, PairWork&
   return true;
 }
 
-template <int HD>
+template <int HD, bool kPacked>
 __global__ void __launch_bounds__(kFwd2Threads, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const AttnDev p) {
@@ -711,10 +758,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       int nq[2] = {0, 0}, n_kv = 0;
       bool ok = true;
       PairWork w;
-      for (int round = 0; ok && pair_work(p, round, w); ++round) {
+      for (int round = 0; ok && pair_work<kPacked>(p, round, w); ++round) {
         const int hk = w.h / (p.H / p.Hkv);
-        if (!NX_INDEX_OK(w.q0 >= 0 && w.q0 < p.Tq && w.h < p.H && hk < p.Hkv && w.b < p.B && w.jb >= 0 &&
-                         (w.je == w.jb || (w.je - 1) * 128 < p.Tk), p.status)) {
+        if (!NX_INDEX_OK(w.q0 >= 0 && w.q0 < w.Tq && w.h < p.H && hk < p.Hkv && w.b < p.B && w.jb >= 0 &&
+                         (w.je == w.jb || (w.je - 1) * 128 < w.Tk) && w.row0 >= 0 && w.row0 + w.Tk <= p.Tk, p.status)) {
           *abort_flag = 1;
           break;
         }
@@ -729,7 +776,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           }
           ++nq[x];
           mbar_arrive_expect_tx(&q_full[x], C::kQBytes);
-          load_tile<HD>(sQ + x * C::kQBytes, &tm_q, &q_full[x], 128, w.q0 + x * 128, w.h, w.b, p.hfirst);
+          load_tile<HD>(sQ + x * C::kQBytes, &tm_q, &q_full[x], 128, w.row0 + w.q0 + x * 128, w.h, w.b, p.hfirst);
         }
         for (int j = w.jb; ok && j < w.je; ++j, ++n_kv) {
           const int s = n_kv % S;
@@ -739,8 +786,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             break;
           }
           mbar_arrive_expect_tx(&kv_full[s], 2 * C::kKVBytes);
-          load_tile<HD>(sK + s * C::kKVBytes, &tm_k, &kv_full[s], 128, j * 128, hk, w.b, p.hfirst);
-          load_tile<HD>(sV + s * C::kKVBytes, &tm_v, &kv_full[s], 128, j * 128, hk, w.b, p.hfirst);
+          load_tile<HD>(sK + s * C::kKVBytes, &tm_k, &kv_full[s], 128, w.row0 + j * 128, hk, w.b, p.hfirst);
+          load_tile<HD>(sV + s * C::kKVBytes, &tm_v, &kv_full[s], 128, w.row0 + j * 128, hk, w.b, p.hfirst);
         }
       }
     }
@@ -753,7 +800,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     int nqA = 0, nqB = 0, npA = 0, npB = 0, n_kv = 0;
     bool ok = true;
     PairWork w;
-    for (int round = 0; ok && pair_work(p, round, w); ++round) {
+    for (int round = 0; ok && pair_work<kPacked>(p, round, w); ++round) {
       if (w.jeA > w.jbA) {
         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&q_full[0], nqA & 1, abort_flag));
         ++nqA;
@@ -826,23 +873,26 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tmem_s = tmem_base + x * 128 + lane_addr, tmem_o = tmem_base + 256 + x * 128 + lane_addr;
     const float sc = p.scale * kLog2e;
-    const int off = p.Tk - p.Tq;
     int cnt = 0;  // key tiles this group has processed: phase counter of s_full / o_done
+    int kv0 = 0, kv_next = 0;  // key tiles of the earlier items: key tile j of this one sits in stage (kv0 + j - jb) % S
     bool ok = true;
     PairWork w;
-    for (int round = 0; ok && pair_work(p, round, w); ++round) {
+    for (int round = 0; ok && pair_work<kPacked>(p, round, w); ++round) {
+      kv0 = kv_next;
+      kv_next += w.je - w.jb;
       const int jbx = x == 0 ? w.jbA : w.jbB, jex = x == 0 ? w.jeA : w.jeB;
+      const int off = w.Tk - w.Tq;
       if (jex <= jbx) {
         // no visible key for any row of this tile: rows that exist get zeros and -inf (nothing to merge either)
         const int q0x = w.q0 + x * 128, q = q0x + r;
-        if (q < p.Tq && q0x < p.Tq) {
+        if (q < w.Tq && q0x < w.Tq) {
           __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(w.b) * p.o_batch +
-                                static_cast<int64_t>(q) * p.o_row + static_cast<int64_t>(w.h) * p.o_head;
+                                static_cast<int64_t>(w.row0 + q) * p.o_row + static_cast<int64_t>(w.h) * p.o_head;
           const int64_t li = (static_cast<int64_t>(w.b) * p.H + w.h) * p.Tq + q;
-          if (p.merge_o == nullptr) {
+          if (kPacked || p.merge_o == nullptr) {
 #pragma unroll
             for (int g = 0; g < HD / 8; ++g) reinterpret_cast<uint4*>(orow)[g] = make_uint4(0u, 0u, 0u, 0u);
-            if (p.lse) p.lse[li] = -INFINITY;
+            if (!kPacked && p.lse) p.lse[li] = -INFINITY;
           } else {
             const float* mo = p.merge_o + ((static_cast<int64_t>(w.b) * p.Tq + q) * p.H + w.h) * HD;
 #pragma unroll
@@ -863,7 +913,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int q0 = w.q0 + x * 128;
       const int q = q0 + r;
       int row_lo, row_hi;
-      row_limits(p, q, row_lo, row_hi);
+      row_limits(p, w.Tq, w.Tk, q, row_lo, row_hi);
       float m_ref = -INFINITY, l_run = 0.0f;
       for (int j = jbx; j < jex; ++j, ++cnt) {
         const int k0 = j * 128;
@@ -879,7 +929,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) tmem_ld_32x32b_x32(tmem_s + cc * 32, sv[cc]);
         tmem_ld_wait();
-        const bool need_mask = (k0 + 128 > p.Tk) || (p.causal && (k0 + 127 > q0 + off)) ||
+        const bool need_mask = (k0 + 128 > w.Tk) || (p.causal && (k0 + 127 > q0 + off)) ||
                                (p.window > 0 && (k0 < q0 + 127 + off - p.window + 1));
         const int clo = row_lo - k0, chi = row_hi - k0;  // column c is visible iff clo <= c <= chi
         if (need_mask) {
@@ -949,6 +999,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           tmem_st_32x32b_x16(tmem_s + cc * 16, pk);  // two probabilities per column
         }
         l_run += (r0 + r1) + (r2 + r3);
+        if (kPacked && k0 + 128 > w.Tk) {  // both groups clear the whole tail of the shared tile, each before its own P V
+          clear_past_end<HD>(sV + ((kv0 + j - w.jb) % S) * C::kKVBytes, r, w.Tk - k0, 0, 1);
+          fence_proxy_async_smem();
+        }
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
@@ -972,10 +1026,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         for (int c = 0; c < 32; ++c) o_acc[cc * 32 + c] = __uint_as_float(ov[c]);
       }
       tc_fence_before_sync();
-      if (q < p.Tq) {
+      if (q < w.Tq) {
         const int64_t li = (static_cast<int64_t>(w.b) * p.H + w.h) * p.Tq + q;
         float m_fin = m_ref;
-        if (p.merge_o != nullptr) {
+        if (!kPacked && p.merge_o != nullptr) {
           // merge with the result of earlier key/value chunks: softmax over the union of the key sets
           float* mo = p.merge_o + ((static_cast<int64_t>(w.b) * p.Tq + q) * p.H + w.h) * HD;
           const float lse_new = l_run > 0.0f ? (m_ref / kLog2e + logf(l_run)) : -INFINITY;
@@ -1004,7 +1058,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         const float inv = l_run > 0.0f ? p.out_scale / l_run : 0.0f;
         __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(w.b) * p.o_batch +
-                              static_cast<int64_t>(q) * p.o_row + static_cast<int64_t>(w.h) * p.o_head;
+                              static_cast<int64_t>(w.row0 + q) * p.o_row + static_cast<int64_t>(w.h) * p.o_head;
 #pragma unroll
         for (int g = 0; g < HD / 8; ++g) {
           uint4 wv;
@@ -1014,6 +1068,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           wv.w = pack_bf16x2(o_acc[8 * g + 6] * inv, o_acc[8 * g + 7] * inv);
           reinterpret_cast<uint4*>(orow)[g] = wv;
         }
+        if (kPacked) continue;
         const float lse = l_run > 0.0f ? (m_fin / kLog2e + logf(l_run)) : -INFINITY;
         if (p.lse) p.lse[li] = lse;
         if (p.merge_lse) p.merge_lse[li] = lse;
@@ -1398,7 +1453,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const int q0 = qb * 128;
 
   int kv_lo, kv_hi;
-  kv_range(p, q0, min(128, p.Tq - q0), kv_lo, kv_hi);
+  kv_range(p, p.Tq, p.Tk, q0, min(128, p.Tq - q0), kv_lo, kv_hi);
   const int jb = kv_lo / 64;
   const int je = kv_hi > kv_lo ? (kv_hi + 63) / 64 : jb;
   const int iters = je - jb;
@@ -1524,7 +1579,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       p.dsum_out[sidx] = dsum;
     }
     int row_lo, row_hi;
-    row_limits(p, q, row_lo, row_hi);
+    row_limits(p, p.Tq, p.Tk, q, row_lo, row_hi);
     if (q >= p.Tq) row_lo = 0x3fffffff;
     constexpr bool ext_on = EXT;
     const ScoreExt ext = EXT ? make_ext(p, h, b) : ScoreExt{};
@@ -1732,10 +1787,10 @@ extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
   do {                                                                                              \
     static bool once = false;                                                                       \
     if (!once) {                                                                                    \
-      if (set_smem(attn_fwd2_kernel<HD_>, Fwd2Cfg<HD_>::kSmem)) return -2;                          \
+      if (set_smem(attn_fwd2_kernel<HD_, false>, Fwd2Cfg<HD_>::kSmem)) return -2;                          \
       once = true;                                                                                  \
     }                                                                                               \
-    attn_fwd2_kernel<HD_><<<grid2, kFwd2Threads, Fwd2Cfg<HD_>::kSmem, st>>>(tq, tk, tv, p);         \
+    attn_fwd2_kernel<HD_, false><<<grid2, kFwd2Threads, Fwd2Cfg<HD_>::kSmem, st>>>(tq, tk, tv, p);         \
   } while (0)
     if (HD == 64) NX_FWD2(64);
     else NX_FWD2(128);
@@ -1746,10 +1801,10 @@ extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
   do {                                                                                              \
     static bool once = false;                                                                       \
     if (!once) {                                                                                    \
-      if (set_smem(attn_fwd_kernel<HD_, EXT_>, FwdCfg<HD_>::kSmem)) return -2;                      \
+      if (set_smem(attn_fwd_kernel<HD_, EXT_, false>, FwdCfg<HD_>::kSmem)) return -2;                      \
       once = true;                                                                                  \
     }                                                                                               \
-    attn_fwd_kernel<HD_, EXT_><<<grid, kFwdThreads, FwdCfg<HD_>::kSmem, st>>>(tq, tk, tv, p);       \
+    attn_fwd_kernel<HD_, EXT_, false><<<grid, kFwdThreads, FwdCfg<HD_>::kSmem, st>>>(tq, tk, tv, p);       \
   } while (0)
   const int mode = !ext ? 0 : (p.alibi == nullptr && p.dropout_p <= 0.0f && p.scale > 0.0f ? 2 : 1);
   if (HD == 64) {
@@ -1764,6 +1819,53 @@ extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
 #undef NX_FWD
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
+
+extern "C" int nx_attention_fwd_packed(const NxAttnArgs* a, const int32_t* blocks, int32_t count, nx_stream_t stream_) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream_);
+  if (check_args(a) || check_view(a->q) || check_view(a->k) || check_view(a->v) || check_view(a->o)) return -1;
+  if (a->batch != 1 || a->tq != a->tk || !a->causal || a->alibi_slopes != nullptr || a->dropout_p > 0.0f || a->merge_o != nullptr)
+    return -1;
+  if (a->softcap > 0.0f && !(a->scale > 0.0f)) return -1;
+  if (blocks == nullptr || count <= 0 || (reinterpret_cast<uintptr_t>(blocks) & 15)) return -1;
+  const int HD = a->head_dim;
+  CUtensorMap tq, tk, tv;
+  int rc;
+  if ((rc = make_map(&tq, a->q, a->tq, a->heads, 1, HD, 128))) return rc;
+  if ((rc = make_map(&tk, a->k, a->tk, a->kv_heads, 1, HD, 128))) return rc;
+  if ((rc = make_map(&tv, a->v, a->tk, a->kv_heads, 1, HD, 128))) return rc;
+  AttnDev p = base_params(a);
+  p.out = a->o.ptr;
+  p.o_row = a->o.row_stride;
+  p.o_head = a->o.head_stride;
+  p.blocks = reinterpret_cast<const int4*>(blocks);
+  p.nqb = count;
+  p.items = count * a->heads;
+  int sms = 0, dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return -2;
+#define NX_PACKED(KERN_, CFG_, PER_SM_)                                                             \
+  do {                                                                                              \
+    static bool once = false;                                                                       \
+    if (!once) {                                                                                    \
+      if (set_smem(KERN_, CFG_::kSmem)) return -2;                                                  \
+      once = true;                                                                                  \
+    }                                                                                               \
+    KERN_<<<std::min(p.items, sms * PER_SM_), kFwdThreads, CFG_::kSmem, st>>>(tq, tk, tv, p);       \
+  } while (0)
+  // the blocks are of nx_attention_packed_rows() query rows: two tiles where nx_attention_fwd takes the two-tile form too
+  const bool cap = p.softcap > 0.0f;
+  if (HD == 64) {
+    if (cap) NX_PACKED((attn_fwd_kernel<64, 2, true>), FwdCfg<64>, 2);
+    else NX_PACKED((attn_fwd_kernel<64, 0, true>), FwdCfg<64>, 2);
+  } else {
+    if (cap) NX_PACKED((attn_fwd_kernel<128, 2, true>), FwdCfg<128>, 1);
+    else NX_PACKED((attn_fwd2_kernel<128, true>), Fwd2Cfg<128>, 1);
+  }
+#undef NX_PACKED
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int nx_attention_packed_rows(int32_t head_dim, float softcap) { return head_dim == 128 && !(softcap > 0.0f) ? 256 : 128; }
 
 extern "C" int nx_attention_bwd(const NxAttnArgs* a, nx_stream_t stream_) {
   cudaStream_t st = static_cast<cudaStream_t>(stream_);

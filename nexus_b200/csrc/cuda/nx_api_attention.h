@@ -40,6 +40,12 @@ typedef struct NxAttnArgs {
 } NxAttnArgs;
 
 int nx_attention_fwd(const NxAttnArgs* args, nx_stream_t stream);
+// Causal forward over packed sequences: q, k, v, o have batch 1 and `tq` == `tk` rows in all.  `blocks` (device, 16-byte
+// aligned): `count` query blocks {first row of the sequence, its rows, first query row of the block inside it, 0} of
+// nx_attention_packed_rows() rows (the last one of a sequence may be shorter), in the order they are to be started.  Takes
+// window, softcap and out_scale; no log-sum-exp is written.  Rows of no block are left alone.
+int nx_attention_fwd_packed(const NxAttnArgs* args, const int32_t* blocks, int32_t count, nx_stream_t stream);
+int nx_attention_packed_rows(int32_t head_dim, float softcap);
 int nx_attention_bwd(const NxAttnArgs* args, nx_stream_t stream);
 
 #ifdef __cplusplus

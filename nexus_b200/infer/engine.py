@@ -660,6 +660,9 @@ class Engine:
             x = self.wte[tok.long()] + self.wpe[pos.long()]
         bs = self.cfg.block_size
         dl = Hl * D
+        prompts = None
+        if self.fast and Hl and sum(kind == "flash" for kind, *_ in runs) > 1:   # all prompts of the step in one launch a layer
+            prompts = K.PackedBlocks([(r0, r1 - r0) for kind, r0, r1, _ in runs if kind == "flash"], N, D, device=self.dev)
         for l in range(nl):
             lw = self.layers[l]
             if Hl == 0:   # more ranks than heads: this rank only takes part in the all-reduce
@@ -677,10 +680,13 @@ class Engine:
             if self.fast:
                 I.kv_append(k, v, slot, self.k_cache[l], self.v_cache[l], k_scale=self.k_scale[l],
                             v_scale=self.v_scale[l], kv_kind=self.kv_kind)
+                if prompts is not None:
+                    K.attention_fwd_packed(q, k, v, prompts, out=att)
                 for kind, r0, r1, _ in runs:
                     if kind == "flash":
-                        K.attention_fwd(q[r0:r1].unsqueeze(0), k[r0:r1].unsqueeze(0), v[r0:r1].unsqueeze(0), causal=True,
-                                        out=att[r0:r1].unsqueeze(0))
+                        if prompts is None:
+                            K.attention_fwd(q[r0:r1].unsqueeze(0), k[r0:r1].unsqueeze(0), v[r0:r1].unsqueeze(0), causal=True,
+                                            out=att[r0:r1].unsqueeze(0))
                     else:
                         I.paged_attention(q[r0:r1], self.k_cache[l], self.v_cache[l], self.block_table, rseq[r0:r1],
                                           ctx_len[r0:r1], att[r0:r1], block_size=bs, kv_heads=Hl,

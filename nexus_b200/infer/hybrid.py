@@ -33,8 +33,6 @@ from .engine import Chunk, Engine, _Linear
 
 __all__ = ["HybridEngine"]
 
-FLASH_MIN = 128          # fresh prompts from this length on take the tcgen05 flash kernel where the head size allows it
-
 
 def _pad8(n: int) -> int:
     return (n + 7) // 8 * 8
@@ -261,6 +259,7 @@ class HybridEngine(Engine):
         self._stepped = M.Segments(table, 0, single.count + short.count, max(single.max_len, short.max_len),
                                    single.total + short.total)
         self._every = M.Segments(table, 0, first, max(g.max_len for g in groups), sum(g.total for g in groups))
+        self._packed: dict = {}        # blocks of the fresh prompts, per head size, window and cap
         prompt.plan(self, self._prompt_windows, self._prompt_slices)
         return self._body(dv[0], dv[1], dv[2], dv[3], dv[4], dv[5][:logit_rows], runs, nl)
 
@@ -297,21 +296,27 @@ class HybridEngine(Engine):
             M.paged_window_attention(q, *paged, single, splits=self._decode_splits(a, single.count), **kw)
         if not self._many.count:
             return
-        host = self._host_rows[self.INDEX_ROWS:]
-        flash = long_.count > 0 and a.dim == a.vdim and a.dim in (64, 128) and a.scale > 0 and self._many.count <= 64 and all(
-            int(host[1, j]) >= FLASH_MIN and int(host[2, j]) == 0 for j in range(single.count, single.count + self._many.count))
-        if not flash:
+        # fresh prompts take the tcgen05 flash kernel where the head size allows it, all of a step in one launch
+        fresh = self._fresh_prompts() if a.dim == a.vdim and a.dim in (64, 128) and a.scale > 0 else None
+        if not fresh:
             M.paged_window_attention(q, *paged, self._many, **kw)
             return
+        if short.count:
+            M.paged_window_attention(q, *paged, short, **kw)
+        n, key = proj.shape[0], (a.dim, a.window, a.softcap)
+        if key not in self._packed:
+            self._packed[key] = K.PackedBlocks(fresh, n, a.dim, window=a.window, softcap=a.softcap, device=self.dev)
         _, k0, v0 = self.layers[i]["off"][:3]
-        for j in range(single.count, single.count + self._many.count):
-            r0, n = int(host[0, j]), int(host[1, j])
-            rows = proj[r0: r0 + n]
-            K.attention_fwd(rows[:, off: off + a.heads * a.dim].view(1, n, a.heads, a.dim),
-                            rows[:, k0: k0 + a.kv_heads * a.dim].view(1, n, a.kv_heads, a.dim),
-                            rows[:, v0: v0 + a.kv_heads * a.vdim].view(1, n, a.kv_heads, a.vdim), causal=True,
-                            window=a.window, scale=a.scale, softcap=a.softcap, out_scale=out_scale,
-                            out=out[r0: r0 + n].view(1, n, a.heads, a.vdim))
+        K.attention_fwd_packed(q.view(n, a.heads, a.dim), proj[:, k0: k0 + a.kv_heads * a.dim].view(n, a.kv_heads, a.dim),
+                               proj[:, v0: v0 + a.kv_heads * a.vdim].view(n, a.kv_heads, a.vdim), self._packed[key],
+                               scale=a.scale, out_scale=out_scale, out=out.view(n, a.heads, a.vdim))
+
+    def _fresh_prompts(self):
+        """(first row, rows) of the step's long segments if every one starts at position 0."""
+        single, short, long_ = self._groups
+        host, first = self._host_rows[self.INDEX_ROWS:], single.count + short.count
+        segs = [[int(v) for v in host[:3, j]] for j in range(first, first + long_.count)]
+        return [(row0, n) for row0, n, pos in segs] if all(pos == 0 for _, _, pos in segs) else None
 
     def _conv(self, x, w, bias, tail) -> torch.Tensor:
         from ..ops import _mixers as M

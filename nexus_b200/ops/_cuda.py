@@ -564,6 +564,40 @@ def attention_fwd(q, k, v, *, causal=True, window=0, scale=None, out=None, merge
     return o, lse
 
 
+class PackedBlocks:
+    """Query blocks of causal sequences that lie one after another in the rows of a step, for `attention_fwd_packed`: built on the
+    host once per step and head size, read by every layer.  ``segments``: (first row, rows) of each sequence."""
+
+    def __init__(self, segments, rows: int, head_dim: int, *, window: int = 0, softcap: float = 0.0, device="cuda"):
+        size = lib().nx_attention_packed_rows(C.c_int32(head_dim), C.c_float(softcap))
+        back, blocks = window - 1 if window > 0 else rows, []
+        for row0, n in segments:
+            if row0 < 0 or n <= 0 or row0 + n > rows:
+                raise ValueError(f"packed attention: rows {row0}..{row0 + n} of {rows}")
+            blocks.extend((min(q0 + size, n) - max(0, q0 - back), row0, n, q0) for q0 in range(0, n, size))
+        blocks.sort(key=lambda b: -b[0])          # the most keys first: the CTAs finish together
+        self.rows, self.head_dim, self.window, self.softcap, self.count = rows, head_dim, window, softcap, len(blocks)
+        host = torch.tensor([(row0, n, q0, 0) for _, row0, n, q0 in blocks], dtype=torch.int32)
+        self.table = host.pin_memory().to(device, non_blocking=True)
+
+
+def attention_fwd_packed(q, k, v, blocks: PackedBlocks, *, out, scale=None, out_scale=1.0):
+    """Causal attention of each of the packed sequences over its own rows: q [rows, H, D], k / v [rows, Hkv, D] bf16 (strided views
+    allowed) into ``out``.  One launch for all of them; rows of no sequence are left alone."""
+    T, H, D = q.shape
+    if T != blocks.rows or k.shape[0] != T or v.shape[0] != T or out.shape[0] != T or D != blocks.head_dim:
+        raise ValueError("packed attention: the blocks were built for other rows")
+    a = AttnArgs()
+    a.q, a.k, a.v, a.o = (_view(t.unsqueeze(0)) for t in (q, k, v, out))
+    a.status = status_word(q.device).data_ptr()
+    a.batch, a.heads, a.kv_heads, a.tq, a.tk, a.head_dim = 1, H, k.shape[1], T, T, D
+    a.causal, a.window = 1, int(blocks.window)
+    a.scale = scale if scale is not None else D ** -0.5
+    a.softcap, a.out_scale = float(blocks.softcap), float(out_scale)
+    _check(lib().nx_attention_fwd_packed(C.byref(a), _p(blocks.table), C.c_int32(blocks.count), _stream()), "nx_attention_fwd_packed")
+    return out
+
+
 def attention_bwd(q, k, v, o, lse, d_o, *, causal=True, window=0, scale=None, dq=None, dk=None, dv=None,
                   softcap=0.0, alibi_slopes=None, dropout_p=0.0, dropout_seed=0, dropout_offset=0):
     B, Tq, H, D = q.shape

@@ -223,3 +223,43 @@ def test_two_tile_forward_forced_at_head_dim_64():
     env = dict(os.environ, NEXUS_B200_ATTN_FWD="2")
     out = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0 and "ok" in out.stdout, out.stderr[-2000:]
+
+
+@pytest.mark.parametrize("D,H,Hkv,window,softcap", [(64, 3, 3, 0, 0.0), (64, 4, 2, 100, 20.0), (128, 4, 1, 0, 0.0), (128, 2, 2, 150, 15.0)])
+def test_packed_sequences_are_apart(D, H, Hkv, window, softcap):
+    """Sequences that end inside, at and behind a tile's edge, a gap between two, and one of infinities beside finite ones."""
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(3)
+    lens, gap, bad = [1, 17, 127, 128, 129, 256, 257, 700, 40], 5, 5
+    starts = [sum(lens[:i]) + (gap if i > 3 else 0) for i in range(len(lens))]
+    rows = sum(lens) + gap
+    qkv = torch.randn(rows, (H + 2 * Hkv) * D, device="cuda").bfloat16()
+    q, k, v = (t.view(rows, -1, D) for t in qkv.split([H * D, Hkv * D, Hkv * D], 1))
+    v[starts[bad]: starts[bad] + lens[bad]] = float("inf")
+    k[starts[bad]: starts[bad] + lens[bad]] = float("nan")
+    out = torch.full((rows, H, D), 7.0, device="cuda", dtype=torch.bfloat16)
+    blocks = K.PackedBlocks(list(zip(starts, lens)), rows, D, window=window, softcap=softcap)
+    K.attention_fwd_packed(q, k, v, blocks, out=out, scale=0.11, out_scale=0.5)
+    K.check_status()
+    assert (out[sum(lens[:4]): sum(lens[:4]) + gap] == 7.0).all()
+    for i, (s, n) in enumerate(zip(starts, lens)):
+        if i == bad:
+            assert out[s: s + n].isnan().all()
+            continue
+        qs, ks, vs = (t[s: s + n].float().transpose(0, 1) for t in (q, k, v))
+        ks, vs = (t.repeat_interleave(H // Hkv, 0) for t in (ks, vs))
+        sc = qs @ ks.transpose(1, 2) * 0.11
+        if softcap:
+            sc = softcap * torch.tanh(sc / softcap)
+        at = torch.arange(n, device="cuda")
+        hide = (at[None] > at[:, None]) | ((at[None] <= at[:, None] - window) if window else False)
+        want = 0.5 * (sc.masked_fill(hide, float("-inf")).softmax(-1) @ vs).transpose(0, 1)
+        # BF16 probabilities and results: 2^-9 of sums of values up to about 4.5
+        assert (out[s: s + n].float() - want).abs().max() < 2e-2, n
+
+
+def test_packed_blocks_outside_the_rows_are_refused():
+    from nexus_b200.ops import _cuda as K
+    for segs in ([(0, 11)], [(-1, 4)], [(3, 0)], [(8, 3)]):
+        with pytest.raises(ValueError):
+            K.PackedBlocks(segs, 10, 64)
