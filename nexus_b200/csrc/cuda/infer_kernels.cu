@@ -630,34 +630,81 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, int64_t row_stride, c
 }
 
 // gated activation on [n, 2F] = [gate | up]: y = act(gate) * up;  act: 0 SiLU (SwiGLU), 1 GELU-tanh (GeGLU)
-__global__ void gated_fwd_kernel(const __nv_bfloat16* __restrict__ h, __nv_bfloat16* __restrict__ y, int64_t n, int F,
-                                 int act) {
-  NX_GRID_STRIDE(i, n * F) {
-    const int64_t r = i / F;
-    const int c = static_cast<int>(i % F);
-    const float g = __bfloat162float(h[r * 2 * F + c]), u = __bfloat162float(h[r * 2 * F + F + c]);
-    y[i] = __float2bfloat16_rn((act == 0 ? silu_f(g) : gelu_tanh_f(g)) * u);
+// Bound by memory: pieces of eight (16 bytes) where F and the addresses allow it, single elements otherwise.  At n = 4096,
+// F = 5632 (bytes: 21 and 36 us) single elements with a 64-bit division each took 73 us forward and 85 us backward, pieces take
+// 27 and 37 us.
+__device__ __forceinline__ float gated_value(float g, float u, int act) { return (act == 0 ? silu_f(g) : gelu_tanh_f(g)) * u; }
+__device__ __forceinline__ void gated_grad(float g, float u, float d, int act, float& dg, float& du) {
+  float a, da;
+  if (act == 0) {
+    const float sg = 1.0f / (1.0f + __expf(-g));
+    a = g * sg;
+    da = sg * (1.0f + g * (1.0f - sg));
+  } else {
+    a = gelu_tanh_f(g);
+    da = dgelu_tanh_f(g);
+  }
+  dg = d * u * da;
+  du = d * a;
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  return make_uint4(nx::pack_bf16x2(v[0], v[1]), nx::pack_bf16x2(v[2], v[3]), nx::pack_bf16x2(v[4], v[5]), nx::pack_bf16x2(v[6], v[7]));
+}
+template <bool kVec>
+__global__ void __launch_bounds__(256) gated_fwd_kernel(const __nv_bfloat16* __restrict__ h, __nv_bfloat16* __restrict__ y, int64_t n, int F,
+                                                        int act) {
+  if constexpr (kVec) {
+    const uint32_t per = static_cast<uint32_t>(F) >> 3, total = static_cast<uint32_t>(n) * per;  // the host keeps this in 31 bits
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
+      const uint32_t r = i / per, c = (i - r * per) * 8;
+      const __nv_bfloat16* p = h + static_cast<int64_t>(r) * 2 * F + c;
+      float g[8], u[8];
+      unpack8(*reinterpret_cast<const uint4*>(p), g);
+      unpack8(*reinterpret_cast<const uint4*>(p + F), u);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] = gated_value(g[j], u[j], act);
+      *reinterpret_cast<uint4*>(y + static_cast<int64_t>(i) * 8) = pack8(g);
+    }
+  } else {
+    NX_GRID_STRIDE(i, n * F) {
+      const int64_t r = i / F;
+      const int c = static_cast<int>(i % F);
+      y[i] = __float2bfloat16_rn(gated_value(__bfloat162float(h[r * 2 * F + c]), __bfloat162float(h[r * 2 * F + F + c]), act));
+    }
   }
 }
-__global__ void gated_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ dy,
-                                 __nv_bfloat16* __restrict__ dh, int64_t n, int F, int act) {
-  NX_GRID_STRIDE(i, n * F) {
-    const int64_t r = i / F;
-    const int c = static_cast<int>(i % F);
-    const float g = __bfloat162float(h[r * 2 * F + c]), u = __bfloat162float(h[r * 2 * F + F + c]);
-    const float d = __bfloat162float(dy[i]);
-    float a, da;
-    if (act == 0) {
-      const float sg = 1.0f / (1.0f + __expf(-g));
-      a = g * sg;
-      da = sg * (1.0f + g * (1.0f - sg));
-    } else {
-      a = gelu_tanh_f(g);
-      da = dgelu_tanh_f(g);
+template <bool kVec>
+__global__ void __launch_bounds__(256) gated_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ dy,
+                                                        __nv_bfloat16* __restrict__ dh, int64_t n, int F, int act) {
+  if constexpr (kVec) {
+    const uint32_t per = static_cast<uint32_t>(F) >> 3, total = static_cast<uint32_t>(n) * per;
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
+      const uint32_t r = i / per, c = (i - r * per) * 8;
+      const int64_t at = static_cast<int64_t>(r) * 2 * F + c;
+      float g[8], u[8], d[8];
+      unpack8(*reinterpret_cast<const uint4*>(h + at), g);
+      unpack8(*reinterpret_cast<const uint4*>(h + at + F), u);
+      unpack8(*reinterpret_cast<const uint4*>(dy + static_cast<int64_t>(i) * 8), d);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) gated_grad(g[j], u[j], d[j], act, g[j], u[j]);
+      *reinterpret_cast<uint4*>(dh + at) = pack8(g);
+      *reinterpret_cast<uint4*>(dh + at + F) = pack8(u);
     }
-    dh[r * 2 * F + c] = __float2bfloat16_rn(d * u * da);
-    dh[r * 2 * F + F + c] = __float2bfloat16_rn(d * a);
+  } else {
+    NX_GRID_STRIDE(i, n * F) {
+      const int64_t r = i / F;
+      const int c = static_cast<int>(i % F);
+      float dg, du;
+      gated_grad(__bfloat162float(h[r * 2 * F + c]), __bfloat162float(h[r * 2 * F + F + c]), __bfloat162float(dy[i]), act, dg, du);
+      dh[r * 2 * F + c] = __float2bfloat16_rn(dg);
+      dh[r * 2 * F + F + c] = __float2bfloat16_rn(du);
+    }
   }
+}
+// pieces of eight: whole ones, on 16 bytes, counted in 32 bits with room for the grid's stride
+bool gated_vec(const void* a, const void* b, const void* c, int64_t n, int F) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c);
+  return F % 8 == 0 && (at & 15) == 0 && n * (F / 8) < (int64_t{1} << 31);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -919,13 +966,21 @@ extern "C" int nx_rope(void* x, int64_t row_stride, const int32_t* positions, co
 
 extern "C" int nx_gated_fwd(const void* h, void* y, int64_t n, int F, int act, nx_stream_t stream) {
   if (n <= 0) return 0;
-  gated_fwd_kernel<<<blocks_for(n * F, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>((const __nv_bfloat16*)h, (__nv_bfloat16*)y, n, F, act);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const auto* hp = static_cast<const __nv_bfloat16*>(h);
+  auto* yp = static_cast<__nv_bfloat16*>(y);
+  if (gated_vec(h, y, y, n, F)) gated_fwd_kernel<true><<<blocks_for(n * (F / 8), 256), 256, 0, st>>>(hp, yp, n, F, act);
+  else gated_fwd_kernel<false><<<blocks_for(n * F, 256), 256, 0, st>>>(hp, yp, n, F, act);
   return launch_status();
 }
 
 extern "C" int nx_gated_bwd(const void* h, const void* dy, void* dh, int64_t n, int F, int act, nx_stream_t stream) {
   if (n <= 0) return 0;
-  gated_bwd_kernel<<<blocks_for(n * F, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>((const __nv_bfloat16*)h, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dh, n, F, act);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const auto *hp = static_cast<const __nv_bfloat16*>(h), *dp = static_cast<const __nv_bfloat16*>(dy);
+  auto* op = static_cast<__nv_bfloat16*>(dh);
+  if (gated_vec(h, dy, dh, n, F)) gated_bwd_kernel<true><<<blocks_for(n * (F / 8), 256), 256, 0, st>>>(hp, dp, op, n, F, act);
+  else gated_bwd_kernel<false><<<blocks_for(n * F, 256), 256, 0, st>>>(hp, dp, op, n, F, act);
   return launch_status();
 }
 

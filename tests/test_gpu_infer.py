@@ -285,3 +285,18 @@ def test_engine_quantised_modes(weights, kv):
     assert len(generate(eq, toks[:5], 6)) == 6
     if weights != "bf16":
         assert eq.weight_bytes() < e0.weight_bytes()
+
+
+@pytest.mark.parametrize("n,f", [(3, 7), (5, 8), (33, 1408), (2, 12)])
+@pytest.mark.parametrize("act", ["silu", "gelu"])
+def test_gated_pieces_and_single_elements(n, f, act):
+    K, I = _mods()
+    torch.manual_seed(4)
+    h, dy = torch.randn(n, 2 * f, device="cuda").bfloat16(), torch.randn(n, f, device="cuda").bfloat16()
+    hr = h.double().requires_grad_(True)
+    fn = torch.nn.functional.silu if act == "silu" else lambda t: torch.nn.functional.gelu(t, approximate="tanh")
+    want = fn(hr[:, :f]) * hr[:, f:]
+    want.backward(dy.double())
+    # BF16 results: half of the last of 8 bits is up to 2^-8 of the value; and 1e-6 of the factors (up to about 20)
+    for got, ref in ((I.gated_fwd(h, act), want), (I.gated_bwd(h, dy, act), hr.grad)):
+        assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all()
