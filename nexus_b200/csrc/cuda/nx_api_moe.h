@@ -26,6 +26,15 @@ int nx_moe_assign_groups(int32_t* expert, const int32_t* order, int tokens, int 
 // dgate[t, j] = dy[t] . expert_out[expert[t,j]][slot[t,j]]  (BF16 rows of d elements)
 int nx_moe_gate_grad(const void* dy, const void* expert_out, const int32_t* expert, const int32_t* slot, float* dgate,
                      int tokens, int k, int d, int capacity, nx_stream_t stream);
+// buf [experts, capacity, d] BF16: the rows from counts[e] on become zeros
+int nx_moe_clear_padding(const int32_t* counts, void* buf, int experts, int capacity, int d, nx_stream_t stream);
+// dsel[t, j] = gate (dgate - sum_j gate dgate); pieces [tokens][3][pitch] BF16, pitch a multiple of 8: the dense rows of dsel by
+// expert as three pieces whose sum is the FP32 value
+int nx_moe_router_delta(const float* gate, const float* dgate, const int32_t* expert, float* dsel, void* pieces, int tokens, int k,
+                        int experts, int pitch, nx_stream_t stream);
+// dx[t] = sum_j buf[expert_tj][slot_tj] (slot >= 0) + sum_j dsel[t, j] router[expert_tj]; buf, dx BF16, router BF16 or FP32 [experts, d]
+int nx_moe_input_grad(const void* buf, const void* router, int router_dtype, const int32_t* expert, const int32_t* slot,
+                      const float* dsel, void* dx, int tokens, int k, int d, int capacity, nx_stream_t stream);
 
 
 // Experts by token id, for all layers of a step in one launch.  Layer l: table [vocab, top] gives every token's experts;

@@ -210,17 +210,17 @@ class _MoeEpNcclFn(torch.autograd.Function):
         plan.to_owners((dyr.float() * g[:, None]).to(torch.bfloat16), ep.in_local.view(le * cap, d))
         dout = ep.view(ep.in_local)
         dact = K.gemm(dout, down, b_mn=True)
-        ddown = K.gemm(dout, act, a_mn=True, b_mn=True, out_dtype=torch.float32)
+        ddown = K.gemm(dout, act, a_mn=True, b_mn=True, out_dtype=down.dtype)
         dh = I.gated_bwd(h.view(le * cap, F2), dact.view(le * cap, F2 // 2), "silu").view(le, cap, F2)
         K.gemm(dh, up, b_mn=True, out=ep.view(ep.out_local))
-        dup = K.gemm(dh, buf, a_mn=True, b_mn=True, out_dtype=torch.float32)
+        dup = K.gemm(dh, buf, a_mn=True, b_mn=True, out_dtype=up.dtype)
         dxr = plan.from_owners(ep.out_local.view(le * cap, d))
         dx = torch.zeros((N, d), dtype=torch.float32, device=x.device)
         dx.index_add_(0, tok, dxr.float())
         inner = (gate * dgate).sum(-1, keepdim=True)
         dsel = gate * (dgate - inner)
         dlogits = torch.zeros((N, ep.E), dtype=torch.float32, device=x.device).scatter_add_(1, expert.long(), dsel)
-        return dx.to(torch.bfloat16), dlogits, dup.to(up.dtype), ddown.to(down.dtype), None
+        return dx.to(torch.bfloat16), dlogits, dup, ddown, None
 
 
 class _MoeEpFn(torch.autograd.Function):
@@ -266,10 +266,10 @@ class _MoeEpFn(torch.autograd.Function):
         ep.barrier()                                     # gate-scaled d(y) rows are with the owners; outputs were read
         dout = ep.view(ep.in_local)
         dact = K.gemm(dout, down, b_mn=True)                                            # [le, C, F]
-        ddown = K.gemm(dout, act, a_mn=True, b_mn=True, out_dtype=torch.float32)        # [le, d, F]
+        ddown = K.gemm(dout, act, a_mn=True, b_mn=True, out_dtype=down.dtype)        # [le, d, F]
         dh = I.gated_bwd(h.view(le * cap, F2), dact.view(le * cap, F2 // 2), "silu").view(le, cap, F2)
         K.gemm(dh, up, b_mn=True, out=ep.view(ep.out_local))                            # d(buf) [le, C, d]
-        dup = K.gemm(dh, buf, a_mn=True, b_mn=True, out_dtype=torch.float32)            # [le, 2F, d]
+        dup = K.gemm(dh, buf, a_mn=True, b_mn=True, out_dtype=up.dtype)            # [le, 2F, d]
         ep.barrier()                                     # input gradients complete on every owner
         dx = _combine(ep, ep.out_table, expert, slot, torch.ones_like(gate))
         ep.barrier()                                     # nobody reads the result buffers any more
@@ -277,7 +277,7 @@ class _MoeEpFn(torch.autograd.Function):
         inner = (gate * dgate).sum(-1, keepdim=True)
         dsel = gate * (dgate - inner)
         dlogits = torch.zeros((N, ep.E), dtype=torch.float32, device=x.device).scatter_add_(1, expert.long(), dsel)
-        return dx, dlogits, dup.to(up.dtype), ddown.to(down.dtype), None
+        return dx, dlogits, dup, ddown, None
 
 
 class MoeEpLayer(torch.nn.Module):

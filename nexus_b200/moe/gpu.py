@@ -41,11 +41,25 @@ def route(logits: torch.Tensor, k: int, capacity: int):
     return expert, gate, slot, counts, dropped
 
 
-def dispatch(x, expert, slot, E: int, capacity: int, row_scale=None) -> torch.Tensor:
-    """Rows of x [N, d] (BF16) -> zero-padded buffers [E, capacity, d]."""
+def router_logits(x, router_w) -> torch.Tensor:
+    """FP32 logits.  BF16 rows and weights: their products are exact in the tensor cores' FP32 sums; a wider router takes FP32 throughout."""
+    if x.dtype == router_w.dtype == torch.bfloat16 and x.stride(-1) == router_w.stride(-1) == 1 and \
+            all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (x, router_w)):
+        return K.gemm(x, router_w, out_dtype=torch.float32)
+    return x.float() @ router_w.float().t()
+
+
+def dispatch(x, expert, slot, E: int, capacity: int, row_scale=None, counts=None) -> torch.Tensor:
+    """Rows of x [N, d] (BF16) -> zero-padded buffers [E, capacity, d].  ``counts`` [E]: the rows that each expert's tokens fill,
+    from the first on; only the rest is cleared."""
     N, d = x.shape
     k = expert.shape[1]
-    buf = torch.zeros((E, capacity, d), dtype=torch.bfloat16, device=x.device)
+    if counts is None:
+        buf = torch.zeros((E, capacity, d), dtype=torch.bfloat16, device=x.device)
+    else:
+        buf = torch.empty((E, capacity, d), dtype=torch.bfloat16, device=x.device)
+        K._check(K.lib().nx_moe_clear_padding(K._p(counts), K._p(buf), C.c_int(E), C.c_int(capacity), C.c_int(d), K._stream()),
+                 "nx_moe_clear_padding")
     tb = _one(buf)
     K._check(K.lib().nx_moe_dispatch(K._p(x), K._p(None), K._p(expert), K._p(slot), C.byref(tb), C.c_int(N * k),
                                      C.c_int(d), C.c_int(E), C.c_int(capacity), C.c_int(0), C.c_int(1),
@@ -68,21 +82,21 @@ class _MoeFn(torch.autograd.Function):
     def forward(ctx, x, router_w, up, down, k, capacity):
         N, d = x.shape
         E, F2, _ = up.shape
-        logits = x.float() @ router_w.float().t()
+        logits = router_logits(x, router_w)
         expert, gate, slot, counts, dropped = route(logits, k, capacity)
-        buf = dispatch(x, expert, slot, E, capacity)
+        buf = dispatch(x, expert, slot, E, capacity, counts=counts)
         h = K.gemm(buf, up)                                            # [E, C, 2F]
         act = I.gated_fwd(h.view(E * capacity, F2), "silu").view(E, capacity, F2 // 2)
         out = K.gemm(act, down)                                        # [E, C, d]
         y = combine(out, expert, slot, gate, E, capacity)
-        ctx.save_for_backward(x, router_w, up, down, expert, gate, slot, buf, h, act, out, logits)
+        ctx.save_for_backward(x, router_w, up, down, expert, gate, slot, buf, h, act, out, counts.clone())
         ctx.k, ctx.capacity = k, capacity
         ctx.mark_non_differentiable(counts, dropped)
         return y, counts, dropped
 
     @staticmethod
     def backward(ctx, dy, _c, _d):
-        x, router_w, up, down, expert, gate, slot, buf, h, act, out, logits = ctx.saved_tensors
+        x, router_w, up, down, expert, gate, slot, buf, h, act, out, counts = ctx.saved_tensors
         k, cap = ctx.k, ctx.capacity
         N, d = x.shape
         E, F2, _ = up.shape
@@ -90,21 +104,29 @@ class _MoeFn(torch.autograd.Function):
         dgate = torch.empty((N, k), dtype=torch.float32, device=x.device)
         K._check(K.lib().nx_moe_gate_grad(K._p(dy), K._p(out), K._p(expert), K._p(slot), K._p(dgate), C.c_int(N), C.c_int(k),
                                           C.c_int(d), C.c_int(cap), K._stream()), "nx_moe_gate_grad")
-        dout = dispatch(dy, expert, slot, E, cap, row_scale=gate.contiguous().view(-1))
+        dout = dispatch(dy, expert, slot, E, cap, row_scale=gate.contiguous().view(-1), counts=counts)
         dact = K.gemm(dout, down, b_mn=True)                           # [E, C, F]
-        ddown = K.gemm(dout, act, a_mn=True, b_mn=True, out_dtype=torch.float32)      # [E, d, F]
+        ddown = K.gemm(dout, act, a_mn=True, b_mn=True, out_dtype=down.dtype)         # [E, d, F]
         dh = I.gated_bwd(h.view(E * cap, F2), dact.view(E * cap, F2 // 2), "silu").view(E, cap, F2)
         dbuf = K.gemm(dh, up, b_mn=True)                               # [E, C, d]
-        dup = K.gemm(dh, buf, a_mn=True, b_mn=True, out_dtype=torch.float32)          # [E, 2F, d]
-        ones = torch.ones_like(gate)
-        dx = combine(dbuf, expert, slot, ones, E, cap).float()
+        dup = K.gemm(dh, buf, a_mn=True, b_mn=True, out_dtype=up.dtype)               # [E, 2F, d]
         # router: gate = softmax over the selected logits
-        inner = (gate * dgate).sum(-1, keepdim=True)
-        dsel = gate * (dgate - inner)
-        dlogits = torch.zeros_like(logits).scatter_add_(1, expert.long(), dsel)
-        drouter = dlogits.t() @ x.float()
-        dx = dx + dlogits @ router_w.float()
-        return dx.to(x.dtype), drouter.to(router_w.dtype), dup.to(up.dtype), ddown.to(down.dtype), None, None
+        pitch = (E + 7) // 8 * 8
+        dsel = torch.empty((N, k), dtype=torch.float32, device=x.device)
+        pieces = torch.empty((N, 3 * pitch), dtype=torch.bfloat16, device=x.device)
+        K._check(K.lib().nx_moe_router_delta(K._p(gate), K._p(dgate), K._p(expert), K._p(dsel), K._p(pieces), C.c_int(N), C.c_int(k),
+                                             C.c_int(E), C.c_int(pitch), K._stream()), "nx_moe_router_delta")
+        xc, router = x.contiguous(), router_w.contiguous()
+        drouter = K.gemm(pieces, xc, a_mn=True, b_mn=True, out_dtype=torch.float32, split_k=0, deterministic=True)
+        drouter = drouter.view(3, pitch, d)[:, :E].sum(0)
+        if router.dtype not in (torch.bfloat16, torch.float32):
+            router = router.float()
+        elif router.data_ptr() % 16:
+            router = router.clone()
+        dx = torch.empty((N, d), dtype=torch.bfloat16, device=x.device)
+        K._check(K.lib().nx_moe_input_grad(K._p(dbuf), K._p(router), C.c_int(K._DT[router.dtype]), K._p(expert), K._p(slot), K._p(dsel),
+                                           K._p(dx), C.c_int(N), C.c_int(k), C.c_int(d), C.c_int(cap), K._stream()), "nx_moe_input_grad")
+        return dx.to(x.dtype), drouter.to(router_w.dtype), dup, ddown, None, None
 
 
 def route_groups(select: torch.Tensor, k: int, capacity: int, groups: int = 1, reroute: bool = False):
@@ -170,10 +192,10 @@ class _MoeGroupsFn(torch.autograd.Function):
                                           C.c_int(d), C.c_int(cap), K._stream()), "nx_moe_gate_grad")
         dout = dispatch(dy, expert, slot, E, cap, row_scale=gate.contiguous().view(-1))
         dact = K.gemm(dout, down, b_mn=True)
-        ddown = K.gemm(dout, act, a_mn=True, b_mn=True, out_dtype=torch.float32)
+        ddown = K.gemm(dout, act, a_mn=True, b_mn=True, out_dtype=down.dtype)
         dh = I.gated_bwd(h.view(E * cap, F2), dact.view(E * cap, F2 // 2), "silu").view(E, cap, F2)
         dbuf = K.gemm(dh, up, b_mn=True)
-        dup = K.gemm(dh, buf, a_mn=True, b_mn=True, out_dtype=torch.float32)
+        dup = K.gemm(dh, buf, a_mn=True, b_mn=True, out_dtype=up.dtype)
         dx = combine(dbuf, expert, slot, torch.ones_like(gate), E, cap).float()
         inner = (gate * dgate).sum(-1, keepdim=True)
         dsel = gate * (dgate - inner)
@@ -185,7 +207,7 @@ class _MoeGroupsFn(torch.autograd.Function):
             dnl = dselect * eps * torch.sigmoid(nl)
             dnoise = (dnl.t() @ x.float()).to(noise_w.dtype)
             dx = dx + dnl @ noise_w.float()
-        return (dx.to(x.dtype), drouter.to(router_w.dtype), dnoise, dup.to(up.dtype), ddown.to(down.dtype),
+        return (dx.to(x.dtype), drouter.to(router_w.dtype), dnoise, dup, ddown,
                 None, None, None, None, None)
 
 

@@ -92,3 +92,38 @@ def test_moe_gpu_groups_reroute_and_noisy_router_match_the_cpu_core(groups, over
     assert rel(rg.grad.float().cpu(), rc.grad.t()) < 4e-2
     if noisy:
         assert rel(ng.grad.float().cpu(), nc.grad.t()) < 6e-2
+
+
+@pytest.mark.parametrize("N,d,E,k,cap,rdt", [(77, 72, 8, 1, 16, "bf16"), (301, 136, 10, 3, 40, "bf16"), (64, 128, 16, 8, 8, "f32"), (513, 264, 64, 2, 24, "bf16")])
+def test_moe_router_types_and_odd_sizes(N, d, E, k, cap, rdt):
+    """Experts that fill no multiple of eight, every expert over and under its capacity, BF16 and FP32 routers."""
+    from nexus_b200.moe import gpu as G
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(N)
+    F = 64
+    x = torch.randn(N, d, device="cuda").bfloat16().requires_grad_(True)
+    router = (torch.randn(E, d, device="cuda") * d ** -0.5).to(torch.bfloat16 if rdt == "bf16" else torch.float32).requires_grad_(True)
+    up = (torch.randn(E, 2 * F, d, device="cuda") * d ** -0.5).bfloat16().requires_grad_(True)
+    down = (torch.randn(E, d, F, device="cuda") * F ** -0.5).bfloat16().requires_grad_(True)
+    y, counts, dropped = G.moe_ffn(x, router, up, down, k, cap)
+    dy = torch.randn_like(y)
+    got = torch.autograd.grad(y, (x, router, up, down), dy)
+    K.check_status()
+    xr, rr, ur, dr = (t.detach().double().requires_grad_(True) for t in (x, router, up, down))
+    logits = xr @ rr.t()
+    val, idx = torch.sort(logits, dim=-1, descending=True, stable=True)
+    gate, idx = torch.softmax(val[:, :k], -1), idx[:, :k]
+    fill, want, kept = [0] * E, torch.zeros_like(xr), 0
+    for j in range(k):
+        for t, e in enumerate(idx[:, j].tolist()):
+            if fill[e] < cap:
+                fill[e] += 1
+                kept += 1
+                h = ur[e] @ xr[t]
+                want = want.index_add(0, torch.tensor([t], device="cuda"),
+                                      (gate[t, j] * (dr[e] @ (torch.nn.functional.silu(h[:F]) * h[F:])))[None])
+    assert counts.tolist() == fill and int(dropped) == N * k - kept
+    ref = (want, *torch.autograd.grad(want, (xr, rr, ur, dr), dy.double()))
+    # BF16 activations between the products: 2^-9 each over four roundings, with room for the router's cancelling sums
+    for g, r, name in zip((y, *got), ref, ("y", "dx", "drouter", "dup", "ddown")):
+        assert (g.double() - r).norm() <= 2e-2 * r.norm(), name
