@@ -76,6 +76,12 @@ int nx_cross_entropy_shifted_scaled(void* logits, int logits_dtype, const int32_
                                     int ignore_index, float smoothing, float z_loss, float grad_scale,
                                     const float* grad_scale_dev, int write_grad, nx_stream_t stream);
 
+// The same with the gradient written to `grad` [rows, ld] of the logits' type (it may be the logits): they are left as they are.
+int nx_cross_entropy_shifted_to(const void* logits, void* grad, int logits_dtype, const int32_t* tokens, const int32_t* targets,
+                                float* row_loss, void* ce_state, float* loss_out, float loss_weight, int accumulate_loss,
+                                int64_t rows, int seq_len, int vocab, int64_t ld, int ignore_index, float smoothing, float z_loss,
+                                float grad_scale, const float* grad_scale_dev, int write_grad, nx_stream_t stream);
+
 // ---- dropout / rng -----------------------------------------------------------------------------
 int nx_dropout(const void* in, void* out, int dtype, int64_t n, float p, uint64_t seed, uint64_t offset,
                int backward, nx_stream_t stream);
@@ -118,6 +124,16 @@ int nx_colsum(const void* dy, int dtype, float* out, float* scratch, int rows, i
 int nx_colsum_static_max_cols(void);
 int nx_colsum_static(const void* dy, int dtype, float* out, int rows, int cols, int64_t ld, int accumulate,
                      nx_stream_t stream);
+
+// ---- elementwise passes of the autograd operators ----------------------------------------------
+// out = dy * act'(x), n elements of BF16 or FP16; act: NX_ACT_GELU, NX_ACT_SILU or NX_ACT_RELU
+int nx_act_bwd(const void* x, const void* dy, void* out, int dtype, int64_t n, int act, nx_stream_t stream);
+// out = in * *factor (a device scalar), n elements of BF16 or FP32
+int nx_scale(const void* in, const float* factor, void* out, int dtype, int64_t n, nx_stream_t stream);
+// Rotate-half embedding of the first `heads` heads of BF16 rows of pitch ldx into rows of pitch ldy (they may be the same ones);
+// position of row r: r % seq_len; cos / sin FP32 [positions, half]; half and head_dim multiples of 8, columns past 2 * half are copied.
+int nx_rope_rows(const void* x, int64_t ldx, void* y, int64_t ldy, const float* cos_t, const float* sin_t, int rows, int seq_len,
+                 int heads, int head_dim, int half, int inverse, nx_stream_t stream);
 
 #ifdef __cplusplus
 }

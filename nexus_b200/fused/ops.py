@@ -79,27 +79,9 @@ class _FusedLinear(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        if ctx.act == "gelu":
-            pre = aux.float().requires_grad_(True)
-            with torch.enable_grad():
-                gelu_tanh(pre).backward(dy2.float())
-            dpre = pre.grad.to(dy2.dtype)
-        elif ctx.act in ("relu", "silu"):
-            pre = aux.float().requires_grad_(True)
-            with torch.enable_grad():
-                _act_fwd(pre, ctx.act).backward(dy2.float())
-            dpre = pre.grad.to(dy2.dtype)
-        else:
-            dpre = dy2
+        dpre = dy2 if ctx.act == "identity" else K.act_bwd(aux, dy2.to(aux.dtype), ctx.act)
         dx = K.gemm(dpre, w, b_mn=True).view(ctx.x_shape) if ctx.needs_input_grad[0] else None
-        dw = None
-        if ctx.needs_input_grad[1]:
-            rows = x2.shape[0]
-            if rows % 8 == 0:
-                dw = K.gemm(dpre, x2, a_mn=True, b_mn=True, out_dtype=torch.float32,
-                            split_k=max(1, min(8, rows // 2048))).to(w.dtype)
-            else:
-                dw = (dpre.float().t() @ x2.float()).to(w.dtype)
+        dw = K.weight_grad(dpre, x2, w.dtype) if ctx.needs_input_grad[1] else None
         db = K.colsum(dpre).to(w.dtype) if (ctx.has_bias and ctx.needs_input_grad[2]) else None
         return dx, dw, db, None
 
@@ -204,8 +186,8 @@ class _FusedNorm(torch.autograd.Function):
         xs, g, mean, rstd = ctx.saved_tensors
         dy2 = dy.reshape(-1, ctx.shape[-1]).contiguous()
         add = dsum.reshape(-1, ctx.shape[-1]).contiguous() if dsum is not None else None
-        dg = torch.zeros(ctx.shape[-1], dtype=torch.float32, device=dy.device)
-        db = torch.zeros(ctx.shape[-1], dtype=torch.float32, device=dy.device) if ctx.has_beta else None
+        dg = torch.empty(ctx.shape[-1], dtype=torch.float32, device=dy.device)
+        db = torch.empty(ctx.shape[-1], dtype=torch.float32, device=dy.device) if ctx.has_beta else None
         dx = K.norm_bwd(dy2, xs, g, None if ctx.rms else mean, rstd, rms=ctx.rms, add=add, dx_dtype=xs.dtype,
                         dgamma=dg, dbeta=db).view(ctx.shape)
         dgamma = dg.to(ctx.pdtypes[0])
@@ -322,6 +304,68 @@ def attention(q, k, v, causal=True, window=0, scale=None, softcap=0.0, alibi_slo
                                dropout_offset)
 
 
+class _QkvAttention(torch.autograd.Function):
+    """Causal attention on the packed rows [queries | keys | values] of a projection, with the rotary embedding of queries and keys:
+    one node, whose backward writes the three gradients into one packed tensor (as separate views each of them was a zeroed copy
+    of the whole, and these were added up)."""
+
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, heads, kv_heads, dim, window, softcap, alibi_slopes, dropout):
+        from ..ops import _cuda as K
+        B, T, W = qkv.shape
+        nq, nk = heads * dim, kv_heads * dim
+        qk = qkv
+        if cos is not None:
+            qk = torch.empty((B, T, nq + nk), dtype=qkv.dtype, device=qkv.device)
+            K.rope_rows(qkv.view(B * T, W), qk.view(B * T, nq + nk), cos, sin, seq_len=T, heads=heads + kv_heads, head_dim=dim)
+        q, k = qk[..., :nq].view(B, T, heads, dim), qk[..., nq: nq + nk].view(B, T, kv_heads, dim)
+        v = qkv[..., nq + nk:].view(B, T, kv_heads, dim)
+        kw = dict(causal=True, window=window, softcap=softcap, alibi_slopes=alibi_slopes, dropout_p=dropout[0], dropout_seed=dropout[1],
+                  dropout_offset=dropout[2])
+        o, lse = K.attention_fwd(q, k, v, **kw)
+        ctx.save_for_backward(q, k, v, o, lse, cos, sin)
+        ctx.kw = kw
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        from ..ops import _cuda as K
+        q, k, v, o, lse, cos, sin = ctx.saved_tensors
+        (B, T, H, D), Hk = q.shape, k.shape[2]
+        W = (H + 2 * Hk) * D
+        dqkv = torch.empty((B, T, W), dtype=q.dtype, device=q.device)
+        parts = dqkv.split([H * D, Hk * D, Hk * D], -1)
+        dq, dk, dv = (t.view(B, T, n, D) for t, n in zip(parts, (H, Hk, Hk)))
+        K.attention_bwd(q, k, v, o, lse, do.contiguous(), dq=dq, dk=dk, dv=dv, **ctx.kw)
+        if cos is not None:
+            rows = dqkv.view(B * T, W)
+            K.rope_rows(rows, rows, cos, sin, seq_len=T, heads=H + Hk, head_dim=D, inverse=True)
+        return (dqkv,) + (None,) * 9
+
+
+def qkv_attention_ok(qkv, dim: int, rope=None) -> bool:
+    """Whether `qkv_attention` takes these rows (and these tables [positions, half], FP32): CUDA BF16, head size 64 or 128."""
+    if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 3 and qkv.is_contiguous() and dim in (64, 128)
+            and qkv.numel() > 0 and qkv.data_ptr() % 16 == 0):
+        return False
+    if rope is None:
+        return _use_kernels(qkv)
+    cos, sin = rope
+    return (_use_kernels(qkv) and all(t.device == qkv.device and t.dtype == torch.float32 and t.is_contiguous() for t in (cos, sin))
+            and cos.shape == sin.shape and cos.shape[1] % 8 == 0 and 0 < 2 * cos.shape[1] <= dim and cos.shape[0] >= qkv.shape[1]
+            and not (cos.requires_grad or sin.requires_grad))
+
+
+def qkv_attention(qkv, heads: int, kv_heads: int, dim: int, rope=None, window=0, softcap=0.0, alibi_slopes=None, dropout_p=0.0,
+                  dropout_seed=0, dropout_offset=0):
+    """Causal attention of rows [B, T, (heads + 2 kv_heads) dim] that hold queries, keys and values side by side; ``rope``: (cos, sin)
+    tables for positions 0 .. T - 1.  See `qkv_attention_ok`.  Returns [B, T, heads, dim]."""
+    slopes = None if alibi_slopes is None else alibi_slopes.detach().float().contiguous().to(qkv.device)
+    cos, sin = rope if rope is not None else (None, None)
+    return _QkvAttention.apply(qkv, cos, sin, heads, kv_heads, dim, window, float(softcap), slopes,
+                               (float(dropout_p), int(dropout_seed), int(dropout_offset)))
+
+
 def attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k=None, causal=True, window=0, scale=None, softcap=0.0,
                      alibi_slopes=None, dropout_p=0.0, dropout_seed=0, dropout_offset=0):
     """Attention over a packed batch of variable-length sequences.
@@ -381,18 +425,24 @@ class _FusedCE(torch.autograd.Function):
             ctx.save_for_backward(work)
             return torch.tensor(loss, dtype=torch.float32)
         from ..ops import _cuda as K
-        work = logits.reshape(-1, logits.shape[-1]).clone()  # gradient is produced in place in this copy
+        flat = logits.reshape(-1, logits.shape[-1])
+        if flat.stride(1) != 1 or (flat.shape[0] > 1 and flat.stride(0) != flat.shape[1]):
+            flat = flat.contiguous()
+        work = torch.empty(flat.shape, dtype=flat.dtype, device=flat.device)  # the gradient; the logits stay as they are
         tk = tokens.to(torch.int32).contiguous() if tokens is not None else None
         tg = targets.to(torch.int32).contiguous().reshape(-1) if targets is not None else None
         T = tokens.shape[-1] if tokens is not None else 1
-        loss = K.cross_entropy_shifted(work, tk, targets=tg, vocab=vocab, ignore_index=ignore_index,
-                                       smoothing=smoothing, z_loss=z_loss, grad_scale=1.0, seq_len=T)
+        loss = K.cross_entropy_shifted(flat, tk, targets=tg, vocab=vocab, ignore_index=ignore_index,
+                                       smoothing=smoothing, z_loss=z_loss, grad_scale=1.0, seq_len=T, grad=work)
         ctx.save_for_backward(work)
         return loss.reshape(())
 
     @staticmethod
     def backward(ctx, dloss):
         (g,) = ctx.saved_tensors
+        if g.is_cuda:
+            from ..ops import _cuda as K
+            return K.scale(g, dloss.float()).to(ctx.dtype).view(ctx.shape), None, None, None, None, None, None
         return (g * dloss.to(g.dtype)).to(ctx.dtype).view(ctx.shape), None, None, None, None, None, None
 
 

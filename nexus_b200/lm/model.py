@@ -113,6 +113,13 @@ class Attention(nn.Module):
         B, T, _ = x.shape
         H, Hk, D = cfg.n_head, cfg.kv_heads(), cfg.hdim()
         qkv = self.qkv(x)
+        p_drop = cfg.attn_dropout if self.training else 0.0
+        seed, off = rng if rng is not None else (0, 0)
+        tables = None if rope is None else (rope.cos, rope.sin)
+        if self.q_norm is None and cache is None and positions is None and F_.qkv_attention_ok(qkv, D, tables):
+            o = F_.qkv_attention(qkv, H, Hk, D, tables, window=cfg.window, softcap=cfg.attn_softcap, alibi_slopes=slopes,
+                                 dropout_p=p_drop, dropout_seed=seed, dropout_offset=off)
+            return self.o(o.reshape(B, T, H * D))
         if H == Hk:
             qkv5 = qkv.view(B, T, 3, H, D)
             q, k, v = qkv5[:, :, 0], qkv5[:, :, 1], qkv5[:, :, 2]
@@ -127,8 +134,6 @@ class Attention(nn.Module):
             k = apply_rope(k, rope.cos, rope.sin, positions)
         if cache is not None:
             k, v = cache.append(k, v)
-        p_drop = cfg.attn_dropout if self.training else 0.0
-        seed, off = rng if rng is not None else (0, 0)
         o = F_.attention(q, k, v, causal=True, window=cfg.window, softcap=cfg.attn_softcap, alibi_slopes=slopes,
                          dropout_p=p_drop, dropout_seed=seed, dropout_offset=off)
         return self.o(o.reshape(B, T, H * D))

@@ -191,6 +191,57 @@ def auto_split_k(m: int, n: int, k: int, clusters: int = 74) -> int:
     return s
 
 
+def weight_split_k(m: int, n: int, k: int, clusters: int = 74) -> int:
+    """Number of K slices of a weight gradient [m, n] over k rows whose slices meet in a workspace: the cost of `auto_split_k` plus
+    the reduction pass (about 3 us, and 8 bytes of traffic per slice and element), in units of one 64-deep block of a 256 x 256
+    tile (0.39 us).  Slicing by the number of rows alone cost 146 us of reduction beside 147 us of product at 32000 x 2048 x 4096."""
+    key = (-m, n, k)
+    s = _split_cache.get(key)
+    if s is None:
+        tiles, kb = -(-m // 256) * -(-n // 256), -(-k // 64)
+        best, s = None, 1
+        for cand in range(1, min(16, kb) + 1):
+            per = -(-kb // cand)
+            cand = -(-kb // per)
+            cost = -(-tiles * cand // clusters) * (per + 6) + (0 if cand == 1 else 8 + cand * m * n * 8 / 2.0e6)
+            if best is None or cost < best:
+                best, s = cost, cand
+        _split_cache[key] = s
+    return s
+
+
+def weight_grad(dy, x, dtype) -> torch.Tensor:
+    """dy^T x for dy [rows, m], x [rows, n] in ``dtype``, summed in FP32 in a fixed order; any number of rows."""
+    out = dtype if dtype in (torch.bfloat16, torch.float32) else torch.float32
+    return gemm(dy, x, a_mn=True, b_mn=True, out_dtype=out, split_k=weight_split_k(dy.shape[1], x.shape[1], dy.shape[0]),
+                deterministic=True).to(dtype)
+
+
+def act_bwd(x, dy, act: str) -> torch.Tensor:
+    """dy * act'(x) for contiguous BF16 / FP16 tensors of one shape; ``act``: gelu (tanh form), silu or relu."""
+    out = torch.empty_like(x)
+    _check(lib().nx_act_bwd(_p(x), _p(dy), _p(out), C.c_int(_DT[x.dtype]), C.c_int64(x.numel()), C.c_int(ACT[act]), _stream()),
+           "nx_act_bwd")
+    return out
+
+
+def scale(x, factor) -> torch.Tensor:
+    """x * factor for a contiguous BF16 / FP32 tensor and an FP32 device scalar."""
+    out = torch.empty_like(x)
+    _check(lib().nx_scale(_p(x), _p(factor), _p(out), C.c_int(_DT[x.dtype]), C.c_int64(x.numel()), _stream()), "nx_scale")
+    return out
+
+
+def rope_rows(x, y, cos, sin, *, seq_len: int, heads: int, head_dim: int, inverse: bool = False) -> None:
+    """Rotate-half embedding of the first ``heads`` heads of the BF16 rows x [rows, >= heads * head_dim] into y (may be x); the
+    position of row r is ``r % seq_len``; cos / sin FP32 [positions, half]."""
+    if cos.shape[0] < min(seq_len, x.shape[0]):
+        raise ValueError("rope_rows: the tables are shorter than the sequences")
+    _check(lib().nx_rope_rows(_p(x), C.c_int64(x.stride(0)), _p(y), C.c_int64(y.stride(0)), _p(cos), _p(sin), C.c_int(x.shape[0]),
+                              C.c_int(seq_len), C.c_int(heads), C.c_int(head_dim), C.c_int(cos.shape[1]), C.c_int(int(inverse)),
+                              _stream()), "nx_rope_rows")
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          bias: Optional[torch.Tensor] = None, act: Optional[str] = None,
          aux_in: Optional[torch.Tensor] = None, aux_out: Optional[torch.Tensor] = None,
@@ -411,9 +462,9 @@ def embedding_bwd(tokens, dx, dwte, dwpe, batch, seq_len, deterministic=True):
 # ------------------------------------------------------------------------------------ cross-entropy
 def cross_entropy_shifted(logits, tokens, *, targets=None, vocab=None, ignore_index=-100, smoothing=0.0,
                           z_loss=0.0, grad_scale=1.0, write_grad=True, loss_out=None, loss_weight=1.0,
-                          accumulate_loss=False, seq_len=None, grad_scale_dev=None):
-    """In-place fused CE.  ``logits`` [rows, ld] becomes d(loss*grad_scale)/dlogits.  Returns the loss
-    tensor (1 element, device).  ``grad_scale_dev``: a 1-element FP32 device tensor that multiplies the gradient too
+                          accumulate_loss=False, seq_len=None, grad_scale_dev=None, grad=None):
+    """In-place fused CE.  ``logits`` [rows, ld] becomes d(loss*grad_scale)/dlogits, or ``grad`` (of the same layout and type)
+    does and the logits stay.  Returns the loss tensor (1 element, device).  ``grad_scale_dev``: a 1-element FP32 device tensor that multiplies the gradient too
     (the dynamic loss scale inside the optimizer state)."""
     L = lib()
     rows, ld = logits.shape[0], logits.stride(0)
@@ -423,12 +474,14 @@ def cross_entropy_shifted(logits, tokens, *, targets=None, vocab=None, ignore_in
     state = scratch(int(L.nx_ce_state_bytes()), "ce_state", logits.device)
     if loss_out is None:
         loss_out = torch.empty(1, dtype=torch.float32, device=logits.device)
-    _check(L.nx_cross_entropy_shifted_scaled(_p(logits), C.c_int(_DT[logits.dtype]), _p(tokens), _p(targets),
-                                             _p(row_loss), _p(state), _p(loss_out), C.c_float(loss_weight),
-                                             C.c_int(int(accumulate_loss)), C.c_int64(rows), C.c_int(T), C.c_int(vocab),
-                                             C.c_int64(ld), C.c_int(ignore_index), C.c_float(smoothing),
-                                             C.c_float(z_loss), C.c_float(grad_scale), _p(grad_scale_dev),
-                                             C.c_int(int(write_grad)), _stream()),
+    if grad is not None and (grad.shape != logits.shape or grad.stride(0) != ld or grad.dtype != logits.dtype):
+        raise ValueError("cross_entropy_shifted: the gradient needs the layout and type of the logits")
+    _check(L.nx_cross_entropy_shifted_to(_p(logits), _p(logits if grad is None else grad), C.c_int(_DT[logits.dtype]), _p(tokens),
+                                         _p(targets), _p(row_loss), _p(state), _p(loss_out), C.c_float(loss_weight),
+                                         C.c_int(int(accumulate_loss)), C.c_int64(rows), C.c_int(T), C.c_int(vocab),
+                                         C.c_int64(ld), C.c_int(ignore_index), C.c_float(smoothing),
+                                         C.c_float(z_loss), C.c_float(grad_scale), _p(grad_scale_dev),
+                                         C.c_int(int(write_grad)), _stream()),
            "nx_cross_entropy_shifted")
     return loss_out
 

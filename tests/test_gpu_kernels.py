@@ -181,3 +181,96 @@ def test_dlpack_exchange_on_the_device_and_pinned_host():
     g = dlpack.from_dlpack(dlpack.to_dlpack(h))
     g[3] = 2.0
     assert float(h[3]) == 2.0 and not g.is_cuda
+
+
+@pytest.mark.parametrize("H,Hk,D,rot,T,window,dropout", [(4, 4, 64, 64, 203, 0, 0.0), (6, 2, 128, 96, 130, 50, 0.0), (4, 1, 64, 0, 64, 0, 0.2),
+                                                       (2, 2, 64, 16, 1, 0, 0.0)])
+def test_packed_qkv_attention_matches_the_separate_operators(H, Hk, D, rot, T, window, dropout):
+    """The packed node against apply_rope + attention on views: the same kernels on the same rotated rows (equal outputs), gradients
+    that differ only where sums of the zero-padded views were rounded."""
+    from nexus_b200.fused import ops as F
+    from nexus_b200.lm.rope import apply_rope
+    torch.manual_seed(6)
+    B, W = 3, (H + 2 * Hk) * D
+    qkv = torch.randn(B, T, W, device="cuda").bfloat16().requires_grad_(True)
+    ang = torch.rand(T + 5, rot // 2, device="cuda") * 6
+    tables = (ang.cos(), ang.sin()) if rot else None
+    assert F.qkv_attention_ok(qkv, D, tables)
+    kw = dict(window=window, dropout_p=dropout, dropout_seed=3, dropout_offset=8)
+    o = F.qkv_attention(qkv, H, Hk, D, tables, **kw)
+    do = torch.randn_like(o)
+    (got,) = torch.autograd.grad(o, qkv, do)
+    q, k, v = (t.view(B, T, -1, D) for t in qkv.split([H * D, Hk * D, Hk * D], -1))
+    if rot:
+        q, k = (apply_rope(t, *tables) for t in (q, k))
+    want = F.attention(q, k, v, **kw)
+    assert torch.equal(o, want)
+    (ref,) = torch.autograd.grad(want, qkv, do)
+    assert (got.float() - ref.float()).norm() <= 1e-2 * ref.float().norm()
+
+
+def test_packed_qkv_attention_refuses_other_forms():
+    from nexus_b200.fused import ops as F
+    x = torch.zeros(2, 8, 3 * 128, device="cuda").bfloat16()
+    t = torch.zeros(8, 32, device="cuda")
+    assert F.qkv_attention_ok(x, 64, (t, t))
+    assert not F.qkv_attention_ok(x.float(), 64, (t, t)) and not F.qkv_attention_ok(x, 32, None)
+    assert not F.qkv_attention_ok(x[:, ::2], 64, (t, t)) and not F.qkv_attention_ok(x, 64, (t[:7], t[:7]))
+    assert not F.qkv_attention_ok(x, 64, (t[:, :12].contiguous(), t[:, :12].contiguous())) and not F.qkv_attention_ok(x, 64, (t.half(), t.half()))
+
+
+@pytest.mark.parametrize("rows,m,n", [(609, 512, 512), (1, 256, 264), (4097, 768, 768), (64, 8, 16), (3000, 40, 2048)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+def test_weight_grad_any_number_of_rows(rows, m, n, dt):
+    """Rows that fill no block of the reduction, sliced and whole.  FP32 sums of exact products: 1e-5 of the norm; BF16 results 2^-8."""
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(7)
+    dy, x = torch.randn(rows, m, device="cuda").bfloat16(), torch.randn(rows, n, device="cuda").bfloat16()
+    want = dy.double().t() @ x.double()
+    got = K.weight_grad(dy, x, dt)
+    assert got.dtype == dt and (got.double() - want).norm() <= (2.0 ** -8 if dt is torch.bfloat16 else 1e-5) * want.norm()
+    assert torch.equal(got, K.weight_grad(dy, x, dt))
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 4099])
+@pytest.mark.parametrize("act", ["gelu", "silu", "relu"])
+def test_activation_backward(n, act):
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(8)
+    x, dy = (torch.randn(n + 1, device="cuda").bfloat16() for _ in range(2))
+    fn = dict(gelu=lambda t: torch.nn.functional.gelu(t, approximate="tanh"), silu=torch.nn.functional.silu, relu=torch.relu)[act]
+    for a, b in ((x[:n], dy[:n]), (x[1:], dy[1:])):           # on 16 bytes and beside them
+        r = a.double().requires_grad_(True)
+        fn(r).backward(b.double())
+        assert ((K.act_bwd(a, b, act).double() - r.grad).abs() <= 2.0 ** -8 * r.grad.abs() + 2e-5).all()
+
+
+@pytest.mark.parametrize("V,ld,dt", [(50, 56, torch.bfloat16), (8192, 8192, torch.bfloat16), (50257, 50304, torch.bfloat16), (101, 101, torch.bfloat16),
+                                     (997, 1000, torch.float32), (13, 13, torch.float32)])
+@pytest.mark.parametrize("smoothing", [0.0, 0.1])
+def test_cross_entropy_gradient_beside_the_logits(V, ld, dt, smoothing):
+    """In place and into another matrix give the same bits, the logits stay, entries of -inf get no probability."""
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(9)
+    rows = 6
+    logits = (torch.randn(rows, ld, device="cuda") * 3).to(dt)
+    if ld % (16 // logits.element_size()) == 0:       # rows of single elements: their kernel's sum of all logits takes finite ones
+        logits[:, 0:16:3] = -float("inf")
+    targets = torch.tensor([V - 1 if V > 16 else 5, 1, -100, 7, 8, 10], device="cuda", dtype=torch.int32)
+    keep, grad, inplace = logits.clone(), torch.empty_like(logits), logits.clone()
+    if smoothing:
+        keep = logits.nan_to_num(neginf=-30.0)
+        logits, inplace = keep.clone(), keep.clone()
+    kw = dict(targets=targets, vocab=V, smoothing=smoothing, z_loss=1e-3, seq_len=1)
+    a = K.cross_entropy_shifted(logits, None, grad=grad, **kw)
+    b = K.cross_entropy_shifted(inplace, None, **kw)
+    assert torch.equal(logits, keep) and torch.equal(grad, inplace) and torch.equal(a, b)
+    r = keep[:, :V].double().requires_grad_(True)
+    lse, ok = r.logsumexp(1), targets >= 0
+    nll = lse - r.gather(1, targets.long().clamp(min=0)[:, None])[:, 0]
+    per = (1 - smoothing) * nll + (smoothing * (lse - r.mean(1)) if smoothing else 0) + 1e-3 * lse * lse
+    want = per[ok].sum() / ok.sum()
+    want.backward()
+    assert abs(float(a) - float(want)) < 1e-4 * max(1.0, abs(float(want)))
+    err = (grad[:, :V].double() - r.grad).abs()
+    assert (err <= (2.0 ** -8 if dt is torch.bfloat16 else 1e-5) * r.grad.abs() + 1e-7).all() and (grad[:, V:] == 0).all()
