@@ -274,3 +274,40 @@ def test_cross_entropy_gradient_beside_the_logits(V, ld, dt, smoothing):
     assert abs(float(a) - float(want)) < 1e-4 * max(1.0, abs(float(want)))
     err = (grad[:, :V].double() - r.grad).abs()
     assert (err <= (2.0 ** -8 if dt is torch.bfloat16 else 1e-5) * r.grad.abs() + 1e-7).all() and (grad[:, V:] == 0).all()
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 516), (64, 1600), (3, 1028), (1300, 2048), (5, 4100), (7, 8192), (2, 8196)])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("xdt", [torch.float32, torch.bfloat16])
+def test_norm_rows_that_a_warp_or_a_block_holds(rows, cols, rms, xdt):
+    """Rows of no multiple of 128, on both sides of the widths that a warp's and a block's registers hold, with and without the
+    fused sum.  FP32 statistics: results to 2^-8 of values up to about 6 in BF16, 1e-4 in FP32."""
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(5)
+    x, r = (torch.randn(rows, cols, device="cuda").to(xdt) for _ in range(2))
+    g, b = torch.randn(cols, device="cuda").to(xdt), torch.randn(cols, device="cuda").to(xdt)
+    for res in (None, r):
+        s = torch.empty_like(x) if res is not None else None
+        y, mean, rstd = K.norm_fwd(x, g, None if rms else b, rms=rms, residual=res, sum_out=s)
+        v = (x if res is None else x + r).double()
+        if s is not None:
+            assert torch.equal(s, x + r)
+        mu = 0.0 if rms else v.mean(1, keepdim=True)
+        rs = ((v - mu).square().mean(1, keepdim=True) + 1e-5).rsqrt()
+        want = (v - mu) * rs * g.double() + (0.0 if rms else b.double())
+        assert (y.double() - want).abs().max() < (1e-4 if xdt is torch.float32 else 6e-2)
+        # rows too long for a block's registers take the squares of the sum before it is rounded (2^-9 each, averaged over the row)
+        assert torch.allclose(rstd.double(), rs[:, 0], rtol=3e-4 if cols > 8192 and res is not None and xdt is torch.bfloat16 else 1e-5)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (300, 40), (16384, 3072), (257, 33)])
+def test_colsum_lanes(rows, cols):
+    """Fewer partials than lanes, more, and the 64 there are at most; FP32 sums of BF16: 1e-5 of the sum of magnitudes."""
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(6)
+    x = torch.randn(rows, cols, device="cuda").bfloat16()
+    out = torch.ones(cols, device="cuda")
+    want = x.double().sum(0)
+    assert ((K.colsum(x).double() - want).abs() <= 1e-5 * x.double().abs().sum(0)).all()
+    K.colsum(x, out=out, accumulate=True)
+    assert ((out.double() - 1 - want).abs() <= 1e-5 * (1 + x.double().abs().sum(0))).all()
