@@ -412,7 +412,7 @@ __global__ void philox_uniform_kernel(float* __restrict__ out, int64_t n, uint64
 // ------------------------------------------------------------------------------------------------
 // optimizer
 // ------------------------------------------------------------------------------------------------
-constexpr int kNormChunk = 65536;
+constexpr int kNormChunk = 16384;  // a few million parameters still reach every SM (65536: 33 us at 5.5 million, on 84 of them)
 
 template <typename GT>
 __global__ void grad_norm_partial_kernel(const GT* __restrict__ g, int64_t n, double* __restrict__ partial) {
@@ -634,13 +634,25 @@ __global__ void colsum_partial_vec_kernel(const __nv_bfloat16* __restrict__ dy, 
     }
   }
 }
-__global__ void colsum_final_kernel(const float* __restrict__ partial, float* __restrict__ out, int cols, int chunks,
-                                    int accumulate) {
+// Block (32 columns x 16 chunk lanes), fixed order.  One thread per column walked its up to 64 partials in turn, on a dozen SMs:
+// 9.4 us at 3072 columns.
+constexpr int kColsumLanes = 16;
+__global__ void __launch_bounds__(32 * kColsumLanes) colsum_final_kernel(const float* __restrict__ partial, float* __restrict__ out, int cols,
+                                                                         int chunks, int accumulate) {
   pdl_trigger();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
+  __shared__ float s[kColsumLanes][33];
+  const int c = blockIdx.x * 32 + threadIdx.x;
   float t = 0.0f;
-  for (int k = 0; k < chunks; ++k) t += partial[static_cast<int64_t>(k) * cols + c];
+  if (c < cols) {
+#pragma unroll 4
+    for (int k = threadIdx.y; k < chunks; k += kColsumLanes) t += partial[static_cast<int64_t>(k) * cols + c];
+  }
+  s[threadIdx.y][threadIdx.x] = t;
+  __syncthreads();
+  if (threadIdx.y != 0 || c >= cols) return;
+  t = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kColsumLanes; ++k) t += s[k][threadIdx.x];
   out[c] = accumulate ? out[c] + t : t;
 }
 
@@ -861,7 +873,7 @@ extern "C" int nx_colsum(const void* dy, int dtype, float* out, float* scratch, 
   } else if (dtype == NX_F32) colsum_partial_kernel<float><<<grid, block, 0, st>>>((const float*)dy, scratch, rows, cols, ld, rpc);
   else if (dtype == NX_BF16) colsum_partial_kernel<__nv_bfloat16><<<grid, block, 0, st>>>((const __nv_bfloat16*)dy, scratch, rows, cols, ld, rpc);
   else return -1;
-  colsum_final_kernel<<<(cols + 255) / 256, 256, 0, st>>>(scratch, out, cols, chunks, accumulate);
+  colsum_final_kernel<<<(cols + 31) / 32, dim3(32, kColsumLanes), 0, st>>>(scratch, out, cols, chunks, accumulate);
   return launch_status();
 }
 
@@ -948,6 +960,6 @@ extern "C" int nx_colsum_static(const void* dy, int dtype, float* out, int rows,
   } else {
     return -1;
   }
-  colsum_final_kernel<<<(cols + 255) / 256, 256, 0, st>>>(scratch, out, cols, chunks, accumulate);
+  colsum_final_kernel<<<(cols + 31) / 32, dim3(32, kColsumLanes), 0, st>>>(scratch, out, cols, chunks, accumulate);
   return launch_status();
 }

@@ -517,8 +517,9 @@ def unpack_opt_state(raw: bytes) -> OptState:
     return OptState.from_buffer_copy(raw)
 
 
-def make_chunks(segments, chunk=1 << 16, device="cuda") -> torch.Tensor:
-    """segments: iterable of (offset, count, wd_scale, lr_scale) -> device chunk table (uint8 tensor)."""
+def make_chunks(segments, chunk=1 << 14, device="cuda") -> torch.Tensor:
+    """segments: iterable of (offset, count, wd_scale, lr_scale) -> device chunk table (uint8 tensor).  A chunk is one block's
+    work: of 2^16 elements, the 5.5 million parameters of a small model kept 84 SMs busy for 106 us (26 us of traffic)."""
     items = []
     for off, cnt, wd, lr in segments:
         pos = 0
