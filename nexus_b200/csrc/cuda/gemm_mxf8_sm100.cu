@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cuda_fp8.h>
+#include <initializer_list>
 
 namespace {
 using namespace nx;
@@ -134,6 +135,109 @@ __global__ void mx_quantize_kernel(const void* __restrict__ src, int src_dtype, 
       for (int t = 0; t < 32 && k0 + t < Kc; ++t) cp[t] = enc8(v[t] * inv, fmt);
     }
   }
+}
+
+// The same codes and scales for BF16 sources whose rows lie on 16 bytes, from tiles of 128 x 128 that pass through shared memory
+// once: along the columns (ROW), along the rows (COL: the transposed matrix), or both from one read of the source.  A tile is one
+// scale atom of either matrix.  The kernel above reads a column of 32 elements per thread for the transposed form: 95 us on average
+// for the three operands of a Llama-7B layer at 8192 rows (49 us for the other form), where the bytes take 20 to 42.
+template <bool ROW, bool COL>
+__global__ void __launch_bounds__(256) mx_quantize_tile_kernel(const __nv_bfloat16* __restrict__ src, int64_t ld, int rows, int cols,
+                                                               uint8_t* __restrict__ codes, uint8_t* __restrict__ scales,
+                                                               uint8_t* __restrict__ codes_t, uint8_t* __restrict__ scales_t, int fmt) {
+  constexpr int kPitch = 136;  // elements of a tile row: 16 bytes past 128, so that neither pass meets one bank with a whole warp
+  __shared__ __align__(16) __nv_bfloat16 tile[128 * kPitch];
+  __shared__ __align__(16) uint8_t atom[kAtomBytes], atom_t[kAtomBytes];
+  const int c0 = blockIdx.x * 128, r0 = blockIdx.y * 128;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int at = threadIdx.x + i * 256, r = at >> 4, c = (at & 15) * 8;
+    uint4 q = make_uint4(0u, 0u, 0u, 0u);
+    if (r0 + r < rows) {
+      const __nv_bfloat16* p = src + static_cast<int64_t>(r0 + r) * ld + c0 + c;
+      if (c0 + c + 8 <= cols) {
+        q = *reinterpret_cast<const uint4*>(p);
+      } else {
+        __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&q);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (c0 + c + j < cols) e[j] = p[j];
+      }
+    }
+    *reinterpret_cast<uint4*>(tile + r * kPitch + c) = q;
+  }
+  __syncthreads();
+  // codes of one block: 32 bytes at `out`, `left` of them inside the matrix
+  auto emit = [&](const float (&v)[32], uint32_t sb, uint8_t* out, int left, bool whole) {
+    const float inv = mx_inv_scale(sb);
+    if (whole && left >= 32) {
+      uint32_t w[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        w[q] = enc8(v[4 * q] * inv, fmt) | (enc8(v[4 * q + 1] * inv, fmt) << 8) | (enc8(v[4 * q + 2] * inv, fmt) << 16) |
+               (enc8(v[4 * q + 3] * inv, fmt) << 24);
+      reinterpret_cast<uint4*>(out)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      reinterpret_cast<uint4*>(out)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < 32; ++t)
+        if (t < left) out[t] = enc8(v[t] * inv, fmt);
+    }
+  };
+  if (ROW) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int at = threadIdx.x + i * 256, r = at >> 2, j = at & 3, k0 = c0 + j * 32;
+      uint32_t sb = 127;
+      if (r0 + r < rows && k0 < cols) {
+        float v[32], am = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint4 u = *reinterpret_cast<const uint4*>(tile + r * kPitch + j * 32 + q * 8);
+          unpack_bf16x2(u.x, v[8 * q + 0], v[8 * q + 1]);
+          unpack_bf16x2(u.y, v[8 * q + 2], v[8 * q + 3]);
+          unpack_bf16x2(u.z, v[8 * q + 4], v[8 * q + 5]);
+          unpack_bf16x2(u.w, v[8 * q + 6], v[8 * q + 7]);
+        }
+#pragma unroll
+        for (int t = 0; t < 32; ++t) am = fmaxf(am, fabsf(v[t]));
+        sb = mx_scale_byte(am, fmt);
+        emit(v, sb, codes + static_cast<int64_t>(r0 + r) * cols + k0, cols - k0, (cols & 15) == 0);
+      }
+      atom[(r & 31) * 16 + (r >> 5) * 4 + j] = static_cast<uint8_t>(sb);
+    }
+  }
+  if (COL) {
+    const int c = (threadIdx.x & 63) * 2, j = threadIdx.x >> 6, k0 = r0 + j * 32;
+    float v0[32], v1[32], am0 = 0.0f, am1 = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+      unpack_bf16x2(*reinterpret_cast<const uint32_t*>(tile + (j * 32 + t) * kPitch + c), v0[t], v1[t]);
+      am0 = fmaxf(am0, fabsf(v0[t]));
+      am1 = fmaxf(am1, fabsf(v1[t]));
+    }
+    const bool in = k0 < rows, whole = (rows & 15) == 0;
+    const uint32_t s0 = in && c0 + c < cols ? mx_scale_byte(am0, fmt) : 127u, s1 = in && c0 + c + 1 < cols ? mx_scale_byte(am1, fmt) : 127u;
+    uint8_t* out = codes_t + static_cast<int64_t>(c0 + c) * rows + k0;
+    if (in && c0 + c < cols) emit(v0, s0, out, rows - k0, whole);
+    if (in && c0 + c + 1 < cols) emit(v1, s1, out + rows, rows - k0, whole);
+    atom_t[(c & 31) * 16 + (c >> 5) * 4 + j] = static_cast<uint8_t>(s0);
+    atom_t[((c + 1) & 31) * 16 + (c >> 5) * 4 + j] = static_cast<uint8_t>(s1);
+  }
+  __syncthreads();
+  if (ROW && threadIdx.x < 32)
+    reinterpret_cast<uint4*>(scales + (static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x) * kAtomBytes)[threadIdx.x] =
+        reinterpret_cast<const uint4*>(atom)[threadIdx.x];
+  if (COL && threadIdx.x >= 32 && threadIdx.x < 64)
+    reinterpret_cast<uint4*>(scales_t + (static_cast<size_t>(blockIdx.x) * gridDim.y + blockIdx.y) * kAtomBytes)[threadIdx.x - 32] =
+        reinterpret_cast<const uint4*>(atom_t)[threadIdx.x - 32];
+}
+
+// BF16 rows on 16 bytes, outputs on 16 bytes, a grid that fits
+bool mx_tiles(const void* src, int src_dtype, int64_t ld, int rows, std::initializer_list<const void*> outs) {
+  uintptr_t at = reinterpret_cast<uintptr_t>(src);
+  for (const void* p : outs) at |= reinterpret_cast<uintptr_t>(p);
+  return src_dtype == NX_BF16 && (ld & 7) == 0 && (at & 15) == 0 && (rows + 127) / 128 <= 65535;
 }
 
 __global__ void mx_dequantize_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, int fmt,
@@ -670,6 +774,14 @@ extern "C" int nx_mx_quantize(const void* src, int src_dtype, int64_t ld, int ro
   if (fmt != NX_E4M3 && fmt != NX_E5M2) return -1;
   if (src_dtype != NX_BF16 && src_dtype != NX_F32 && src_dtype != NX_F16) return -1;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (mx_tiles(src, src_dtype, ld, rows, {codes, scales})) {
+    const dim3 grid(static_cast<unsigned>((cols + 127) / 128), static_cast<unsigned>((rows + 127) / 128));
+    const auto* x = static_cast<const __nv_bfloat16*>(src);
+    auto *c = static_cast<uint8_t*>(codes), *s = static_cast<uint8_t*>(scales);
+    if (transpose) mx_quantize_tile_kernel<false, true><<<grid, 256, 0, stream>>>(x, ld, rows, cols, nullptr, nullptr, c, s, fmt);
+    else mx_quantize_tile_kernel<true, false><<<grid, 256, 0, stream>>>(x, ld, rows, cols, c, s, nullptr, nullptr, fmt);
+    return launch_status();
+  }
   const int R = transpose ? cols : rows, Kc = transpose ? rows : cols;
   const int64_t total = static_cast<int64_t>((R + 127) & ~127) * (((Kc + 127) >> 7) * 4);
   const int threads = 128;
@@ -680,6 +792,21 @@ extern "C" int nx_mx_quantize(const void* src, int src_dtype, int64_t ld, int ro
   else
     mx_quantize_kernel<false><<<blocks, threads, 0, stream>>>(src, src_dtype, ld, rows, cols, static_cast<uint8_t*>(codes),
                                                               static_cast<uint8_t*>(scales), fmt);
+  return launch_status();
+}
+
+extern "C" int nx_mx_quantize_both(const void* src, int src_dtype, int64_t ld, int rows, int cols, void* codes, void* scales, void* codes_t,
+                                   void* scales_t, int fmt, nx_stream_t stream_) {
+  if (src == nullptr || codes == nullptr || scales == nullptr || codes_t == nullptr || scales_t == nullptr || rows <= 0 || cols <= 0) return -1;
+  if (fmt != NX_E4M3 && fmt != NX_E5M2) return -1;
+  if (!mx_tiles(src, src_dtype, ld, rows, {codes, scales, codes_t, scales_t})) {
+    const int rc = nx_mx_quantize(src, src_dtype, ld, rows, cols, codes, scales, fmt, 0, stream_);
+    return rc != 0 ? rc : nx_mx_quantize(src, src_dtype, ld, rows, cols, codes_t, scales_t, fmt, 1, stream_);
+  }
+  const dim3 grid(static_cast<unsigned>((cols + 127) / 128), static_cast<unsigned>((rows + 127) / 128));
+  mx_quantize_tile_kernel<true, true><<<grid, 256, 0, static_cast<cudaStream_t>(stream_)>>>(
+      static_cast<const __nv_bfloat16*>(src), ld, rows, cols, static_cast<uint8_t*>(codes), static_cast<uint8_t*>(scales),
+      static_cast<uint8_t*>(codes_t), static_cast<uint8_t*>(scales_t), fmt);
   return launch_status();
 }
 

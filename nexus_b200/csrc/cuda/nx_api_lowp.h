@@ -27,6 +27,9 @@ size_t nx_mx_scale_bytes(int rows, int cols);
 //                 the backward GEMMs need.  `scales` has nx_mx_scale_bytes(rows of the codes, columns of the codes).
 int nx_mx_quantize(const void* src, int src_dtype, int64_t ld, int rows, int cols, void* codes, void* scales, int fmt,
                    int transpose, nx_stream_t stream);
+// Both forms from one read of the source.
+int nx_mx_quantize_both(const void* src, int src_dtype, int64_t ld, int rows, int cols, void* codes, void* scales, void* codes_t,
+                        void* scales_t, int fmt, nx_stream_t stream);
 // dst [rows][cols] = codes * scale (the inverse of nx_mx_quantize with transpose == 0); for tests and fallbacks.
 int nx_mx_dequantize(const void* codes, const void* scales, int fmt, int rows, int cols, void* dst, int dst_dtype,
                      nx_stream_t stream);

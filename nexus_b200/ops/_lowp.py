@@ -157,6 +157,20 @@ def mx_quantize(x: torch.Tensor, dtype=torch.float8_e4m3fn, transpose: bool = Fa
     return codes, scales
 
 
+def mx_quantize_both(x: torch.Tensor, dtype=torch.float8_e4m3fn):
+    """``mx_quantize(x), mx_quantize(x, transpose=True)``, from one read of x on a GPU."""
+    if not x.is_cuda:
+        return mx_quantize_reference(x, dtype, False), mx_quantize_reference(x, dtype, True)
+    assert x.dim() == 2 and x.stride(1) == 1
+    rows, cols = x.shape
+    out = [(torch.empty((r, k), dtype=dtype, device=x.device), torch.empty(mx_scale_bytes(r, k), dtype=torch.uint8, device=x.device))
+           for r, k in ((rows, cols), (cols, rows))]
+    (c, s), (ct, st) = out
+    K._check(K.lib().nx_mx_quantize_both(K._p(x), C.c_int(K._DT[x.dtype]), C.c_int64(x.stride(0)), C.c_int(rows), C.c_int(cols), K._p(c),
+                                         K._p(s), K._p(ct), K._p(st), C.c_int(_FMT[dtype]), K._stream()), "nx_mx_quantize_both")
+    return out
+
+
 def mx_dequantize(codes: torch.Tensor, scales: torch.Tensor, dtype=torch.float32) -> torch.Tensor:
     if not codes.is_cuda:
         return mx_dequantize_reference(codes, scales).to(dtype)
@@ -267,12 +281,11 @@ class _MxLinearFn(torch.autograd.Function):
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
-        gq, gs = mx_quantize(dy2, torch.float8_e5m2)                    # [M, N], blocks along N
+        (gq, gs), (gtq, gts) = mx_quantize_both(dy2, torch.float8_e5m2)  # [M, N], blocks along N; [N, M], blocks along M
         wtq, wts = mx_weight_cache.get(w, True)                         # [K, N], blocks along N
         dx = mx_gemm(gq, gs, wtq, wts, out_dtype=x2.dtype)              # [M, K]
-        gtq, gts = mx_quantize(dy2, torch.float8_e5m2, transpose=True)  # [N, M], blocks along M
         xtq, xts = mx_quantize(x2, transpose=True)                      # [K, M], blocks along M
-        dw = mx_gemm(gtq, gts, xtq, xts, out_dtype=torch.float32).to(w.dtype)  # [N, K]
+        dw = mx_gemm(gtq, gts, xtq, xts, out_dtype=w.dtype if w.dtype in (torch.bfloat16, torch.float32) else torch.float32).to(w.dtype)
         db = dy2.float().sum(0).to(dy.dtype) if ctx.has_bias else None
         return dx.reshape(ctx.shape), dw, db
 

@@ -166,3 +166,27 @@ def test_mx_linear_gradients_close_to_fp32():
     for got, want in ((x.grad, x2.grad), (w.grad, w2.grad), (b.grad, b2.grad)):
         assert (got.float() - want).norm() / want.norm() < 0.08
     K.check_status()
+
+
+@pytest.mark.parametrize("rows,cols,ld", [(1, 8, 8), (127, 129, 136), (128, 128, 128), (300, 264, 272), (1040, 33, 40), (31, 4096, 4096)])
+def test_mx_quantize_both_forms_from_one_read(rows, cols, ld):
+    """Edges of the 128 x 128 tiles, odd widths inside a wider pitch, NaN and infinities: the bytes of the reference in both forms; rows
+    that lie on no 16 bytes take the general kernel and give the same."""
+    from nexus_b200.ops import _lowp as L
+    torch.manual_seed(5)
+    x = (torch.randn(rows, ld, device="cuda") * torch.logspace(-4, 4, ld, device="cuda")).bfloat16()[:, :cols]
+    odd = torch.zeros(rows, ld + 1, device="cuda").bfloat16()[:, 1: 1 + cols]
+    odd.copy_(x)
+    for dt in (torch.float8_e4m3fn, torch.float8_e5m2):
+        for src in (x, odd):
+            for (q, s), tr in zip(L.mx_quantize_both(src, dt), (False, True)):
+                rq, rs = L.mx_quantize_reference(x, dt, transpose=tr)
+                one = L.mx_quantize(src, dt, transpose=tr)
+                for a, b in ((q, s), one):
+                    assert torch.equal(a.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(b, rs)
+    if rows > 1:
+        x[1, :3] = torch.tensor([float("nan"), float("inf"), 2.0], device="cuda").bfloat16()
+        odd.copy_(x)
+        for dt in (torch.float8_e4m3fn, torch.float8_e5m2):
+            for a, b in zip(L.mx_quantize_both(x, dt), L.mx_quantize_both(odd, dt)):
+                assert torch.equal(a[0].view(torch.uint8), b[0].view(torch.uint8)) and torch.equal(a[1], b[1])
