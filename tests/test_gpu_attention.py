@@ -263,3 +263,20 @@ def test_packed_blocks_outside_the_rows_are_refused():
     for segs in ([(0, 11)], [(-1, 4)], [(3, 0)], [(8, 3)]):
         with pytest.raises(ValueError):
             K.PackedBlocks(segs, 10, 64)
+
+
+def test_backward_in_a_thread_that_made_no_runtime_call_yet():
+    """The autograd engine's thread may reach the tensor maps first: every buffer comes from the allocator's cache."""
+    import threading
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(4)
+    q, k, v, do = (torch.randn(1, 256, 2, 64, device="cuda").bfloat16() for _ in range(4))
+    o, lse = K.attention_fwd(q, k, v)
+    want = K.attention_bwd(q, k, v, o, lse, do)
+    out, outs = [], [torch.empty_like(q) for _ in range(3)]
+    spare = torch.empty(1, 2, 256, device="cuda")      # what the call takes from the cache for its row sums
+    del spare
+    th = threading.Thread(target=lambda: out.append(K.attention_bwd(q, k, v, o, lse, do, dq=outs[0], dk=outs[1], dv=outs[2])))
+    th.start()
+    th.join()
+    assert out and all(torch.equal(a, b) for a, b in zip(out[0], want))
