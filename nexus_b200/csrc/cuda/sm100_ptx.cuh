@@ -140,14 +140,16 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // Bounded wait. Returns false when the limit ran out or when another role of the CTA raised
 // `*abort_flag` (a shared-memory int): the caller must then leave its loop.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
+  // The clock is first read after 64 tries: its read takes long beside a short wait, and most waits are short.
+  uint64_t t0 = 0;
   uint32_t spins = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((++spins & 63u) == 0u) {
       if (*abort_flag != 0) return false;
-      if (globaltimer_ns() - t0 > NX_WAIT_LIMIT_NS) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > NX_WAIT_LIMIT_NS) {
         *abort_flag = 1;
         return false;
       }
