@@ -15,6 +15,7 @@
 // Features: causal, sliding window, GQA (H % Hkv == 0), Tq != Tk (bottom-right aligned causal
 // mask), head_dim 64 or 128, softmax scale.  Parity: src/cuda/flash_attention.cu:230-857 and
 // include/nexus/attention/params.hpp:18-46 of the reference (which uses mma.sync m16n8k16).
+#include "common.cuh"
 #include "flash_common.cuh"
 #include "nx_api_attention.h"
 #include "sm100_ptx.cuh"
@@ -25,8 +26,6 @@
 
 namespace {
 using namespace nx;
-
-constexpr int kThreads = 192;  // warps 0-3: softmax / row math, warp 4: TMA, warp 5: MMA + TMEM
 
 struct AttnDev {
   void* out;        // fwd: O [B,Tq,H,D] bf16;   dq kernel: dQ;   dkdv kernel: dK
@@ -375,6 +374,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();  // the set-up above overlaps the end of the kernel in front
   const uint32_t tmem_s = tmem_base;
   const uint32_t tmem_o = tmem_base + 128;
 
@@ -752,6 +752,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();  // the set-up above overlaps the end of the kernel in front
 
   if (warp == 8) {
     if (lane == 0) {
@@ -1090,26 +1091,76 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 }
 
 // ================================================================================================
+// backward.  Both kernels are bound by the row math (conversions, exponentials, stores of P and dS) and by the hand-overs between
+// it and the tensor core, so the score products of chunk i + 1 are issued ahead of the gradient products of chunk i:
+//   head_dim 128, one CTA per SM: into a second pair of score tiles, while the math of chunk i runs;
+//   head_dim 64, two CTAs per SM with 256 TMEM columns each: into the same tiles, as soon as the math of chunk i has read them.
+// At head_dim 128 two threads (warps w and w + 4) share a row, 32 of a chunk's 64 columns each; at 64, where the other CTA's warps
+// fill the gaps, one thread has it (two per row took 112 us for dQ on 16 x 12 x 1024 x 64, against 103 before this scheme).  The
+// factor `scale` of dS goes to the results.
+// On 2 x 32 (8) x 4096 x 128, causal, dK / dV takes 542 us and dQ 510; with four math warps and the four steps in turn it was 797
+// and 759, the tensor cores busy for a quarter of that.  At head_dim 64 two CTAs per SM had hidden most of it already.
+// ================================================================================================
+constexpr int bwd_math_warps(int hd) { return hd == 64 ? 4 : 8; }  // row quarter = warp & 3, column half = warp >> 2
+constexpr int bwd_threads(int hd) { return (bwd_math_warps(hd) + 2) * 32; }  // then one warp for TMA, one for MMA + TMEM
+
+// NC score columns and as many of dP, one wait
+template <int NC>
+__device__ __forceinline__ void load_scores(uint32_t s_addr, uint32_t dp_addr, uint32_t (&sv)[NC], uint32_t (&dv)[NC]) {
+  if constexpr (NC == 32) {
+    tmem_ld_32x32b_x32(s_addr, sv);
+    tmem_ld_32x32b_x32(dp_addr, dv);
+  } else {
+    tmem_ld_32x32b_x16(s_addr, sv);
+    tmem_ld_32x32b_x16(dp_addr, dv);
+  }
+  tmem_ld_wait();
+}
+// NC values of row r, columns c0 .. of a swizzled [128][64] tile
+template <int NC>
+__device__ __forceinline__ void store_tile_cols(uint8_t* tile, int r, int c0, const uint32_t (&w)[NC / 2]) {
+#pragma unroll
+  for (int g = 0; g < NC / 8; ++g)
+    *reinterpret_cast<uint4*>(tile + sw128_off(r, c0 / 8 + g)) = make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
+}
+// 32 accumulator columns, times `f`, as BF16
+__device__ __forceinline__ void store_row32_scaled(__nv_bfloat16* dst, const uint32_t (&a)[32], float f) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    uint4 w;
+    w.x = pack_bf16x2(__uint_as_float(a[8 * g + 0]) * f, __uint_as_float(a[8 * g + 1]) * f);
+    w.y = pack_bf16x2(__uint_as_float(a[8 * g + 2]) * f, __uint_as_float(a[8 * g + 3]) * f);
+    w.z = pack_bf16x2(__uint_as_float(a[8 * g + 4]) * f, __uint_as_float(a[8 * g + 5]) * f);
+    w.w = pack_bf16x2(__uint_as_float(a[8 * g + 6]) * f, __uint_as_float(a[8 * g + 7]) * f);
+    reinterpret_cast<uint4*>(dst)[g] = w;
+  }
+}
+
+// ================================================================================================
 // backward, part 1: dK / dV.  One CTA per (kv block of 128, kv head, batch); loops over the q heads
 // of the group and over q chunks of 64 rows.  TMEM: S^T [128 kv][64 q], dP^T [128][64], dV [128][HD],
-// dK [128][HD].  Thread r owns kv row r.
+// dK [128][HD].  The two threads of row r own kv row r.
 // ================================================================================================
 template <int HD>
 struct DkvCfg {
   static constexpr int kKVBytes = 128 * HD * 2;   // K and V tiles (resident)
   static constexpr int kQBytes = 64 * HD * 2;     // Q / dO chunk
   static constexpr int kPBytes = 128 * 64 * 2;    // P^T and dS^T
-  static constexpr int kSmem = 2 * kKVBytes + 4 * kQBytes + 2 * kPBytes + 2 * 2 * 64 * 4 + 128;
-  static constexpr int kTmemCols = (HD == 64) ? 256 : 512;  // 64 + 64 + 2*HD
+  static constexpr int kTiles = (HD == 64) ? 1 : 2;   // score tiles in TMEM
+  static constexpr int kStages = (HD == 64) ? 2 : 3;  // Q / dO chunks
+  static constexpr int kPBufs = (HD == 64) ? 1 : 2;   // P^T / dS^T buffers (two CTAs per SM leave room for one)
+  static constexpr int kSmem = 2 * kKVBytes + 2 * kStages * kQBytes + 2 * kPBufs * kPBytes + 4 * 2 * 64 * 4 + 192;
+  static constexpr int kTmemCols = (HD == 64) ? 256 : 512;  // kTiles * 128 + 2 * HD
 };
 
 template <int HD, bool EXT>  // EXT: soft-capping / ALiBi / dropout row math (a build of its own)
-__global__ void __launch_bounds__(kThreads, (HD == 64 ? 2 : 1))
+__global__ void __launch_bounds__(bwd_threads(HD), (HD == 64 ? 2 : 1))
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                      const AttnDev p) {
   pdl_launch_dependents();
   using C = DkvCfg<HD>;
+  constexpr int NS = C::kStages, NT = C::kTiles, NP = C::kPBufs, NC = 32, MW = bwd_math_warps(HD), kSpan = 64 / (MW / 4);  // kSpan: columns of a chunk per math thread
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1 KiB aligned base; uniform early exit
@@ -1118,21 +1169,21 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   }
   uint8_t* sK = smem;
   uint8_t* sV = sK + C::kKVBytes;
-  uint8_t* sQ = sV + C::kKVBytes;        // 2 stages
-  uint8_t* sDO = sQ + 2 * C::kQBytes;    // 2 stages
-  uint8_t* sPT = sDO + 2 * C::kQBytes;   // [128 kv][64 q] bf16
-  uint8_t* sDST = sPT + C::kPBytes;      // [128 kv][64 q] bf16
-  float* sLse = reinterpret_cast<float*>(sDST + C::kPBytes);  // [2][64] (log2 domain)
-  float* sDsum = sLse + 2 * 64;                               // [2][64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sDsum + 2 * 64);
+  uint8_t* sQ = sV + C::kKVBytes;          // NS stages
+  uint8_t* sDO = sQ + NS * C::kQBytes;     // NS stages
+  uint8_t* sPT = sDO + NS * C::kQBytes;    // NP x [128 kv][64 q] bf16
+  uint8_t* sDST = sPT + NP * C::kPBytes;   // NP x [128 kv][64 q] bf16
+  float* sLse = reinterpret_cast<float*>(sDST + NP * C::kPBytes);  // [4][64] (log2 domain)
+  float* sDsum = sLse + 4 * 64;                                    // [4][64]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sDsum + 4 * 64);
   uint64_t* kv_full = bars;
-  uint64_t* q_full = bars + 1;    // [2]
-  uint64_t* q_empty = bars + 3;   // [2]
-  uint64_t* s_full = bars + 5;    // S^T and dP^T ready
-  uint64_t* p_full = bars + 6;    // P^T and dS^T written
-  uint64_t* acc_done = bars + 7;  // dV/dK MMAs of this chunk retired (P^T/dS^T reusable)
-  uint64_t* stat_full = bars + 8;  // per-q statistics of the chunk staged in shared memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  uint64_t* q_full = bars + 1;      // [3]
+  uint64_t* q_empty = bars + 4;     // [3]
+  uint64_t* s_full = bars + 7;      // [2] S^T and dP^T of a chunk ready, by its parity
+  uint64_t* p_full = bars + 9;      // [2] P^T and dS^T written (and the scores read), by the chunk's parity
+  uint64_t* acc_done = bars + 11;   // [2] dV / dK products retired: buffer `chunk % NP` of P^T / dS^T may be rewritten
+  uint64_t* stat_full = bars + 13;  // [4] per-q statistics of a chunk staged, by the chunk modulo 4
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1155,18 +1206,20 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < 3; ++s) {
       mbar_init(&q_full[s], 1);
       mbar_init(&q_empty[s], 1);
     }
-    mbar_init(s_full, 1);
-    mbar_init(p_full, 4);  // one arrival per math warp
-    mbar_init(acc_done, 1);
-    mbar_init(stat_full, 2);  // warps 0 and 1 stage the statistics
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&p_full[s], MW);  // one arrival per math warp
+      mbar_init(&acc_done[s], 1);
+    }
+    for (int s = 0; s < 4; ++s) mbar_init(&stat_full[s], 2);  // warps 0 and 1 stage the statistics
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 5) {
+  if (warp == MW + 1) {
     tmem_alloc(tmem_slot, C::kTmemCols);
     tmem_relinquish();
   }
@@ -1174,21 +1227,20 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_st = tmem_base;         // S^T   64 cols
-  const uint32_t tmem_dpt = tmem_base + 64;   // dP^T  64 cols
-  const uint32_t tmem_dv = tmem_base + 128;   // dV    HD cols
-  const uint32_t tmem_dk = tmem_base + 128 + HD;
+  pdl_wait();  // the set-up above overlaps the end of the kernel in front
+  const uint32_t tmem_dv = tmem_base + NT * 128;  // score tile i: S^T at 128 i, dP^T at 128 i + 64
+  const uint32_t tmem_dk = tmem_dv + HD;
 
-  if (warp == 4) {
+  if (warp == MW) {
     if (lane == 0) {
       mbar_arrive_expect_tx(kv_full, 2 * C::kKVBytes);
       load_tile<HD>(sK, &tm_k, kv_full, 128, k0, hk, b, p.hfirst);
       load_tile<HD>(sV, &tm_v, kv_full, 128, k0, hk, b, p.hfirst);
       for (int it = 0; it < iters; ++it) {
-        const int s = it & 1;
+        const int s = it % NS;
         const int hq = hk * group + it / nchunk;
         const int c0 = (cb + it % nchunk) * 64;
-        if (!mbar_wait_bounded(&q_empty[s], ((it >> 1) & 1) ^ 1u, abort_flag)) {
+        if (!mbar_wait_bounded(&q_empty[s], ((it / NS) & 1) ^ 1u, abort_flag)) {
           atomicCAS(p.status, 0, kStatusTimeoutProducer);
           break;
         }
@@ -1197,191 +1249,193 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         load_tile<HD>(sDO + s * C::kQBytes, &tm_do, &q_full[s], 64, c0, hq, b, p.hfirst);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == MW + 1) {
     // the whole warp walks the loop (descriptors stay in uniform registers); one elected lane issues
-    {
-      const bool leader = elect_one();
-      const uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, false, false, 128, 64);   // K Q^T, V dO^T
-      const uint32_t idesc_g = make_idesc(kFmtBF16, kFmtBF16, false, true, 128, HD);    // P^T dO, dS^T Q
-      bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(kv_full, 0, abort_flag));
-      if (!ok && leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
-      const uint64_t dK = desc_kmajor(smem_u32(sK), 128, 0), dV = desc_kmajor(smem_u32(sV), 128, 0);
-      const uint64_t dPT = desc_kmajor(smem_u32(sPT), 128, 0), dDST = desc_kmajor(smem_u32(sDST), 128, 0);
-      for (int it = 0; it < iters && ok; ++it) {
-        const int s = it & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&q_full[s], (it >> 1) & 1, abort_flag))) {
-          if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
-          break;
-        }
-        tc_fence_after_sync();
-        const uint32_t aQ = smem_u32(sQ + s * C::kQBytes), aDO = smem_u32(sDO + s * C::kQBytes);
-        const uint64_t dQk = desc_kmajor(aQ, 64, 0), dDOk = desc_kmajor(aDO, 64, 0);
-        const uint64_t dQm = desc_mnmajor(aQ, 64, 0), dDOm = desc_mnmajor(aDO, 64, 0);
-        if (leader) {
+    const bool leader = elect_one();
+    const uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, false, false, 128, 64);   // K Q^T, V dO^T
+    const uint32_t idesc_g = make_idesc(kFmtBF16, kFmtBF16, false, true, 128, HD);    // P^T dO, dS^T Q
+    const uint64_t dK = desc_kmajor(smem_u32(sK), 128, 0), dV = desc_kmajor(smem_u32(sV), 128, 0);
+    bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(kv_full, 0, abort_flag));
+    auto scores = [&](int it) {  // S^T and dP^T of chunk `it`
+      const int s = it % NS;
+      ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&q_full[s], (it / NS) & 1, abort_flag));
+      if (!ok) return;
+      tc_fence_after_sync();
+      const uint64_t dQk = desc_kmajor(smem_u32(sQ + s * C::kQBytes), 64, 0), dDOk = desc_kmajor(smem_u32(sDO + s * C::kQBytes), 64, 0);
+      const uint32_t tmem_st = tmem_base + (it % NT) * 128;
+      if (leader) {
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks)
-            umma_f16_ss(tmem_st, dK + kstep_kmajor(128, ks), dQk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < HD / 16; ++ks)
+          umma_f16_ss(tmem_st, dK + kstep_kmajor(128, ks), dQk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks)
-            umma_f16_ss(tmem_dpt, dV + kstep_kmajor(128, ks), dDOk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
-          umma_commit(s_full);
-        }
-        __syncwarp();
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(p_full, it & 1, abort_flag))) {
-          if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
-          break;
-        }
-        tc_fence_after_sync();
-        // dV += P^T dO ; dK += dS^T Q   (reduction over the 64 q rows of the chunk: 4 k-steps)
-        if (leader) {
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma_f16_ss(tmem_dv, dPT + kstep_kmajor(128, ks), dDOm + kstep_mnmajor(ks), idesc_g,
-                        (it > 0 || ks > 0) ? 1u : 0u);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma_f16_ss(tmem_dk, dDST + kstep_kmajor(128, ks), dQm + kstep_mnmajor(ks), idesc_g,
-                        (it > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&q_empty[s]);
-          umma_commit(acc_done);
-        }
-        __syncwarp();
+        for (int ks = 0; ks < HD / 16; ++ks)
+          umma_f16_ss(tmem_st + 64, dV + kstep_kmajor(128, ks), dDOk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
+        umma_commit(&s_full[it & 1]);
       }
+      __syncwarp();
+    };
+    if (iters > 0) scores(0);
+    for (int it = 0; it < iters && ok; ++it) {
+      if (NT == 2 && it + 1 < iters) scores(it + 1);
+      ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&p_full[it & 1], (it >> 1) & 1, abort_flag));
+      if (NT == 1 && it + 1 < iters) scores(it + 1);
+      if (!ok) break;
+      tc_fence_after_sync();
+      // dV += P^T dO ; dK += dS^T Q   (reduction over the 64 q rows of the chunk: 4 k-steps)
+      const int s = it % NS;
+      const uint64_t dQm = desc_mnmajor(smem_u32(sQ + s * C::kQBytes), 64, 0), dDOm = desc_mnmajor(smem_u32(sDO + s * C::kQBytes), 64, 0);
+      const uint64_t dPT = desc_kmajor(smem_u32(sPT + (it % NP) * C::kPBytes), 128, 0);
+      const uint64_t dDST = desc_kmajor(smem_u32(sDST + (it % NP) * C::kPBytes), 128, 0);
+      if (leader) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          umma_f16_ss(tmem_dv, dPT + kstep_kmajor(128, ks), dDOm + kstep_mnmajor(ks), idesc_g, (it > 0 || ks > 0) ? 1u : 0u);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          umma_f16_ss(tmem_dk, dDST + kstep_kmajor(128, ks), dQm + kstep_mnmajor(ks), idesc_g, (it > 0 || ks > 0) ? 1u : 0u);
+        umma_commit(&q_empty[s]);
+        umma_commit(&acc_done[it % NP]);
+      }
+      __syncwarp();
     }
+    if (!ok && leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
   } else {
-    const int r = warp * 32 + lane;  // kv row inside the block == TMEM lane
+    const int r = (warp & 3) * 32 + lane;  // kv row inside the block == TMEM lane
+    const int h0 = (warp >> 2) * kSpan;    // first of this thread's columns of a chunk
     const int k = k0 + r;
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const float sc = p.scale * kLog2e;
     // queries that may attend to key k:  k - off <= q (causal),  q <= k - off + window - 1 (window)
     int q_row_lo = p.causal ? k - off : 0;
     int q_row_hi = p.Tq - 1;
     if (p.window > 0) q_row_hi = min(q_row_hi, k - off + p.window - 1);
     if (k >= p.Tk) q_row_lo = 0x3fffffff;  // key out of range: nothing valid
+    // The per-q statistics of a chunk come one chunk ahead into one of four slots (by then every warp has left the chunk three
+    // before it), and their loads are issued another chunk earlier.
+    float st_lse = 0.0f, st_dsum = 0.0f;
+    auto load_stats = [&](int it) {
+      const int q = (cb + it % nchunk) * 64 + r;
+      const int64_t idx = (static_cast<int64_t>(b) * p.H + hk * group + it / nchunk) * p.Tq + q;
+      st_lse = q < p.Tq ? p.lse[idx] : INFINITY;
+      st_dsum = q < p.Tq ? p.dsum[idx] : 0.0f;
+    };
+    auto store_stats = [&](int it) {
+      sLse[(it & 3) * 64 + r] = (st_lse == -INFINITY ? INFINITY : st_lse) * kLog2e;  // -inf: a row that saw no key, no probabilities
+      sDsum[(it & 3) * 64 + r] = st_dsum;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&stat_full[it & 3]);
+    };
+    if (warp < 2 && iters > 0) {
+      load_stats(0);
+      store_stats(0);
+      if (iters > 1) load_stats(1);
+    }
     bool ok = true;
+    int hq = hk * group, chunk = 0;
     for (int it = 0; it < iters; ++it) {
-      const int hq = hk * group + it / nchunk;
-      const int c0 = (cb + it % nchunk) * 64;
-      // stage the per-q statistics of this chunk (double-buffered by iteration parity)
-      float* lse_s = sLse + (it & 1) * 64;
-      float* ds_s = sDsum + (it & 1) * 64;
-      if (r < 64) {
-        const int q = c0 + r;
-        const int64_t idx = (static_cast<int64_t>(b) * p.H + hq) * p.Tq + q;
-        float l = q < p.Tq ? p.lse[idx] : INFINITY;
-        if (l == -INFINITY) l = INFINITY;  // row that saw no key: probabilities are zero
-        lse_s[r] = l * kLog2e;
-        ds_s[r] = q < p.Tq ? p.dsum[idx] : 0.0f;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(stat_full);
+      const int c0 = (cb + chunk) * 64;
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&s_full[it & 1], (it >> 1) & 1, abort_flag));
+      if (ok && warp < 2 && it + 1 < iters) {
+        store_stats(it + 1);
+        if (it + 2 < iters) load_stats(it + 2);
       }
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(stat_full, it & 1, abort_flag));
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(s_full, it & 1, abort_flag));
-      if (ok && it > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_done, (it - 1) & 1, abort_flag));
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(&stat_full[it & 3], (it >> 2) & 1, abort_flag));
       if (!ok) {
         if (lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
         break;
       }
       tc_fence_after_sync();
+      const float *lse_s = sLse + (it & 3) * 64 + h0, *ds_s = sDsum + (it & 3) * 64 + h0;
+      uint8_t *pt = sPT + (it % NP) * C::kPBytes, *dst = sDST + (it % NP) * C::kPBytes;
+      const uint32_t tmem_st = tmem_base + (it % NT) * 128 + lane_addr + h0;
       const bool need_mask = (k0 + 128 > p.Tk) || (c0 + 64 > p.Tq) || (p.causal && (k0 + 127 > c0 + off)) ||
                              (p.window > 0 && (k0 < c0 + 63 + off - p.window + 1));
-      constexpr bool ext_on = EXT;
       const ScoreExt ext = EXT ? make_ext(p, hq, b) : ScoreExt{};
-      auto body = [&](auto mask_tag, auto ext_tag) {
+      auto body = [&](auto mask_tag) {
         constexpr bool kMask = decltype(mask_tag)::value;
-        constexpr bool kExt = decltype(ext_tag)::value;
 #pragma unroll 1
-        for (int cc = 0; cc < 2; ++cc) {
-          uint32_t sv[32], dv[32];
-          tmem_ld_32x32b_x32(tmem_st + lane_addr + cc * 32, sv);
-          tmem_ld_32x32b_x32(tmem_dpt + lane_addr + cc * 32, dv);
-          tmem_ld_wait();
-          const int clo = q_row_lo - c0 - cc * 32, chi = q_row_hi - c0 - cc * 32;  // valid iff clo <= c <= chi
-          float pr[32], dsv[32];
+        for (int cc = 0; cc < kSpan; cc += NC) {
+          uint32_t sv[NC], dv[NC], pr[NC / 2], dsv[NC / 2];
+          load_scores<NC>(tmem_st + cc, tmem_st + 64 + cc, sv, dv);
+          const int clo = q_row_lo - c0 - h0 - cc, chi = q_row_hi - c0 - h0 - cc;  // valid iff clo <= c <= chi
 #pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const int qi = cc * 32 + c;
-            float sraw = __uint_as_float(sv[c]), dfac = 1.0f;
-            if (kExt) sraw = score_ext(ext, sraw, k - (c0 + qi + off), dfac);
-            float e = ex2f(fmaf(sraw, sc, -lse_s[qi]));
-            if (kMask && (c < clo || c > chi)) e = 0.0f;
-            float dp = __uint_as_float(dv[c]), keep = 1.0f;
-            if (kExt && ext.drop_p > 0.0f) {
-              keep = drop_scale_qk(ext, c0 + qi, k);
-              dp *= keep;
+          for (int c4 = 0; c4 < NC; c4 += 4) {
+            const float4 l4 = *reinterpret_cast<const float4*>(lse_s + cc + c4), d4 = *reinterpret_cast<const float4*>(ds_s + cc + c4);
+            const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, dd[4] = {d4.x, d4.y, d4.z, d4.w};
+            float e[4], g[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int c = c4 + u, qi = h0 + cc + c;
+              float sraw = __uint_as_float(sv[c]), dfac = 1.0f, keep = 1.0f;
+              if (EXT) sraw = score_ext(ext, sraw, k - (c0 + qi + off), dfac);
+              e[u] = ex2f(fmaf(sraw, sc, -ls[u]));
+              if (kMask && (c < clo || c > chi)) e[u] = 0.0f;
+              float dp = __uint_as_float(dv[c]);
+              if (EXT && ext.drop_p > 0.0f) {
+                keep = drop_scale_qk(ext, c0 + qi, k);
+                dp *= keep;
+              }
+              g[u] = e[u] * (dp - dd[u]);
+              if (EXT) {
+                g[u] *= dfac;
+                e[u] *= keep;  // what met V in the forward pass
+              }
             }
-            pr[c] = e * keep;  // what met V in the forward pass
-            dsv[c] = e * (dp - ds_s[qi]) * p.scale;
-            if (kExt) dsv[c] *= dfac;
+            pr[c4 / 2] = pack_bf16x2(e[0], e[1]);
+            pr[c4 / 2 + 1] = pack_bf16x2(e[2], e[3]);
+            dsv[c4 / 2] = pack_bf16x2(g[0], g[1]);
+            dsv[c4 / 2 + 1] = pack_bf16x2(g[2], g[3]);
           }
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 w, z;
-            w.x = pack_bf16x2(pr[8 * g + 0], pr[8 * g + 1]);
-            w.y = pack_bf16x2(pr[8 * g + 2], pr[8 * g + 3]);
-            w.z = pack_bf16x2(pr[8 * g + 4], pr[8 * g + 5]);
-            w.w = pack_bf16x2(pr[8 * g + 6], pr[8 * g + 7]);
-            z.x = pack_bf16x2(dsv[8 * g + 0], dsv[8 * g + 1]);
-            z.y = pack_bf16x2(dsv[8 * g + 2], dsv[8 * g + 3]);
-            z.z = pack_bf16x2(dsv[8 * g + 4], dsv[8 * g + 5]);
-            z.w = pack_bf16x2(dsv[8 * g + 6], dsv[8 * g + 7]);
-            const uint32_t o = sw128_off(r, cc * 4 + g);
-            *reinterpret_cast<uint4*>(sPT + o) = w;
-            *reinterpret_cast<uint4*>(sDST + o) = z;
+          if (cc == 0 && it >= NP) {  // the products that read this buffer's previous contents have retired
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_done[it % NP], (it / NP - 1) & 1, abort_flag));
+            if (!ok) return;
           }
+          store_tile_cols<NC>(pt, r, h0 + cc, pr);
+          store_tile_cols<NC>(dst, r, h0 + cc, dsv);
         }
       };
-      if (ext_on) {
-        if (need_mask) body(std::true_type{}, std::true_type{});
-        else body(std::false_type{}, std::true_type{});
-      } else {
-        if (need_mask) body(std::true_type{}, std::false_type{});
-        else body(std::false_type{}, std::false_type{});
+      if (need_mask) body(std::true_type{});
+      else body(std::false_type{});
+      if (!ok) {
+        if (lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
+        break;
       }
       fence_proxy_async_smem();  // this thread's tile writes -> visible to the tensor core's reads
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&p_full[it & 1]);
+      if (++chunk == nchunk) {
+        chunk = 0;
+        ++hq;
+      }
     }
     // drain: wait for the last accumulation, then write dK / dV rows
     if (ok && iters > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_done, (iters - 1) & 1, abort_flag));
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_done[(iters - 1) % NP], ((iters - 1) / NP) & 1, abort_flag));
       if (!ok && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
     }
     if (ok) {  // warp-uniform: the TMEM loads below are warp-collective, only the stores are per row
       tc_fence_after_sync();
-      const bool row_ok = k < p.Tk;
+      const int d0 = (warp >> 2) * (HD / (MW / 4));
       __nv_bfloat16* dk = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(b) * p.o_batch +
-                          static_cast<int64_t>(k) * p.o_row + static_cast<int64_t>(hk) * p.o_head;
+                          static_cast<int64_t>(k) * p.o_row + static_cast<int64_t>(hk) * p.o_head + d0;
       __nv_bfloat16* dvp = reinterpret_cast<__nv_bfloat16*>(p.out2) + static_cast<int64_t>(b) * p.o2_batch +
-                           static_cast<int64_t>(k) * p.o2_row + static_cast<int64_t>(hk) * p.o2_head;
+                           static_cast<int64_t>(k) * p.o2_row + static_cast<int64_t>(hk) * p.o2_head + d0;
 #pragma unroll 1
-      for (int cc = 0; cc < HD / 32; ++cc) {
-        uint32_t a[32], c[32];
+      for (int cc = 0; cc < HD / (MW / 4); cc += 32) {
+        uint32_t a[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) a[i] = 0u;
         if (iters > 0) {
-          tmem_ld_32x32b_x32(tmem_dk + lane_addr + cc * 32, a);
-          tmem_ld_32x32b_x32(tmem_dv + lane_addr + cc * 32, c);
+          tmem_ld_32x32b_x32(tmem_dk + lane_addr + d0 + cc, a);
           tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) a[i] = c[i] = 0u;
         }
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 w, z;
-          w.x = pack_bf16x2(__uint_as_float(a[8 * g + 0]), __uint_as_float(a[8 * g + 1]));
-          w.y = pack_bf16x2(__uint_as_float(a[8 * g + 2]), __uint_as_float(a[8 * g + 3]));
-          w.z = pack_bf16x2(__uint_as_float(a[8 * g + 4]), __uint_as_float(a[8 * g + 5]));
-          w.w = pack_bf16x2(__uint_as_float(a[8 * g + 6]), __uint_as_float(a[8 * g + 7]));
-          z.x = pack_bf16x2(__uint_as_float(c[8 * g + 0]), __uint_as_float(c[8 * g + 1]));
-          z.y = pack_bf16x2(__uint_as_float(c[8 * g + 2]), __uint_as_float(c[8 * g + 3]));
-          z.z = pack_bf16x2(__uint_as_float(c[8 * g + 4]), __uint_as_float(c[8 * g + 5]));
-          z.w = pack_bf16x2(__uint_as_float(c[8 * g + 6]), __uint_as_float(c[8 * g + 7]));
-          if (row_ok) {
-            reinterpret_cast<uint4*>(dk + cc * 32)[g] = w;
-            reinterpret_cast<uint4*>(dvp + cc * 32)[g] = z;
-          }
+        if (k < p.Tk) store_row32_scaled(dk + cc, a, p.scale);
+        if (iters > 0) {
+          tmem_ld_32x32b_x32(tmem_dv + lane_addr + d0 + cc, a);
+          tmem_ld_wait();
         }
+        if (k < p.Tk) store_row32_scaled(dvp + cc, a, 1.0f);
       }
     }
   }
@@ -1393,7 +1447,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(2000);
     __syncthreads();
   }
-  if (warp == 5) {
+  if (warp == MW + 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, C::kTmemCols);
   }
@@ -1401,27 +1455,27 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
 // ================================================================================================
 // backward, part 2: dQ.  One CTA per (q block of 128, head, batch); loops over kv chunks of 64.
-// TMEM: S [128 q][64 kv], dP [128][64], dQ [128][HD].  Thread r owns q row r.
+// TMEM: S [128 q][64 kv], dP [128][64], dQ [128][HD].  The two threads of row r own q row r.
 // ================================================================================================
 template <int HD>
 struct DqCfg {
   static constexpr int kQBytes = 128 * HD * 2;   // Q and dO tiles (resident)
   static constexpr int kKVBytes = 64 * HD * 2;   // K / V chunk
   static constexpr int kPBytes = 128 * 64 * 2;   // dS
-#ifndef NX_DQ_STAGES
-#define NX_DQ_STAGES 2
-#endif
-  static constexpr int kStages = (HD == 64) ? NX_DQ_STAGES : 2;  // K / V chunk stages (a third one measured no faster)
-  static constexpr int kSmem = 2 * kQBytes + 2 * kStages * kKVBytes + kPBytes + 256;
-  static constexpr int kTmemCols = 256;  // 64 + 64 + HD
+  static constexpr int kTiles = (HD == 64) ? 1 : 2;  // score tiles in TMEM
+  static constexpr int kStages = 3;
+  static constexpr int kSmem = 2 * kQBytes + 2 * kStages * kKVBytes + 2 * kPBytes + 192;
+  static constexpr int kTmemCols = (HD == 64) ? 256 : 512;  // kTiles * 128 + HD
 };
 
 template <int HD, bool EXT>  // EXT: soft-capping / ALiBi / dropout row math (a build of its own)
-__global__ void __launch_bounds__(kThreads, (HD == 64 ? 2 : 1))
+__global__ void __launch_bounds__(bwd_threads(HD), (HD == 64 ? 2 : 1))
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                    const AttnDev p) {
+  pdl_launch_dependents();
   using C = DqCfg<HD>;
+  constexpr int NS = C::kStages, NT = C::kTiles, NC = 32, MW = bwd_math_warps(HD), kSpan = 64 / (MW / 4);  // kSpan: columns of a chunk per math thread
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1 KiB aligned base; uniform early exit
@@ -1430,18 +1484,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
   uint8_t* sQ = smem;
   uint8_t* sDO = sQ + C::kQBytes;
-  constexpr int NS = C::kStages;
   uint8_t* sK = sDO + C::kQBytes;        // NS stages
   uint8_t* sV = sK + NS * C::kKVBytes;   // NS stages
-  uint8_t* sDS = sV + NS * C::kKVBytes;  // [128 q][64 kv] bf16
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + C::kPBytes);
+  uint8_t* sDS = sV + NS * C::kKVBytes;  // 2 x [128 q][64 kv] bf16
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + 2 * C::kPBytes);
   uint64_t* q_full = bars;
-  uint64_t* kv_full = bars + 1;        // [NS]
-  uint64_t* kv_empty = kv_full + NS;   // [NS]
-  uint64_t* s_full = kv_empty + NS;
-  uint64_t* p_full = s_full + 1;
-  uint64_t* acc_done = p_full + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+  uint64_t* kv_full = bars + 1;    // [NS]
+  uint64_t* kv_empty = bars + 4;   // [NS]
+  uint64_t* s_full = bars + 7;     // [2] by the chunk's parity, as the two below
+  uint64_t* p_full = bars + 9;     // [2]
+  uint64_t* acc_done = bars + 11;  // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1464,13 +1517,15 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       mbar_init(&kv_full[s], 1);
       mbar_init(&kv_empty[s], 1);
     }
-    mbar_init(s_full, 1);
-    mbar_init(p_full, 4);  // one arrival per math warp
-    mbar_init(acc_done, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&p_full[s], MW);  // one arrival per math warp
+      mbar_init(&acc_done[s], 1);
+    }
     *abort_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 5) {
+  if (warp == MW + 1) {
     tmem_alloc(tmem_slot, C::kTmemCols);
     tmem_relinquish();
   }
@@ -1478,11 +1533,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base;
-  const uint32_t tmem_dp = tmem_base + 64;
-  const uint32_t tmem_dq = tmem_base + 128;
+  pdl_wait();  // the set-up above overlaps the end of the kernel in front
+  const uint32_t tmem_dq = tmem_base + NT * 128;  // score tile i: S at 128 i, dP at 128 i + 64
 
-  if (warp == 4) {
+  if (warp == MW) {
     if (lane == 0) {
       mbar_arrive_expect_tx(q_full, 2 * C::kQBytes);
       load_tile<HD>(sQ, &tm_q, q_full, 128, q0, h, b, p.hfirst);
@@ -1498,72 +1552,75 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         load_tile<HD>(sV + s * C::kKVBytes, &tm_v, &kv_full[s], 64, (jb + it) * 64, hk, b, p.hfirst);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp == MW + 1) {
     // the whole warp walks the loop (descriptors stay in uniform registers); one elected lane issues
-    {
-      const bool leader = elect_one();
-      const uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, false, false, 128, 64);  // Q K^T, dO V^T
-      const uint32_t idesc_g = make_idesc(kFmtBF16, kFmtBF16, false, true, 128, HD);   // dS K
-      bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(q_full, 0, abort_flag));
-      if (!ok && leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
-      const uint64_t dQ = desc_kmajor(smem_u32(sQ), 128, 0), dDO = desc_kmajor(smem_u32(sDO), 128, 0);
-      const uint64_t dDS = desc_kmajor(smem_u32(sDS), 128, 0);
-      for (int it = 0; it < iters && ok; ++it) {
-        const int s = it % NS;
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&kv_full[s], (it / NS) & 1, abort_flag))) {
-          if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
-          break;
-        }
-        tc_fence_after_sync();
-        const uint32_t aK = smem_u32(sK + s * C::kKVBytes), aV = smem_u32(sV + s * C::kKVBytes);
-        const uint64_t dKk = desc_kmajor(aK, 64, 0), dVk = desc_kmajor(aV, 64, 0), dKm = desc_mnmajor(aK, 64, 0);
-        if (leader) {
+    const bool leader = elect_one();
+    const uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, false, false, 128, 64);  // Q K^T, dO V^T
+    const uint32_t idesc_g = make_idesc(kFmtBF16, kFmtBF16, false, true, 128, HD);   // dS K
+    const uint64_t dQ = desc_kmajor(smem_u32(sQ), 128, 0), dDO = desc_kmajor(smem_u32(sDO), 128, 0);
+    bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(q_full, 0, abort_flag));
+    auto scores = [&](int it) {  // S and dP of chunk `it`
+      const int s = it % NS;
+      ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&kv_full[s], (it / NS) & 1, abort_flag));
+      if (!ok) return;
+      tc_fence_after_sync();
+      const uint64_t dKk = desc_kmajor(smem_u32(sK + s * C::kKVBytes), 64, 0), dVk = desc_kmajor(smem_u32(sV + s * C::kKVBytes), 64, 0);
+      const uint32_t tmem_s = tmem_base + (it % NT) * 128;
+      if (leader) {
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks)
-            umma_f16_ss(tmem_s, dQ + kstep_kmajor(128, ks), dKk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < HD / 16; ++ks)
+          umma_f16_ss(tmem_s, dQ + kstep_kmajor(128, ks), dKk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks)
-            umma_f16_ss(tmem_dp, dDO + kstep_kmajor(128, ks), dVk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
-          umma_commit(s_full);
-        }
-        __syncwarp();
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(p_full, it & 1, abort_flag))) {
-          if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
-          break;
-        }
-        tc_fence_after_sync();
-        if (leader) {
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma_f16_ss(tmem_dq, dDS + kstep_kmajor(128, ks), dKm + kstep_mnmajor(ks), idesc_g,
-                        (it > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&kv_empty[s]);
-          umma_commit(acc_done);
-        }
-        __syncwarp();
+        for (int ks = 0; ks < HD / 16; ++ks)
+          umma_f16_ss(tmem_s + 64, dDO + kstep_kmajor(128, ks), dVk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
+        umma_commit(&s_full[it & 1]);
       }
+      __syncwarp();
+    };
+    if (iters > 0) scores(0);
+    for (int it = 0; it < iters && ok; ++it) {
+      if (NT == 2 && it + 1 < iters) scores(it + 1);
+      ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&p_full[it & 1], (it >> 1) & 1, abort_flag));
+      if (NT == 1 && it + 1 < iters) scores(it + 1);
+      if (!ok) break;
+      tc_fence_after_sync();
+      const int s = it % NS;
+      const uint64_t dKm = desc_mnmajor(smem_u32(sK + s * C::kKVBytes), 64, 0);
+      const uint64_t dDS = desc_kmajor(smem_u32(sDS + (it & 1) * C::kPBytes), 128, 0);
+      if (leader) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          umma_f16_ss(tmem_dq, dDS + kstep_kmajor(128, ks), dKm + kstep_mnmajor(ks), idesc_g, (it > 0 || ks > 0) ? 1u : 0u);
+        umma_commit(&kv_empty[s]);
+        umma_commit(&acc_done[it & 1]);
+      }
+      __syncwarp();
     }
+    if (!ok && leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
   } else {
-    const int r = warp * 32 + lane;
+    const int r = (warp & 3) * 32 + lane;
+    const int half = warp >> 2, h0 = half * kSpan;  // first of this thread's columns of a chunk
     const int q = q0 + r;
-    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const float sc = p.scale * kLog2e;
     const int off = p.Tk - p.Tq;
     const int64_t sidx = (static_cast<int64_t>(b) * p.H + h) * p.Tq + q;
     float lse_n = q < p.Tq ? p.lse[sidx] : INFINITY;
     if (lse_n == -INFINITY) lse_n = INFINITY;  // row that saw no key: probabilities are zero
     const float lse2 = lse_n * kLog2e;
-    // dsum = rowsum(dO * O) of this thread's row, straight from global memory (the loads overlap the first tiles'
-    // TMA traffic); published for the dK/dV kernel
+    // dsum = rowsum(dO * O) of the row, straight from global memory (the loads overlap the first tiles' TMA traffic), a share of
+    // it from each of its threads; published for the dK / dV kernel.  Two shares meet in the dS buffers, which are free until all
+    // threads have passed the second barrier.
+    constexpr int kShare = HD / 8 / (MW / 4);  // 16-byte pieces of the row
     float dsum = 0.0f;
     if (q < p.Tq) {
       const uint4* orow = reinterpret_cast<const uint4*>(p.o_in + static_cast<int64_t>(b) * p.oi_batch +
-                                                         static_cast<int64_t>(q) * p.oi_row + static_cast<int64_t>(h) * p.oi_head);
+                                                         static_cast<int64_t>(q) * p.oi_row + static_cast<int64_t>(h) * p.oi_head) + half * kShare;
       const uint4* grow = reinterpret_cast<const uint4*>(p.do_in + static_cast<int64_t>(b) * p.di_batch +
-                                                         static_cast<int64_t>(q) * p.di_row + static_cast<int64_t>(h) * p.di_head);
+                                                         static_cast<int64_t>(q) * p.di_row + static_cast<int64_t>(h) * p.di_head) + half * kShare;
       float a0 = 0.0f, a1 = 0.0f;
 #pragma unroll
-      for (int i = 0; i < HD / 8; ++i) {
+      for (int i = 0; i < kShare; ++i) {
         const uint4 ov = orow[i], gv = grow[i];
         const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
@@ -1576,98 +1633,93 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
       }
       dsum = a0 + a1;
-      p.dsum_out[sidx] = dsum;
     }
+    if constexpr (MW == 8) {
+      float* sX = reinterpret_cast<float*>(sDS);  // [2][128]
+      sX[half * 128 + r] = dsum;
+      softmax_bar();
+      dsum = sX[r] + sX[128 + r];
+      softmax_bar();
+    }
+    if (half == 0 && q < p.Tq) p.dsum_out[sidx] = dsum;
     int row_lo, row_hi;
     row_limits(p, p.Tq, p.Tk, q, row_lo, row_hi);
     if (q >= p.Tq) row_lo = 0x3fffffff;
-    constexpr bool ext_on = EXT;
     const ScoreExt ext = EXT ? make_ext(p, h, b) : ScoreExt{};
     bool ok = true;
     for (int it = 0; it < iters; ++it) {
       const int k0 = (jb + it) * 64;
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(s_full, it & 1, abort_flag));
-      if (ok && it > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_done, (it - 1) & 1, abort_flag));
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&s_full[it & 1], (it >> 1) & 1, abort_flag));
       if (!ok) {
         if (lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
         break;
       }
       tc_fence_after_sync();
+      uint8_t* ds_t = sDS + (it & 1) * C::kPBytes;
+      const uint32_t tmem_s = tmem_base + (it % NT) * 128 + lane_addr + h0;
       const bool need_mask = (k0 + 64 > p.Tk) || (q0 + 128 > p.Tq) || (p.causal && (k0 + 63 > q0 + off)) ||
                              (p.window > 0 && (k0 < q0 + 127 + off - p.window + 1));
-      auto body = [&](auto mask_tag, auto ext_tag) {
+      auto body = [&](auto mask_tag) {
         constexpr bool kMask = decltype(mask_tag)::value;
-        constexpr bool kExt = decltype(ext_tag)::value;
 #pragma unroll 1
-        for (int cc = 0; cc < 2; ++cc) {
-          uint32_t sv[32], dv[32];
-          tmem_ld_32x32b_x32(tmem_s + lane_addr + cc * 32, sv);
-          tmem_ld_32x32b_x32(tmem_dp + lane_addr + cc * 32, dv);
-          tmem_ld_wait();
-          const int clo = row_lo - k0 - cc * 32, chi = row_hi - k0 - cc * 32;
-          float dsv[32];
+        for (int cc = 0; cc < kSpan; cc += NC) {
+          uint32_t sv[NC], dv[NC], dsv[NC / 2];
+          load_scores<NC>(tmem_s + cc, tmem_s + 64 + cc, sv, dv);
+          const int clo = row_lo - k0 - h0 - cc, chi = row_hi - k0 - h0 - cc;
 #pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            float sraw = __uint_as_float(sv[c]), dfac = 1.0f;
-            if (kExt) sraw = score_ext(ext, sraw, k0 + cc * 32 + c - (q + off), dfac);
-            float e = ex2f(fmaf(sraw, sc, -lse2));
-            if (kMask && (c < clo || c > chi)) e = 0.0f;
-            float dp = __uint_as_float(dv[c]);
-            if (kExt && ext.drop_p > 0.0f) dp *= drop_scale_qk(ext, q, k0 + cc * 32 + c);
-            dsv[c] = e * (dp - dsum) * p.scale;
-            if (kExt) dsv[c] *= dfac;
-          }
+          for (int c2 = 0; c2 < NC; c2 += 2) {
+            float g[2];
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 z;
-            z.x = pack_bf16x2(dsv[8 * g + 0], dsv[8 * g + 1]);
-            z.y = pack_bf16x2(dsv[8 * g + 2], dsv[8 * g + 3]);
-            z.z = pack_bf16x2(dsv[8 * g + 4], dsv[8 * g + 5]);
-            z.w = pack_bf16x2(dsv[8 * g + 6], dsv[8 * g + 7]);
-            *reinterpret_cast<uint4*>(sDS + sw128_off(r, cc * 4 + g)) = z;
+            for (int u = 0; u < 2; ++u) {
+              const int c = c2 + u, kk = k0 + h0 + cc + c;
+              float sraw = __uint_as_float(sv[c]), dfac = 1.0f;
+              if (EXT) sraw = score_ext(ext, sraw, kk - (q + off), dfac);
+              float e = ex2f(fmaf(sraw, sc, -lse2));
+              if (kMask && (c < clo || c > chi)) e = 0.0f;
+              float dp = __uint_as_float(dv[c]);
+              if (EXT && ext.drop_p > 0.0f) dp *= drop_scale_qk(ext, q, kk);
+              g[u] = e * (dp - dsum);
+              if (EXT) g[u] *= dfac;
+            }
+            dsv[c2 / 2] = pack_bf16x2(g[0], g[1]);
           }
+          if (cc == 0 && it >= 2) {  // the product that read this buffer's previous contents has retired
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_done[it & 1], (it / 2 - 1) & 1, abort_flag));
+            if (!ok) return;
+          }
+          store_tile_cols<NC>(ds_t, r, h0 + cc, dsv);
         }
       };
-      if (ext_on) {
-        if (need_mask) body(std::true_type{}, std::true_type{});
-        else body(std::false_type{}, std::true_type{});
-      } else {
-        if (need_mask) body(std::true_type{}, std::false_type{});
-        else body(std::false_type{}, std::false_type{});
+      if (need_mask) body(std::true_type{});
+      else body(std::false_type{});
+      if (!ok) {
+        if (lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
+        break;
       }
-      fence_proxy_async_smem();  // this thread's tile writes -> visible to the tensor core's reads
+      fence_proxy_async_smem();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&p_full[it & 1]);
     }
     if (ok && iters > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_done, (iters - 1) & 1, abort_flag));
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&acc_done[(iters - 1) & 1], ((iters - 1) >> 1) & 1, abort_flag));
       if (!ok && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
     }
     if (ok) {  // warp-uniform: the TMEM loads below are warp-collective, only the stores are per row
       tc_fence_after_sync();
-      const bool row_ok = q < p.Tq;
+      const int d0 = half * (HD / (MW / 4));
       __nv_bfloat16* dq = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(b) * p.o_batch +
-                          static_cast<int64_t>(q) * p.o_row + static_cast<int64_t>(h) * p.o_head;
+                          static_cast<int64_t>(q) * p.o_row + static_cast<int64_t>(h) * p.o_head + d0;
 #pragma unroll 1
-      for (int cc = 0; cc < HD / 32; ++cc) {
+      for (int cc = 0; cc < HD / (MW / 4); cc += 32) {
         uint32_t a[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) a[i] = 0u;
         if (iters > 0) {
-          tmem_ld_32x32b_x32(tmem_dq + lane_addr + cc * 32, a);
+          tmem_ld_32x32b_x32(tmem_dq + lane_addr + d0 + cc, a);
           tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) a[i] = 0u;
         }
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 w;
-          w.x = pack_bf16x2(__uint_as_float(a[8 * g + 0]), __uint_as_float(a[8 * g + 1]));
-          w.y = pack_bf16x2(__uint_as_float(a[8 * g + 2]), __uint_as_float(a[8 * g + 3]));
-          w.z = pack_bf16x2(__uint_as_float(a[8 * g + 4]), __uint_as_float(a[8 * g + 5]));
-          w.w = pack_bf16x2(__uint_as_float(a[8 * g + 6]), __uint_as_float(a[8 * g + 7]));
-          if (row_ok) reinterpret_cast<uint4*>(dq + cc * 32)[g] = w;
-        }
+        if (q < p.Tq) store_row32_scaled(dq + cc, a, p.scale);
       }
     }
   }
@@ -1679,7 +1731,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(2000);
     __syncthreads();
   }
-  if (warp == 5) {
+  if (warp == MW + 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, C::kTmemCols);
   }
@@ -1790,7 +1842,7 @@ extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
       if (set_smem(attn_fwd2_kernel<HD_, false>, Fwd2Cfg<HD_>::kSmem)) return -2;                          \
       once = true;                                                                                  \
     }                                                                                               \
-    attn_fwd2_kernel<HD_, false><<<grid2, kFwd2Threads, Fwd2Cfg<HD_>::kSmem, st>>>(tq, tk, tv, p);         \
+    NX_PDL((attn_fwd2_kernel<HD_, false>), grid2, kFwd2Threads, Fwd2Cfg<HD_>::kSmem, st, tq, tk, tv, p);    \
   } while (0)
     if (HD == 64) NX_FWD2(64);
     else NX_FWD2(128);
@@ -1804,7 +1856,7 @@ extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
       if (set_smem(attn_fwd_kernel<HD_, EXT_, false>, FwdCfg<HD_>::kSmem)) return -2;                      \
       once = true;                                                                                  \
     }                                                                                               \
-    attn_fwd_kernel<HD_, EXT_, false><<<grid, kFwdThreads, FwdCfg<HD_>::kSmem, st>>>(tq, tk, tv, p);       \
+    NX_PDL((attn_fwd_kernel<HD_, EXT_, false>), grid, kFwdThreads, FwdCfg<HD_>::kSmem, st, tq, tk, tv, p);  \
   } while (0)
   const int mode = !ext ? 0 : (p.alibi == nullptr && p.dropout_p <= 0.0f && p.scale > 0.0f ? 2 : 1);
   if (HD == 64) {
@@ -1850,7 +1902,7 @@ extern "C" int nx_attention_fwd_packed(const NxAttnArgs* a, const int32_t* block
       if (set_smem(KERN_, CFG_::kSmem)) return -2;                                                  \
       once = true;                                                                                  \
     }                                                                                               \
-    KERN_<<<std::min(p.items, sms * PER_SM_), kFwdThreads, CFG_::kSmem, st>>>(tq, tk, tv, p);       \
+    NX_PDL(KERN_, std::min(p.items, sms * PER_SM_), kFwdThreads, CFG_::kSmem, st, tq, tk, tv, p);   \
   } while (0)
   // the blocks are of nx_attention_packed_rows() query rows: two tiles where nx_attention_fwd takes the two-tile form too
   const bool cap = p.softcap > 0.0f;
@@ -1883,7 +1935,7 @@ extern "C" int nx_attention_bwd(const NxAttnArgs* a, nx_stream_t stream_) {
       if (set_smem(KERN_<HD_, EXT_>, CFG_<HD_>::kSmem)) return -2;                                  \
       once = true;                                                                                  \
     }                                                                                               \
-    KERN_<HD_, EXT_><<<grid, kThreads, CFG_<HD_>::kSmem, st>>>(tq, tk, tv, tdo, p);                 \
+    NX_PDL((KERN_<HD_, EXT_>), grid, bwd_threads(HD_), CFG_<HD_>::kSmem, st, tq, tk, tv, tdo, p);           \
   } while (0)
   // part 1: dQ (also forms dsum = rowsum(dO * O) and leaves it for part 2)
   {

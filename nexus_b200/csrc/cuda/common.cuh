@@ -16,6 +16,34 @@ constexpr int kNumSmsB200 = 148;
 // when the next launch is an ordinary one.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The other side: blocks until the grids in front have completed and their memory is visible.  A kernel launched by `launch_pdl`
+// passes this before it touches anything that a kernel in front may have written, and before its own first write.
+__device__ __forceinline__ void pdl_dependency() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A launch that may begin while the kernel in front of it drains (its blocks are placed and its constants set up by then): in a
+// chain of short kernels, as decoding is, about half a microsecond per launch.  For kernels that call `pdl_dependency` only.
+template <typename... KArgs, typename... Args>
+inline int launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...) == cudaSuccess) return 0;
+  (void)cudaGetLastError();
+  return -2;
+}
+// The launch in a function that returns 0 or an error: NX_PDL((kernel), grid, threads, shared memory, stream, arguments ...)
+#define NX_PDL(KERN_, GRID_, BLOCK_, SMEM_, ST_, ...)                                                  \
+  do {                                                                                                 \
+    if (::nx::launch_pdl(KERN_, dim3(GRID_), dim3(BLOCK_), SMEM_, ST_, __VA_ARGS__) != 0) return -2;    \
+  } while (0)
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
