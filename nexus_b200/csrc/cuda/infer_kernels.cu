@@ -1,6 +1,5 @@
 // Inference kernels: paged KV cache append (BF16 / INT8 / FP8-E4M3 with per-(slot, head) scales), paged
-// attention for decode with split-KV and a combine pass, skinny GEMM for small batches (result of a
-// row does not depend on the batch it is in), row gather, single-kernel sampler (repetition /
+// attention for decode with split-KV and a combine pass, row gather, single-kernel sampler (repetition /
 // frequency / presence penalties, temperature, top-k, top-p, min-p, Philox draw, greedy ties ->
 // lowest id), token counting, NLL, RoPE (rotate-half and interleaved), SwiGLU / GeGLU forward and
 // backward, weight-only INT8 / INT4 (group-wise) GEMV and dequantisation, activation row quantisation.
@@ -359,58 +358,6 @@ __global__ void paged_combine_kernel(const float* __restrict__ part_o, const flo
 }
 
 // ------------------------------------------------------------------------------------------------
-// skinny GEMM: y[m][n] = act(sum_k x[m][k] * w[n][k] + bias[n]) (+ residual / accumulate), m <= 16.
-// One warp per output column; the reduction order of a row is fixed (independent of m).
-// ------------------------------------------------------------------------------------------------
-constexpr int kSkinnyMaxRows = 16;
-
-template <int M, typename YT>
-__global__ void __launch_bounds__(256)
-skinny_gemm_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const __nv_bfloat16* __restrict__ w, int64_t ldw,
-                   const __nv_bfloat16* __restrict__ bias, const YT* residual, int64_t ldr, YT* y, int64_t ldy, int n,
-                   int k, int act) {
-  const int col = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (col >= n) return;
-  float acc[M];
-#pragma unroll
-  for (int i = 0; i < M; ++i) acc[i] = 0.0f;
-  const __nv_bfloat16* wr = w + static_cast<int64_t>(col) * ldw;
-  for (int c = lane * 8; c < k; c += 256) {
-    float wv[8];
-    unpack8(*reinterpret_cast<const uint4*>(wr + c), wv);
-#pragma unroll
-    for (int i = 0; i < M; ++i) {
-      float xv[8];
-      unpack8(*reinterpret_cast<const uint4*>(x + i * ldx + c), xv);
-      float s = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s += xv[j] * wv[j];
-      acc[i] += s;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < M; ++i) {
-    float s = acc[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    acc[i] = s;
-  }
-  if (lane == 0) {
-    const float b = bias ? __bfloat162float(bias[col]) : 0.0f;
-#pragma unroll
-    for (int i = 0; i < M; ++i) {
-      float v = acc[i] + b;
-      if (act == NX_ACT_GELU) v = gelu_tanh_f(v);
-      else if (act == NX_ACT_RELU) v = fmaxf(v, 0.0f);
-      else if (act == NX_ACT_SILU) v = silu_f(v);
-      else if (act == NX_ACT_RELU2) v = fmaxf(v, 0.0f) * fmaxf(v, 0.0f);
-      if (residual) v += Num<YT>::load(residual + i * ldr + col);
-      Num<YT>::store(y + i * ldy + col, v);
-    }
-  }
-}
-
-// ------------------------------------------------------------------------------------------------
 // row gather / token counts / NLL
 // ------------------------------------------------------------------------------------------------
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ rows,
@@ -711,6 +658,8 @@ bool gated_vec(const void* a, const void* b, const void* c, int64_t n, int F) {
 // weight-only quantised GEMV (m <= 16): INT8 per-output-row scale, INT4 group-wise (AWQ-style,
 // two nibbles per byte, value = (nibble - 8) * scale[group]); plus dequantisation to BF16.
 // ------------------------------------------------------------------------------------------------
+constexpr int kGemvMaxRows = 16;
+
 template <int M, int BITS>
 __global__ void __launch_bounds__(256)
 wq_gemv_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const uint8_t* __restrict__ wq,
@@ -886,33 +835,6 @@ extern "C" int nx_paged_attention_decode(const NxPagedArgs* a, nx_stream_t strea
   return launch_status();
 }
 
-extern "C" int nx_skinny_max_rows(void) { return kSkinnyMaxRows; }
-
-extern "C" int nx_skinny_gemm(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* bias,
-                              const void* residual, int64_t ldr, void* y, int64_t ldy, int out_dtype, int m, int n,
-                              int k, int act, nx_stream_t stream) {
-  if (m < 1 || m > kSkinnyMaxRows || n <= 0 || k <= 0 || (k & 7) || (ldx & 7) || (ldw & 7)) return -1;
-  if (out_dtype != NX_BF16 && out_dtype != NX_F32) return -1;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int blocks = (n + 7) / 8;
-#define NX_SK(M_)                                                                                                      \
-  case M_:                                                                                                             \
-    if (out_dtype == NX_F32)                                                                                     \
-      skinny_gemm_kernel<M_, float><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, ldw, \
-          (const __nv_bfloat16*)bias, (const float*)residual, ldr, (float*)y, ldy, n, k, act);                          \
-    else                                                                                                               \
-      skinny_gemm_kernel<M_, __nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)x, ldx,                       \
-          (const __nv_bfloat16*)w, ldw, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, ldr,                \
-          (__nv_bfloat16*)y, ldy, n, k, act);                                                                          \
-    break
-  switch (m) {
-    NX_SK(1); NX_SK(2); NX_SK(3); NX_SK(4); NX_SK(5); NX_SK(6); NX_SK(7); NX_SK(8);
-    NX_SK(9); NX_SK(10); NX_SK(11); NX_SK(12); NX_SK(13); NX_SK(14); NX_SK(15); NX_SK(16);
-  }
-#undef NX_SK
-  return launch_status();
-}
-
 extern "C" int nx_gather_rows(const void* x, const int32_t* rows, void* out, int n, int cols, nx_stream_t stream) {
   if (n <= 0) return 0;
   if (cols & 7) return -1;
@@ -986,7 +908,7 @@ extern "C" int nx_gated_bwd(const void* h, const void* dy, void* dh, int64_t n, 
 
 extern "C" int nx_wq_gemv(const void* x, int64_t ldx, const void* wq, const float* scales, int bits, int group,
                           const void* bias, void* y, int64_t ldy, int m, int n, int k, nx_stream_t stream) {
-  if (m < 1 || m > kSkinnyMaxRows || (k & 7) || (bits != 8 && bits != 4)) return -1;
+  if (m < 1 || m > kGemvMaxRows || (k & 7) || (bits != 8 && bits != 4)) return -1;
   if (bits == 4 && (group <= 0 || (group & 7) || k % group)) return -1;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int blocks = (n + 7) / 8;

@@ -39,12 +39,14 @@ typedef struct NxPagedArgs {
 int nx_paged_attention_decode(const NxPagedArgs* args, nx_stream_t stream);
 
 // y[m][n] = act(x[m][:] . w[n][:] + bias[n]) + residual[m][n], 1 <= m <= nx_skinny_max_rows().
-// The reduction order of a row is fixed, so a row's result does not depend on the batch it is in.
+// The reduction order of a row is fixed, so a row's result does not depend on the batch it is in (one order for up to 16 rows,
+// another above).
 int nx_skinny_max_rows(void);
-// y and residual share out_dtype (BF16 or FP32); y may alias residual.
+// y and residual share out_dtype (BF16 or FP32); y may alias residual.  `w_const`: no kernel that may still be running on the
+// device writes w (weights of a loaded model): they are fetched while the kernel before this one finishes.
 int nx_skinny_gemm(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* bias, const void* residual,
                    int64_t ldr, void* y, int64_t ldy, int out_dtype, int m, int n, int k, int act,
-                   nx_stream_t stream);
+                   int w_const, nx_stream_t stream);
 
 int nx_gather_rows(const void* x, const int32_t* rows, void* out, int n, int cols, nx_stream_t stream);
 // counts[row_of[i]][tokens[i]] += 1

@@ -539,13 +539,20 @@ class Engine:
                 return residual.add_(y)
             return y if od == torch.bfloat16 else y.to(od)
         w = lin.dense()
-        if n <= self._skinny:
-            return I.skinny_gemm(x, w, lin.bias, act=act, residual=residual, out=residual, out_dtype=od)
+        if self._few_rows(n, lin.n, lin.k):
+            return I.skinny_gemm(x, w, lin.bias, act=act, residual=residual, out=residual, out_dtype=od, w_const=lin.quant == "bf16")
         # a few rows give the tensor-core GEMM one row of tiles: slices along K keep every SM busy (fixed summation
         # order, so a row's result does not depend on what else is in the batch)
         few = n < 256
         return K.gemm(x, w, bias=lin.bias, act=act, residual=residual, out=residual, out_dtype=od,
                       split_k=0 if few else 1, block_n=128 if few else 0, deterministic=True)
+
+    def _few_rows(self, rows: int, n: int, k: int) -> bool:
+        """Whether a product reads its weights once, straight into registers: up to 16 rows always; up to 64 where the split tcgen05
+        product with its reduction pass is slower (64 rows: 7.2 against 12.4 us at 1600 x 1600, 12.8 against 16.7 at 6400 x 1600,
+        8.7 against 10.6 at 768 x 3072) and not where it is faster (20.1 against 15.9 at 1600 x 6400; vocabularies, whose tiles
+        fill the machine unsplit: 76 against 39 at 50304 x 1600)."""
+        return rows <= self._skinny or (rows <= 64 and k <= 3072 and n < 16384)
 
     def _norm(self, x, w, b):
         if not self.fast:
@@ -727,8 +734,8 @@ class Engine:
         hf = self._norm(xr, self.lnf_w, self.lnf_b)
         if not self.fast:
             return hf @ self.wte.t()
-        if R <= self._skinny:
-            return I.skinny_gemm(hf, self.wte, out_dtype=torch.float32)
+        if self._few_rows(R, self.Vp, self.d):
+            return I.skinny_gemm(hf, self.wte, out_dtype=torch.float32, w_const=True)
         return K.gemm(hf, self.wte, out_dtype=torch.float32)
 
     def _splits(self, rows: int) -> int:

@@ -66,8 +66,9 @@ def paged_attention(q, k_cache, v_cache, block_table, row_seq, ctx_len, out, *, 
     return out
 
 
-def skinny_gemm(x, w, bias=None, *, act=None, residual=None, out=None, out_dtype=None) -> torch.Tensor:
-    """y = act(x @ w^T + bias) + residual for 1 <= rows <= skinny_max_rows(); w is [n, k]."""
+def skinny_gemm(x, w, bias=None, *, act=None, residual=None, out=None, out_dtype=None, w_const=False) -> torch.Tensor:
+    """y = act(x @ w^T + bias) + residual for 1 <= rows <= skinny_max_rows(); w is [n, k].  ``w_const``: w is written by no kernel
+    that may still be running (the weights of a loaded model), so it may be read before the kernel in front has finished."""
     m, k = x.shape
     n = w.shape[0]
     if out is None:
@@ -78,7 +79,7 @@ def skinny_gemm(x, w, bias=None, *, act=None, residual=None, out=None, out_dtype
     K._check(K.lib().nx_skinny_gemm(K._p(x), C.c_int64(x.stride(0)), K._p(w), C.c_int64(w.stride(0)), K._p(bias),
                                     K._p(residual), C.c_int64(residual.stride(0) if residual is not None else 0),
                                     K._p(out), C.c_int64(out.stride(0)), C.c_int(K._DT[out.dtype]), C.c_int(m),
-                                    C.c_int(n), C.c_int(k), C.c_int(K.ACT[act]), K._stream()), "nx_skinny_gemm")
+                                    C.c_int(n), C.c_int(k), C.c_int(K.ACT[act]), C.c_int(int(w_const)), K._stream()), "nx_skinny_gemm")
     return out
 
 

@@ -300,3 +300,41 @@ def test_gated_pieces_and_single_elements(n, f, act):
     # BF16 results: half of the last of 8 bits is up to 2^-8 of the value; and 1e-6 of the factors (up to about 20)
     for got, ref in ((I.gated_fwd(h, act), want), (I.gated_bwd(h, dy, act), hr.grad)):
         assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all()
+
+
+@pytest.mark.parametrize("n,k,dtype", [(64, 64, "f32"), (1, 8, "bf16"), (130, 776, "bf16"), (770, 1600, "f32"), (2400, 768, "bf16"),
+                                       (20000, 264, "f32"), (33, 4104, "bf16")])
+def test_few_rows_at_the_edges_of_its_tiles(n, k, dtype):
+    """Every size class of rows and its neighbours, columns and reductions that fill no tile, padded pitches; a row alone gives the same
+    bits as in any batch of its form.  FP32 sums of BF16 products: 2^-20 per result of order 1; BF16 results 2^-8 of up to 4."""
+    K, I = _mods()
+    torch.manual_seed(2)
+    ld = (k + 7) // 8 * 8 + 8
+    x = torch.randn(64, ld, device="cuda").bfloat16()[:, :k]
+    w = (torch.randn(n, ld, device="cuda") * k ** -0.5).bfloat16()[:, :k]
+    b = torch.randn(n, device="cuda").bfloat16()
+    od = {"f32": torch.float32, "bf16": torch.bfloat16}[dtype]
+    want = x.double() @ w.double().t()
+    res = torch.randn(64, n, device="cuda").to(od)
+    tol = 1e-4 if dtype == "f32" else 2e-2
+    for most, sizes in ((16, (1, 2, 3, 4, 5, 6, 7, 8, 9, 12, 13)), (64, (17, 24, 32, 33, 63))):     # the two forms
+        first = I.skinny_gemm(x[:most], w, out_dtype=od)
+        assert (first.double() - want[:most]).abs().max() < tol
+        for m in sizes:
+            for const in (False, True):
+                assert torch.equal(I.skinny_gemm(x[:m], w, out_dtype=od, w_const=const), first[:m]), m
+    for m in (1, 3, 14, 40, 64):
+        buf = torch.full((m, n + 3), 9.0, device="cuda", dtype=od)      # a pitch that takes no vector accesses
+        y = buf[:, :n]
+        y.copy_(res[:m])
+        I.skinny_gemm(x[:m], w, b, act="relu", residual=y, out=y)
+        assert (y.double() - (torch.relu(want[:m] + b.double()) + res[:m].double())).abs().max() < 2 * tol
+        assert (buf[:, n:] == 9.0).all()
+
+
+def test_few_rows_refuses_what_it_cannot_address():
+    K, I = _mods()
+    x, w = torch.zeros(65, 64, device="cuda").bfloat16(), torch.zeros(8, 64, device="cuda").bfloat16()
+    for bad in (lambda: I.skinny_gemm(x, w), lambda: I.skinny_gemm(x[:4, 1:9], w[:, :8]), lambda: I.skinny_gemm(x[:4, :12], w[:, :12])):
+        with pytest.raises(RuntimeError):
+            bad()
