@@ -28,6 +28,8 @@ __device__ __forceinline__ void unpack8(const uint4& q, float (&v)[8]) {
 __global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
                                  int64_t k_row_stride, int64_t v_row_stride, const int32_t* __restrict__ slots,
                                  __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc, int tokens, int hd) {
+  pdl_trigger();
+  pdl_dependency();
   const int vec = hd >> 3;  // Hkv*D in 16-byte vectors
   NX_GRID_STRIDE(i, static_cast<int64_t>(tokens) * vec) {
     const int t = static_cast<int>(i / vec), c = static_cast<int>(i % vec);
@@ -236,6 +238,8 @@ paged_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
                         const int32_t* __restrict__ ctx_len, int heads, int kv_heads, float scale, int splits,
                         __nv_bfloat16* __restrict__ out, int64_t o_row_stride, float* __restrict__ part_o,
                         float* __restrict__ part_ml, int* __restrict__ status) {
+  pdl_trigger();
+  pdl_dependency();
   constexpr int LPT = D / 8;          // lanes per token
   constexpr int TPP = 128 / LPT;      // tokens per pass of the block (16 at D = 64, 8 at D = 128)
   constexpr int kPage = 16;
@@ -343,6 +347,8 @@ paged_decode_tma_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 template <int D>
 __global__ void paged_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, int splits,
                                      int heads, __nv_bfloat16* __restrict__ out, int64_t o_row_stride) {
+  pdl_trigger();
+  pdl_dependency();
   const int row = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const int64_t base = (static_cast<int64_t>(row) * heads + h) * splits;
   float gm = -INFINITY;
@@ -752,8 +758,7 @@ extern "C" int nx_kv_append(const void* k, const void* v, int64_t k_row_stride, 
   const int hd = kv_heads * D;
   if (kv_kind == 0) {
     if (hd & 7) return -1;
-    kv_append_kernel<<<blocks_for(static_cast<int64_t>(tokens) * (hd / 8), 256), 256, 0, st>>>(
-        (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, k_row_stride, v_row_stride, slots, (__nv_bfloat16*)kc,
+    NX_PDL((kv_append_kernel), blocks_for(static_cast<int64_t>(tokens) * (hd / 8), 256), 256, 0, st, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, k_row_stride, v_row_stride, slots, (__nv_bfloat16*)kc,
         (__nv_bfloat16*)vc, tokens, hd);
   } else {
     const int warps = tokens * kv_heads;
@@ -790,7 +795,7 @@ extern "C" int nx_paged_attention_decode(const NxPagedArgs* a, nx_stream_t strea
       return -3;
     const int smem = 2 * kPagedStages * 16 * D * 2 + kPagedStages * 8;
     if (D == 64)
-      paged_decode_tma_kernel<64><<<grid, 128, smem, st>>>(tk, tv, (const __nv_bfloat16*)a->q, a->q_row_stride, a->block_table,
+      NX_PDL((paged_decode_tma_kernel<64>), grid, 128, smem, st, tk, tv, (const __nv_bfloat16*)a->q, a->q_row_stride, a->block_table,
           a->max_blocks, a->row_seq, a->ctx_len, a->heads, a->kv_heads, a->scale, splits, (__nv_bfloat16*)a->out,
           a->o_row_stride, a->part_o, a->part_ml, a->status);
     else {
@@ -800,7 +805,7 @@ extern "C" int nx_paged_attention_decode(const NxPagedArgs* a, nx_stream_t strea
           return -2;
         once = true;
       }
-      paged_decode_tma_kernel<128><<<grid, 128, smem, st>>>(tk, tv, (const __nv_bfloat16*)a->q, a->q_row_stride, a->block_table,
+      NX_PDL((paged_decode_tma_kernel<128>), grid, 128, smem, st, tk, tv, (const __nv_bfloat16*)a->q, a->q_row_stride, a->block_table,
           a->max_blocks, a->row_seq, a->ctx_len, a->heads, a->kv_heads, a->scale, splits, (__nv_bfloat16*)a->out,
           a->o_row_stride, a->part_o, a->part_ml, a->status);
     }
@@ -808,9 +813,9 @@ extern "C" int nx_paged_attention_decode(const NxPagedArgs* a, nx_stream_t strea
     if (splits > 1) {
       dim3 g2(a->rows, a->heads);
       if (D == 64)
-        paged_combine_kernel<64><<<g2, 64, 0, st>>>(a->part_o, a->part_ml, splits, a->heads, (__nv_bfloat16*)a->out, a->o_row_stride);
+        NX_PDL((paged_combine_kernel<64>), g2, 64, 0, st, a->part_o, a->part_ml, splits, a->heads, (__nv_bfloat16*)a->out, a->o_row_stride);
       else
-        paged_combine_kernel<128><<<g2, 128, 0, st>>>(a->part_o, a->part_ml, splits, a->heads, (__nv_bfloat16*)a->out, a->o_row_stride);
+        NX_PDL((paged_combine_kernel<128>), g2, 128, 0, st, a->part_o, a->part_ml, splits, a->heads, (__nv_bfloat16*)a->out, a->o_row_stride);
     }
     return launch_status();
   }
@@ -828,9 +833,9 @@ extern "C" int nx_paged_attention_decode(const NxPagedArgs* a, nx_stream_t strea
   if (splits > 1) {
     dim3 g2(a->rows, a->heads);
     if (a->head_dim == 64)
-      paged_combine_kernel<64><<<g2, 64, 0, st>>>(a->part_o, a->part_ml, splits, a->heads, (__nv_bfloat16*)a->out, a->o_row_stride);
+      NX_PDL((paged_combine_kernel<64>), g2, 64, 0, st, a->part_o, a->part_ml, splits, a->heads, (__nv_bfloat16*)a->out, a->o_row_stride);
     else
-      paged_combine_kernel<128><<<g2, 128, 0, st>>>(a->part_o, a->part_ml, splits, a->heads, (__nv_bfloat16*)a->out, a->o_row_stride);
+      NX_PDL((paged_combine_kernel<128>), g2, 128, 0, st, a->part_o, a->part_ml, splits, a->heads, (__nv_bfloat16*)a->out, a->o_row_stride);
   }
   return launch_status();
 }

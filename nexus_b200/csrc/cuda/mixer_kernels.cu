@@ -17,6 +17,8 @@ using namespace nx;
 // ------------------------------------------------------------------------------------------------
 template <typename T, int V>
 __global__ void residual_norm_kernel(const NxResidualNormArgs a) {
+  pdl_trigger();
+  pdl_dependency();
   extern __shared__ __align__(16) float s_row[];
   __shared__ float s_red[32];
   const int64_t r = blockIdx.x;
@@ -161,6 +163,8 @@ __global__ void residual_norm_kernel(const NxResidualNormArgs a) {
 // ------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void rope_append_kernel(const NxRopeAppendArgs a) {
+  pdl_trigger();
+  pdl_dependency();
   const int64_t r = blockIdx.x;
   const int half = a.rot_dims / 2;
   T* row = static_cast<T*>(a.proj) + r * a.ld;
@@ -370,6 +374,8 @@ __device__ __forceinline__ void conv_tile(const NxConvArgs& a, Emit emit) {
 
 template <typename T, int TAPS, int V>
 __global__ void conv_silu_kernel(const NxConvArgs a) {
+  pdl_trigger();
+  pdl_dependency();
   T* y = static_cast<T*>(a.y) + (blockIdx.x * blockDim.x + threadIdx.x) * V;
   conv_tile<T, TAPS, V>(a, [&](int64_t row, int, float (&acc)[V]) {
 #pragma unroll
@@ -381,6 +387,8 @@ __global__ void conv_silu_kernel(const NxConvArgs a) {
 // convolution + rotation of neighbouring pairs + value mixing + cache append: a thread's V channels lie in one head
 template <typename T, int TAPS, int V>
 __global__ void conv_rope_kernel(const NxConvRopeArgs a) {
+  pdl_trigger();
+  pdl_dependency();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   const int nq = a.heads * a.dim, nk = a.kv_heads * a.dim, nv = a.kv_heads * a.vdim, half = a.rot_dims / 2;
   const int part = c < nq ? 0 : c < nq + nk ? 1 : 2;                  // q, k, v
@@ -424,6 +432,8 @@ constexpr int kGatedWarpCols = 512;
 
 template <typename T, bool kWarp>
 __global__ void gated_norm_kernel(const NxGatedNormArgs a) {
+  pdl_trigger();
+  pdl_dependency();
   __shared__ float s_red[32];
   const int lanes = kWarp ? 32 : blockDim.x;
   const int64_t item = kWarp ? blockIdx.x * static_cast<int64_t>(blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
@@ -450,6 +460,8 @@ __global__ void gated_norm_kernel(const NxGatedNormArgs a) {
 // the same with vector accesses and the gated values kept in registers: groups of up to 16 values per thread
 template <typename T, int V, bool kWarp>
 __global__ void gated_norm_vec_kernel(const NxGatedNormArgs a) {
+  pdl_trigger();
+  pdl_dependency();
   constexpr int kIter = 16 / V;
   __shared__ float s_red[32];
   const int lanes = kWarp ? 32 : blockDim.x;
@@ -500,6 +512,8 @@ template <typename T>
 __global__ void token_side_kernel(const float* __restrict__ a, int64_t lda, const int32_t* __restrict__ tokens,
                                   const T* __restrict__ table, int64_t ld_table, int offset, T* __restrict__ out,
                                   int64_t ldo, int dim, int rows) {
+  pdl_trigger();
+  pdl_dependency();
   const int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.y) + threadIdx.y;
   if (r >= rows) return;
   const T* e = table + static_cast<int64_t>(tokens[r]) * ld_table + offset;
@@ -514,6 +528,8 @@ __global__ void token_side_kernel(const float* __restrict__ a, int64_t lda, cons
 template <typename T, int V>
 __global__ void glu_kernel(const T* __restrict__ h, int64_t ldh, T* __restrict__ out, int64_t ldo, int half, int interleaved,
                            const NxGlu f) {
+  pdl_trigger();
+  pdl_dependency();
   const int64_t r = blockIdx.y;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (c >= half) return;
@@ -584,14 +600,14 @@ dim3 conv_grid(const NxConvArgs& a, int threads) {
 constexpr int kConvThreads = 128;
 #define NX_CONV_TAPS(KERNEL_, CONV_)                                                                             \
   switch ((CONV_).taps) {                                                                                        \
-    case 1: KERNEL_<T, 1, V><<<conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st>>>(*a); break;             \
-    case 2: KERNEL_<T, 2, V><<<conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st>>>(*a); break;             \
-    case 3: KERNEL_<T, 3, V><<<conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st>>>(*a); break;             \
-    case 4: KERNEL_<T, 4, V><<<conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st>>>(*a); break;             \
-    case 5: KERNEL_<T, 5, V><<<conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st>>>(*a); break;             \
-    case 6: KERNEL_<T, 6, V><<<conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st>>>(*a); break;             \
-    case 7: KERNEL_<T, 7, V><<<conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st>>>(*a); break;             \
-    case 8: KERNEL_<T, 8, V><<<conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st>>>(*a); break;             \
+    case 1: NX_PDL((KERNEL_<T, 1, V>), conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st, *a); break;             \
+    case 2: NX_PDL((KERNEL_<T, 2, V>), conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st, *a); break;             \
+    case 3: NX_PDL((KERNEL_<T, 3, V>), conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st, *a); break;             \
+    case 4: NX_PDL((KERNEL_<T, 4, V>), conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st, *a); break;             \
+    case 5: NX_PDL((KERNEL_<T, 5, V>), conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st, *a); break;             \
+    case 6: NX_PDL((KERNEL_<T, 6, V>), conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st, *a); break;             \
+    case 7: NX_PDL((KERNEL_<T, 7, V>), conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st, *a); break;             \
+    case 8: NX_PDL((KERNEL_<T, 8, V>), conv_grid<V>(CONV_, kConvThreads), kConvThreads, 0, st, *a); break;             \
     default: return -1;                                                                                          \
   }                                                                                                              \
   return launch_status()
@@ -619,8 +635,8 @@ int launch_residual(const NxResidualNormArgs* a, cudaStream_t st) {
                               : cudaFuncSetAttribute(residual_norm_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return -2;
   }
-  if (vec) residual_norm_kernel<T, 4><<<a->rows, threads, smem, st>>>(*a);
-  else residual_norm_kernel<T, 1><<<a->rows, threads, smem, st>>>(*a);
+  if (vec) NX_PDL((residual_norm_kernel<T, 4>), a->rows, threads, smem, st, *a);
+  else NX_PDL((residual_norm_kernel<T, 1>), a->rows, threads, smem, st, *a);
   return launch_status();
 }
 
@@ -649,8 +665,8 @@ extern "C" int nx_rope_append(const NxRopeAppendArgs* a, nx_stream_t stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int work = std::max(a->heads * a->rot_dims / 2, a->kv_heads * std::max(a->dim, a->vdim));
   const int threads = std::max(64, std::min(256, (work + 31) / 32 * 32));
-  if (a->dtype == NX_BF16) rope_append_kernel<__nv_bfloat16><<<a->rows, threads, 0, st>>>(*a);
-  else if (a->dtype == NX_F32) rope_append_kernel<float><<<a->rows, threads, 0, st>>>(*a);
+  if (a->dtype == NX_BF16) NX_PDL((rope_append_kernel<__nv_bfloat16>), a->rows, threads, 0, st, *a);
+  else if (a->dtype == NX_F32) NX_PDL((rope_append_kernel<float>), a->rows, threads, 0, st, *a);
   else return -1;
   return launch_status();
 }
@@ -758,21 +774,21 @@ extern "C" int nx_gated_norm(const NxGatedNormArgs* a, nx_stream_t stream) {
   if (a->dtype == NX_BF16 && a->group_size % 8 == 0 && a->ldy % 8 == 0 && a->ldz % 8 == 0 && a->ldo % 8 == 0 && al(a->y) && al(a->z) &&
       al(a->out) && al(a->w) && a->group_size <= 16384) {
     if (a->group_size <= 512) {
-      gated_norm_vec_kernel<__nv_bfloat16, 8, true><<<static_cast<int>((items + 7) / 8), 256, 0, st>>>(*a);
+      NX_PDL((gated_norm_vec_kernel<__nv_bfloat16, 8, true>), static_cast<int>((items + 7) / 8), 256, 0, st, *a);
     } else {
       const int threads = std::max(64, (a->group_size / 16 + 31) / 32 * 32);
-      gated_norm_vec_kernel<__nv_bfloat16, 8, false><<<static_cast<int>(items), threads, 0, st>>>(*a);
+      NX_PDL((gated_norm_vec_kernel<__nv_bfloat16, 8, false>), static_cast<int>(items), threads, 0, st, *a);
     }
     return launch_status();
   }
   if (a->group_size <= kGatedWarpCols) {
     const int blocks = static_cast<int>((items + 7) / 8);
-    if (a->dtype == NX_BF16) gated_norm_kernel<__nv_bfloat16, true><<<blocks, 256, 0, st>>>(*a);
-    else gated_norm_kernel<float, true><<<blocks, 256, 0, st>>>(*a);
+    if (a->dtype == NX_BF16) NX_PDL((gated_norm_kernel<__nv_bfloat16, true>), blocks, 256, 0, st, *a);
+    else NX_PDL((gated_norm_kernel<float, true>), blocks, 256, 0, st, *a);
   } else {
     const int threads = std::min(512, (a->group_size / 4 + 31) / 32 * 32);
-    if (a->dtype == NX_BF16) gated_norm_kernel<__nv_bfloat16, false><<<static_cast<int>(items), threads, 0, st>>>(*a);
-    else gated_norm_kernel<float, false><<<static_cast<int>(items), threads, 0, st>>>(*a);
+    if (a->dtype == NX_BF16) NX_PDL((gated_norm_kernel<__nv_bfloat16, false>), static_cast<int>(items), threads, 0, st, *a);
+    else NX_PDL((gated_norm_kernel<float, false>), static_cast<int>(items), threads, 0, st, *a);
   }
   return launch_status();
 }
@@ -786,10 +802,10 @@ extern "C" int nx_token_side_gate(const float* a, int64_t lda, const int32_t* to
   const dim3 threads(tx, ty);
   const int blocks = (rows + ty - 1) / ty;
   if (dtype == NX_BF16)
-    token_side_kernel<__nv_bfloat16><<<blocks, threads, 0, st>>>(a, lda, tokens, (const __nv_bfloat16*)table,
+    NX_PDL((token_side_kernel<__nv_bfloat16>), blocks, threads, 0, st, a, lda, tokens, (const __nv_bfloat16*)table,
                                                                ld_table, offset, (__nv_bfloat16*)out, ldo, dim, rows);
   else if (dtype == NX_F32)
-    token_side_kernel<float><<<blocks, threads, 0, st>>>(a, lda, tokens, (const float*)table, ld_table, offset,
+    NX_PDL((token_side_kernel<float>), blocks, threads, 0, st, a, lda, tokens, (const float*)table, ld_table, offset,
                                                        (float*)out, ldo, dim, rows);
   else
     return -1;
@@ -807,7 +823,7 @@ extern "C" int nx_glu(const void* h, int64_t ldh, void* out, int64_t ldo, int ro
     const int n = std::min(65535, rows - r0);
     dim3 grid((half / (vec ? 8 : 1) + 127) / 128, n);
 #define NX_SM(T_, V_) \
-  glu_kernel<T_, V_><<<grid, 128, 0, st>>>((const T_*)h + r0 * ldh, ldh, (T_*)out + r0 * ldo, ldo, half, interleaved, glu)
+  NX_PDL((glu_kernel<T_, V_>), grid, 128, 0, st, (const T_*)h + r0 * ldh, ldh, (T_*)out + r0 * ldo, ldo, half, interleaved, glu)
     if (dtype == NX_BF16) { if (vec) NX_SM(__nv_bfloat16, 8); else NX_SM(__nv_bfloat16, 1); }
     else if (dtype == NX_F32) { if (vec) NX_SM(float, 8); else NX_SM(float, 1); }
     else return -1;

@@ -133,6 +133,7 @@ norm_fwd_reg_kernel(const XT* __restrict__ x, const XT* __restrict__ res, XT* __
                     const PT* __restrict__ gamma, const PT* __restrict__ beta, YT* __restrict__ y,
                     float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols, float eps) {
   pdl_trigger();
+  pdl_dependency();
   const int kCols = kTail ? cols : 128 * VPL, nvec = kCols >> 2;
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -238,6 +239,7 @@ norm_fwd_block_kernel(const XT* __restrict__ x, const XT* __restrict__ res, XT* 
                       const PT* __restrict__ gamma, const PT* __restrict__ beta, YT* __restrict__ y,
                       float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols, float eps) {
   pdl_trigger();
+  pdl_dependency();
   __shared__ float s_scratch[32];
   const int nvec = cols >> 2;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -430,10 +432,10 @@ int launch_fwd(bool rms, const void* x, const void* res, void* sum_out, const vo
 #define NX_FWD_REG(V_, TAIL_)                                                                                                  \
   {                                                                                                                            \
     if (rms)                                                                                                                   \
-      norm_fwd_reg_kernel<XT, PT, YT, true, V_, TAIL_><<<few_blocks, 32 * few_wpb, 0, st>>>(                                   \
+      NX_PDL((norm_fwd_reg_kernel<XT, PT, YT, true, V_, TAIL_>), few_blocks, 32 * few_wpb, 0, st, \
           (const XT*)x, (const XT*)res, (XT*)sum_out, (const PT*)gamma, (const PT*)beta, (YT*)y, mean, rstd, rows, cols, eps); \
     else                                                                                                                       \
-      norm_fwd_reg_kernel<XT, PT, YT, false, V_, TAIL_><<<few_blocks, 32 * few_wpb, 0, st>>>(                                  \
+      NX_PDL((norm_fwd_reg_kernel<XT, PT, YT, false, V_, TAIL_>), few_blocks, 32 * few_wpb, 0, st, \
           (const XT*)x, (const XT*)res, (XT*)sum_out, (const PT*)gamma, (const PT*)beta, (YT*)y, mean, rstd, rows, cols, eps); \
     return launch_status();                                                                                                    \
   }
@@ -457,10 +459,10 @@ int launch_fwd(bool rms, const void* x, const void* res, void* sum_out, const vo
 #define NX_FWD_BLOCK(V_)                                                                                                       \
   {                                                                                                                            \
     if (rms)                                                                                                                   \
-      norm_fwd_block_kernel<XT, PT, YT, true, V_><<<grid, threads, 0, st>>>(                                                   \
+      NX_PDL((norm_fwd_block_kernel<XT, PT, YT, true, V_>), grid, threads, 0, st, \
           (const XT*)x, (const XT*)res, (XT*)sum_out, (const PT*)gamma, (const PT*)beta, (YT*)y, mean, rstd, rows, cols, eps); \
     else                                                                                                                       \
-      norm_fwd_block_kernel<XT, PT, YT, false, V_><<<grid, threads, 0, st>>>(                                                  \
+      NX_PDL((norm_fwd_block_kernel<XT, PT, YT, false, V_>), grid, threads, 0, st, \
           (const XT*)x, (const XT*)res, (XT*)sum_out, (const PT*)gamma, (const PT*)beta, (YT*)y, mean, rstd, rows, cols, eps); \
     return launch_status();                                                                                                    \
   }

@@ -235,6 +235,8 @@ paged_prefill_kernel(const NxPagedWindowArgs a, int rt, int tq, int head_tiles) 
 template <int DP, bool kBias>
 __global__ void __launch_bounds__(128)
 paged_decode_mma_kernel(const NxPagedWindowArgs a, int head_tiles) {
+  pdl_trigger();
+  pdl_dependency();
   constexpr int LD = DP + 8;
   extern __shared__ __align__(16) __nv_bfloat16 sm[];
   __nv_bfloat16* sQ = sm;                       // [16][LD]
@@ -384,6 +386,8 @@ paged_decode_mma_kernel(const NxPagedWindowArgs a, int head_tiles) {
 }
 
 __global__ void paged_decode_merge_kernel(const NxPagedWindowArgs a) {
+  pdl_trigger();
+  pdl_dependency();
   const int sg = blockIdx.x, h = blockIdx.y;
   if (a.seg.len[sg] <= 0) return;
   const int64_t base = (static_cast<int64_t>(sg) * a.heads + h) * a.splits, row = a.seg.row0[sg];
@@ -504,7 +508,7 @@ int launch_decode_as(const NxPagedWindowArgs* a, dim3 grid, int head_tiles, cuda
     if (cudaFuncSetAttribute(paged_decode_mma_kernel<DP, kBias>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return -2;
     once = true;
   }
-  paged_decode_mma_kernel<DP, kBias><<<grid, 128, kSmem, st>>>(*a, head_tiles);
+  NX_PDL((paged_decode_mma_kernel<DP, kBias>), grid, 128, kSmem, st, *a, head_tiles);
   return launch_status();
 }
 template <int DP>
@@ -546,7 +550,7 @@ extern "C" int nx_paged_window_decode(const NxPagedWindowArgs* a, nx_stream_t st
     default: return -1;
   }
   if (rc == 0 && a->splits > 1) {
-    paged_decode_merge_kernel<<<dim3(a->seg.count, a->heads), std::min(256, (a->vdim + 31) / 32 * 32), 0, st>>>(*a);
+    NX_PDL((paged_decode_merge_kernel), dim3(a->seg.count, a->heads), std::min(256, (a->vdim + 31) / 32 * 32), 0, st, *a);
     rc = launch_status();
   }
   return rc;

@@ -40,6 +40,8 @@ __device__ __forceinline__ void store_state(const float* s, float* g, int rows, 
 // grid (heads, column tiles, segments); shared: state [N][tile] | B [N] | C [N] | partial sums [groups of rows][tile]
 template <typename T>
 __global__ void __launch_bounds__(kStepThreads) ssd_step_kernel(const NxSsdArgs a, int tile) {
+  pdl_trigger();
+  pdl_dependency();
   extern __shared__ __align__(16) float smem[];
   const int h = blockIdx.x, p0 = blockIdx.y * tile, sg = blockIdx.z;
   const int len = a.seg.len[sg];
@@ -95,6 +97,8 @@ __global__ void __launch_bounds__(kStepThreads) ssd_step_kernel(const NxSsdArgs 
 // grid (heads, column tiles, segments); shared: state [D][tile] | k [D] | q [D] | partial sums [2][row groups][tile]
 template <typename T>
 __global__ void __launch_bounds__(kStepThreads) delta_step_kernel(const NxDeltaArgs a, int tile) {
+  pdl_trigger();
+  pdl_dependency();
   extern __shared__ __align__(16) float smem[];
   const int h = blockIdx.x, v0 = blockIdx.y * tile, sg = blockIdx.z;
   const int len = a.seg.len[sg];
@@ -251,10 +255,10 @@ extern "C" int nx_ssd_step(const NxSsdArgs* a, nx_stream_t stream) {
   dim3 grid(a->heads, (a->vdim + tile - 1) / tile, a->seg.count);
   if (a->dtype == NX_BF16) {
     if (set_smem(ssd_step_kernel<__nv_bfloat16>, smem)) return -2;
-    ssd_step_kernel<__nv_bfloat16><<<grid, kStepThreads, smem, st>>>(*a, tile);
+    NX_PDL((ssd_step_kernel<__nv_bfloat16>), grid, kStepThreads, smem, st, *a, tile);
   } else if (a->dtype == NX_F32) {
     if (set_smem(ssd_step_kernel<float>, smem)) return -2;
-    ssd_step_kernel<float><<<grid, kStepThreads, smem, st>>>(*a, tile);
+    NX_PDL((ssd_step_kernel<float>), grid, kStepThreads, smem, st, *a, tile);
   } else {
     return -1;
   }
@@ -272,10 +276,10 @@ extern "C" int nx_delta_step(const NxDeltaArgs* a, nx_stream_t stream) {
   dim3 grid(a->heads, (a->vdim + tile - 1) / tile, a->seg.count);
   if (a->dtype == NX_BF16) {
     if (set_smem(delta_step_kernel<__nv_bfloat16>, smem)) return -2;
-    delta_step_kernel<__nv_bfloat16><<<grid, kStepThreads, smem, st>>>(*a, tile);
+    NX_PDL((delta_step_kernel<__nv_bfloat16>), grid, kStepThreads, smem, st, *a, tile);
   } else if (a->dtype == NX_F32) {
     if (set_smem(delta_step_kernel<float>, smem)) return -2;
-    delta_step_kernel<float><<<grid, kStepThreads, smem, st>>>(*a, tile);
+    NX_PDL((delta_step_kernel<float>), grid, kStepThreads, smem, st, *a, tile);
   } else {
     return -1;
   }

@@ -21,6 +21,8 @@ template <typename WT, typename OT>
 __global__ void embedding_pos_fwd_kernel(const int32_t* __restrict__ tokens, const int32_t* __restrict__ positions,
                                          const WT* __restrict__ wte, const WT* __restrict__ wpe, OT* __restrict__ out,
                                          int64_t rows, int seq_len, int cols) {
+  pdl_trigger();
+  pdl_dependency();
   const int vec = cols >> 2;
   NX_GRID_STRIDE(i, rows * vec) {
     const int64_t r = i / vec;
@@ -668,7 +670,7 @@ extern "C" int nx_embedding_pos_fwd(const int32_t* tokens, const int32_t* positi
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int blocks = blocks_for(rows * (cols / 4), 256);
 #define NX_E(WT, OT)                                                                                          \
-  embedding_pos_fwd_kernel<WT, OT><<<blocks, 256, 0, st>>>(tokens, positions, (const WT*)wte, (const WT*)wpe, \
+  NX_PDL((embedding_pos_fwd_kernel<WT, OT>), blocks, 256, 0, st, tokens, positions, (const WT*)wte, (const WT*)wpe, \
                                                            (OT*)out, rows, seq_len, cols)
   if (w_dtype == NX_F32 && out_dtype == NX_F32) NX_E(float, float);
   else if (w_dtype == NX_F32 && out_dtype == NX_BF16) NX_E(float, __nv_bfloat16);
