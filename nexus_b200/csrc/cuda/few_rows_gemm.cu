@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(128, M > 8 ? 2 : (M > 2 ? 3 : 5)) skinny_kerne
   }
 }
 
-// The same sums with a column per warp and no prefetch of its own: many small warps per SM instead.
+// The same sums of exactly M rows with a column per warp and no prefetch of its own: many small warps per SM instead.
 template <int M, typename YT>
 __global__ void __launch_bounds__(256) skinny_wide_kernel(const FewRowsArgs a) {
   const int col = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(256) skinny_wide_kernel(const FewRowsArgs a) {
   float acc[M];
 #pragma unroll
   for (int i = 0; i < M; ++i) acc[i] = 0.0f;
+  const __nv_bfloat16* __restrict__ x = a.x;
+  const int64_t ldx = a.ldx;
   const __nv_bfloat16* wr = a.w + static_cast<int64_t>(col) * a.ldw;
   for (int c = lane * 8; c < a.k; c += 256) {
     float wv[8];
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(256) skinny_wide_kernel(const FewRowsArgs a) {
 #pragma unroll
     for (int i = 0; i < M; ++i) {
       float xv[8];
-      unpack8(*reinterpret_cast<const uint4*>(a.x + min(i, a.m - 1) * a.ldx + c), xv);
+      unpack8(*reinterpret_cast<const uint4*>(x + i * ldx + c), xv);
       float t = 0.0f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) t += xv[j] * wv[j];
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(256) skinny_wide_kernel(const FewRowsArgs a) {
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == i) sum = t;
   }
-  if (lane >= M || lane >= a.m) return;
+  if (lane >= M) return;
   float v = apply_act(sum + (a.bias != nullptr ? __bfloat162float(a.bias[col]) : 0.0f), a.act);
   if (a.residual != nullptr) v += Num<YT>::load(static_cast<const YT*>(a.residual) + lane * a.ldr + col);
   Num<YT>::store(static_cast<YT*>(a.y) + lane * a.ldy + col, v);
@@ -201,19 +203,21 @@ int launch_skinny(const FewRowsArgs& a, cudaStream_t st) {
   // 3 to 8 rows: columns per warp share what a row costs besides its products, but there have to be warps enough to have most of
   // the matrix requested at once (sixteen per SM at four columns, eight at two).  8 rows, one column per warp without prefetch and
   // now: 15.5 -> 8.8 us at 768 x 3072, 31.3 -> 17.3 at 1600 x 6400, 38.7 -> 33.3 at 32000 x 1024.
-  // 1, 2 and 9 to 16 rows: prefetch while the columns do not fill the machine with warps by themselves (one row: 6.4 -> 4.6 us at
-  // 1024 x 4096, but 16.1 against 25.9 us at 50304 x 768; 16 rows: 26.7 -> 13.7 us at 768 x 3072, but 24.1 against 28.2 at
-  // 4800 x 1600).
-  const bool four = a.n >= 4 * 16 * kNumSmsB200, two = a.n >= 2 * 8 * kNumSmsB200, many = a.n > (a.m > 8 ? 16 : 28) * kNumSmsB200;
-#define NX_SK(M_)                                                                                                                     \
-  if (a.m <= M_) {                                                                                                                    \
-    if constexpr (M_ > 2 && M_ <= 8) {                                                                                                \
-      if (four) return launch_skinny_as<M_, 4, YT>(a, st);                                                                            \
-      if (two) return launch_skinny_as<M_, 2, YT>(a, st);                                                                             \
-    } else {                                                                                                                          \
-      if (many) return launch_pdl(skinny_wide_kernel<M_, YT>, dim3(static_cast<unsigned>((a.n + 7) / 8)), dim3(256), 0, st, a);       \
-    }                                                                                                                                 \
-    return launch_skinny_as<M_, 1, YT>(a, st);                                                                                        \
+  // 1, 2 and 9 to 16 rows: prefetch while the columns do not fill the machine with warps by themselves (one row: 6.4 -> 5.3 us at
+  // 1024 x 4096, but 15.6 without against 25.9 us at 50304 x 768; 16 rows: 26.7 -> 13.7 us at 768 x 3072, but 12.5 against 18.3 at
+  // 4128 x 1024).
+  const bool four = a.n >= 4 * 16 * kNumSmsB200, two = a.n >= 2 * 8 * kNumSmsB200, many = a.n > (a.m > 8 ? 16 : 20) * kNumSmsB200;
+#define NX_WIDE(M_) \
+  if (many && a.m == M_) return launch_pdl(skinny_wide_kernel<M_, YT>, dim3(static_cast<unsigned>((a.n + 7) / 8)), dim3(256), 0, st, a);
+  NX_WIDE(1) NX_WIDE(2) NX_WIDE(9) NX_WIDE(10) NX_WIDE(11) NX_WIDE(12) NX_WIDE(13) NX_WIDE(14) NX_WIDE(15) NX_WIDE(16)
+#undef NX_WIDE
+#define NX_SK(M_)                                                  \
+  if (a.m <= M_) {                                                 \
+    if constexpr (M_ > 2 && M_ <= 8) {                             \
+      if (four) return launch_skinny_as<M_, 4, YT>(a, st);         \
+      if (two) return launch_skinny_as<M_, 2, YT>(a, st);          \
+    }                                                              \
+    return launch_skinny_as<M_, 1, YT>(a, st);                     \
   }
   NX_SK(1) NX_SK(2) NX_SK(3) NX_SK(4) NX_SK(6) NX_SK(8) NX_SK(12) NX_SK(16)
 #undef NX_SK
@@ -394,9 +398,11 @@ extern "C" int nx_skinny_gemm(const void* x, int64_t ldx, const void* w, int64_t
           (residual == nullptr || (!(reinterpret_cast<uintptr_t>(residual) & align) && !(ldr & 3)));
   const int blocks = (n + kCols - 1) / kCols;
   if (blocks > 65535) return -1;
-  // Enough CTAs to have the weights of the whole matrix requested at once (two per SM), at least 64 elements of K each.
+  // Enough CTAs to have the weights of the whole matrix requested at once (two per SM), at least 64 elements of K each, but no more
+  // than are resident at 64 rows (three per SM): a second wave cost 12.6 us against 7.9 at 64 rows of
+  // 4128 x 1024, 15.6 against 13.9 at 8192 x 1024.
   int parts = 1;
-  while (parts < 8 && blocks * parts < 2 * kNumSmsB200 && k >= 2 * parts * 64) parts *= 2;
+  while (parts < 8 && blocks * parts < 2 * kNumSmsB200 && 2 * blocks * parts <= 3 * kNumSmsB200 && k >= 2 * parts * 64) parts *= 2;
   a.k_per = ((k + parts - 1) / parts + 31) / 32 * 32;
 #define NX_FEW(MT_) return out_dtype == NX_F32 ? launch_few<MT_, float>(a, parts, st) : launch_few<MT_, __nv_bfloat16>(a, parts, st)
   if (m <= 32) NX_FEW(4);
