@@ -207,8 +207,13 @@ int launch_skinny(const FewRowsArgs& a, cudaStream_t st) {
   // 1024 x 4096, but 15.6 without against 25.9 us at 50304 x 768; 16 rows: 26.7 -> 13.7 us at 768 x 3072, but 12.5 against 18.3 at
   // 4128 x 1024).
   const bool four = a.n >= 4 * 16 * kNumSmsB200, two = a.n >= 2 * 8 * kNumSmsB200, many = a.n > (a.m > 8 ? 16 : 20) * kNumSmsB200;
-#define NX_WIDE(M_) \
-  if (many && a.m == M_) return launch_pdl(skinny_wide_kernel<M_, YT>, dim3(static_cast<unsigned>((a.n + 7) / 8)), dim3(256), 0, st, a);
+#define NX_WIDE(M_)                                                                                                                  \
+  if (many && a.m == M_) {                                                                                                          \
+    const dim3 grid(static_cast<unsigned>((a.n + 7) / 8));                                                                          \
+    if constexpr (M_ == 1) return launch_pdl(skinny_wide_kernel<M_, YT>, grid, dim3(256), 0, st, a);                                \
+    skinny_wide_kernel<M_, YT><<<grid, 256, 0, st>>>(a);                                                                            \
+    return launch_status();                                                                                                         \
+  }
   NX_WIDE(1) NX_WIDE(2) NX_WIDE(9) NX_WIDE(10) NX_WIDE(11) NX_WIDE(12) NX_WIDE(13) NX_WIDE(14) NX_WIDE(15) NX_WIDE(16)
 #undef NX_WIDE
 #define NX_SK(M_)                                                  \
