@@ -207,6 +207,8 @@ int launch_skinny(const FewRowsArgs& a, cudaStream_t st) {
   // 1024 x 4096, but 15.6 without against 25.9 us at 50304 x 768; 16 rows: 26.7 -> 13.7 us at 768 x 3072, but 12.5 against 18.3 at
   // 4128 x 1024).
   const bool four = a.n >= 4 * 16 * kNumSmsB200, two = a.n >= 2 * 8 * kNumSmsB200, many = a.n > (a.m > 8 ? 16 : 20) * kNumSmsB200;
+  // Of the wide form one row alone is a dependent launch (4128 x 1024: 3.9 -> 3.5 us): with more rows the blocks that wait take warps
+  // from the grid in front (4800 x 1600, dependent and plain: 8.0 and 7.1 us with 2 rows, 27.7 and 25.5 with 16).
 #define NX_WIDE(M_)                                                                                                                  \
   if (many && a.m == M_) {                                                                                                          \
     const dim3 grid(static_cast<unsigned>((a.n + 7) / 8));                                                                          \

@@ -551,8 +551,9 @@ class Engine:
         """Whether a product reads its weights once, straight into registers: up to 16 rows always; up to 64 where the split tcgen05
         product with its reduction pass is slower (64 rows: 7.2 against 12.4 us at 1600 x 1600, 12.8 against 16.7 at 6400 x 1600,
         8.7 against 10.6 at 768 x 3072) and not where it is faster (20.1 against 15.9 at 1600 x 6400; vocabularies, whose tiles
-        fill the machine unsplit: 76 against 39 at 50304 x 1600)."""
-        return rows <= self._skinny or (rows <= 64 and k <= 3072 and n < 16384)
+        fill the machine unsplit: 76 against 39 at 50304 x 1600).  Its time grows with n * k (12.8 us at 10 M, 52 at 33 M), that of
+        the other hardly (16.6 and 19.7): the line lies between."""
+        return rows <= self._skinny or (rows <= 64 and k <= 3072 and n < 16384 and n * k <= 12 << 20)
 
     def _norm(self, x, w, b):
         if not self.fast:
