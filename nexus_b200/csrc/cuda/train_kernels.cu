@@ -261,10 +261,11 @@ __global__ void __launch_bounds__(512, 2) ce_row_vec_kernel(const LT* logits, LT
       se *= ex2_approx((mx - vm) * kL2e);
       mx = vm;
     }
-    // all -inf so far: the differences would be -inf + inf
-    const float neg = mx == -INFINITY ? 0.0f : -mx * kL2e;
+    // The difference first: a product of the maximum, rounded by itself, is off by |mx| 2^-24, which for a masked start of the row
+    // (-1e10, the type's lowest value) is an exponent that overflows.  All -inf so far: -inf - -inf would not be a number.
+    const float base = mx == -INFINITY ? 0.0f : mx;
 #pragma unroll
-    for (int j = 0; j < VN; ++j) se += ex2_approx(fmaf(v[j], kL2e, neg));
+    for (int j = 0; j < VN; ++j) se += ex2_approx((v[j] - base) * kL2e);
     if (kSmooth) {
 #pragma unroll
       for (int j = 0; j < VN; ++j) sl += (v[j] == -INFINITY) ? 0.0f : v[j];

@@ -276,6 +276,42 @@ def test_cross_entropy_gradient_beside_the_logits(V, ld, dt, smoothing):
     assert (err <= (2.0 ** -8 if dt is torch.bfloat16 else 1e-5) * r.grad.abs() + 1e-7).all() and (grad[:, V:] == 0).all()
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [9000, 8997])
+@pytest.mark.parametrize("mask", [-1e9, -1e10, -1e20, -1e30, "lowest"])
+def test_cross_entropy_of_masked_vectors(dt, V, mask):
+    """Large negative finite logits in whole 16-byte vectors from the first column on: one vector, all vectors of the first thread
+    (of 512), all but the target's, none.  Masked entries weigh nothing, as in the 64-bit result: FP32 sums of 9000 terms give 1e-5."""
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(12)
+    mask, ld = torch.finfo(dt).min if mask == "lowest" else mask, 9000
+    n = 16 // torch.empty(0, dtype=dt).element_size()
+    logits = (torch.randn(4, ld, device="cuda") * 3).to(dt)
+    targets = torch.tensor([V - 1, 4500, 4501, 3], device="cuda", dtype=torch.int32)
+    logits[0, :n] = mask
+    for v in range(0, ld, 512 * n):
+        logits[1, v: v + n] = mask
+    kept = logits[2, 4501 // n * n: 4501 // n * n + n].clone()
+    logits[2] = mask
+    logits[2, 4501 // n * n: 4501 // n * n + n] = kept
+    for smoothing in (0.0, 0.1) if abs(mask) < 1e30 else (0.0,):      # the mean of all logits is finite
+        kw = dict(targets=targets, vocab=V, smoothing=smoothing, z_loss=1e-3, seq_len=1)
+        grad, inplace = torch.empty_like(logits), logits.clone()
+        a = K.cross_entropy_shifted(logits, None, grad=grad, **kw)
+        b = K.cross_entropy_shifted(inplace, None, **kw)
+        assert torch.equal(a, b) and torch.equal(grad, inplace)
+        r = logits[:, :V].double().requires_grad_(True)
+        lse = r.logsumexp(1)
+        per = (1 - smoothing) * (lse - r.gather(1, targets.long()[:, None])[:, 0]) + 1e-3 * lse * lse
+        want = (per + (smoothing * (lse - r.mean(1)) if smoothing else 0)).mean()
+        want.backward()
+        assert abs(float(a) - float(want)) <= 1e-5 * max(1.0, abs(float(want)))
+        err = (grad[:, :V].double() - r.grad).abs()
+        assert (err <= (2.0 ** -8 if dt is torch.bfloat16 else 1e-5) * r.grad.abs() + 1e-7).all()
+        if not smoothing:
+            assert (grad[:, :V][logits[:, :V] == mask] == 0).all()
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 516), (64, 1600), (3, 1028), (1300, 2048), (5, 4100), (7, 8192), (2, 8196)])
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("xdt", [torch.float32, torch.bfloat16])
