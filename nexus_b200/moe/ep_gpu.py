@@ -27,6 +27,7 @@ import torch
 
 from ..ops import _cuda as K
 from ..ops import _infer as I
+from .gpu import router_logits
 
 
 class _Table(C.Structure):
@@ -304,7 +305,7 @@ class MoeEpLayer(torch.nn.Module):
 
     def forward(self, x: torch.Tensor):
         ep = self.ep
-        logits = x.float() @ self.router.float().t()
+        logits = router_logits(x, self.router)
         fn = _MoeEpNcclFn if (ep.comm == "nccl" and ep.n > 1) else _MoeEpFn
         y, total = fn.apply(x, logits, self.up, self.down, ep)
         self.last_counts = total

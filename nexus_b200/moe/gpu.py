@@ -42,10 +42,8 @@ def route(logits: torch.Tensor, k: int, capacity: int):
 
 
 def router_logits(x, router_w) -> torch.Tensor:
-    """FP32 logits.  BF16 rows and weights: their products are exact in the tensor cores' FP32 sums; a wider router takes FP32 throughout."""
-    if x.dtype == router_w.dtype == torch.bfloat16 and x.stride(-1) == router_w.stride(-1) == 1 and \
-            all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (x, router_w)):
-        return K.gemm(x, router_w, out_dtype=torch.float32)
+    """FP32 logits of every router.  FP32 products: the tensor cores' sums of the same exact products are 3 to 16 times further from
+    64 bits (2.1e-6 against 1.3e-7 to 3.9e-7 at 2048 columns), and the nearest experts decide by these bits."""
     return x.float() @ router_w.float().t()
 
 
@@ -161,7 +159,7 @@ class _MoeGroupsFn(torch.autograd.Function):
         N, d = x.shape
         E, F2, _ = up.shape
         cap = groups * capacity
-        logits = x.float() @ router_w.float().t()
+        logits = router_logits(x, router_w)
         nl = None
         select = logits
         if noise_w is not None and eps is not None:

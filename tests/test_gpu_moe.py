@@ -127,3 +127,14 @@ def test_moe_router_types_and_odd_sizes(N, d, E, k, cap, rdt):
     # BF16 activations between the products: 2^-9 each over four roundings, with room for the router's cancelling sums
     for g, r, name in zip((y, *got), ref, ("y", "dx", "drouter", "dup", "ddown")):
         assert (g.double() - r).norm() <= 2e-2 * r.norm(), name
+
+
+@pytest.mark.parametrize("N,d,E", [(1111, 2048, 64), (200, 1024, 8)])
+def test_router_logits_are_fp32_sums(N, d, E):
+    """Exact products; d FP32 additions, each rounded to nearest, of partial sums that grow as sqrt(i): about 2.4e-8 sqrt(d / 2) of the
+    result where they are added in turn (7.7e-7 at 2048, 5.4e-7 at 1024), less in pieces.  Sums of less than FP32 are beyond that."""
+    from nexus_b200.moe import gpu as G
+    torch.manual_seed(6)
+    x, r = torch.randn(N, d, device="cuda").bfloat16(), (torch.randn(E, d, device="cuda") * d ** -0.5).bfloat16()
+    want = x.double() @ r.double().t()
+    assert (G.router_logits(x, r).double() - want).norm() <= 2.4e-8 * (d / 2) ** 0.5 * want.norm()
