@@ -38,10 +38,17 @@ __device__ __forceinline__ void store8(T* p, const float (&v)[8]) {
   }
 }
 
+// FP32 to the last bits: the pass is bound by memory, the approximate forms of the GEMM epilogues (tanh to 5e-4) would only lose
+// them.  GELU: t = sigmoid(2 u) = (1 + tanh u) / 2, so that 1 - tanh^2 u = 4 t (1 - t) has no cancellation.
+__device__ __forceinline__ float sigmoid_exact(float x) { return __fdividef(1.0f, 1.0f + expf(-x)); }
 __device__ __forceinline__ float act_grad(float x, float dy, int act) {
-  if (act == NX_ACT_GELU) return dy * dgelu_tanh_f(x);
+  if (act == NX_ACT_GELU) {
+    const float k0 = 0.7978845608028654f, k1 = 0.044715f, x2 = x * x;
+    const float t = sigmoid_exact(2.0f * k0 * (x + k1 * x * x2));
+    return dy * (t + 2.0f * x * t * (1.0f - t) * k0 * (1.0f + 3.0f * k1 * x2));
+  }
   if (act == NX_ACT_SILU) {
-    const float s = 1.0f / (1.0f + __expf(-x));
+    const float s = sigmoid_exact(x);
     return dy * (s * (1.0f + x * (1.0f - s)));
   }
   return x <= 0.0f ? 0.0f : dy;  // relu

@@ -245,6 +245,23 @@ def test_activation_backward(n, act):
         assert ((K.act_bwd(a, b, act).double() - r.grad).abs() <= 2.0 ** -8 * r.grad.abs() + 2e-5).all()
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+def test_activation_backward_rounds_once(act, dt):
+    """FP32 inside: beside the rounding of the result (half a unit in the last place) 2e-6 of the larger of 1 and |x|; tanh to 5e-4
+    would show as 1e-4."""
+    from nexus_b200.ops import _cuda as K
+    torch.manual_seed(13)
+    x = torch.cat([torch.randn(40000, device="cuda") * 2, torch.linspace(-30, 30, 20001, device="cuda"), torch.zeros(1, device="cuda")]).to(dt)
+    dy = torch.ones_like(x)
+    r = x.double().requires_grad_(True)
+    (torch.nn.functional.gelu(r, approximate="tanh") if act == "gelu" else torch.nn.functional.silu(r)).sum().backward()
+    half = torch.finfo(dt).eps / 2
+    floor = torch.finfo(dt).smallest_normal * torch.finfo(dt).eps
+    err = (K.act_bwd(x, dy, act).double() - r.grad).abs()
+    assert (err <= half * r.grad.abs() + 2e-6 * x.double().abs().clamp(min=1.0) + floor).all()
+
+
 @pytest.mark.parametrize("V,ld,dt", [(50, 56, torch.bfloat16), (8192, 8192, torch.bfloat16), (50257, 50304, torch.bfloat16), (101, 101, torch.bfloat16),
                                      (997, 1000, torch.float32), (13, 13, torch.float32)])
 @pytest.mark.parametrize("smoothing", [0.0, 0.1])
