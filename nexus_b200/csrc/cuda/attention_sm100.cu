@@ -326,7 +326,6 @@ template <int HD, int EXT, bool kPacked>  // EXT, row math: 0 plain, 1 soft-capp
 __global__ void __launch_bounds__(kFwdThreads, (HD == 64 ? 2 : 1))
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const AttnDev p) {
-  pdl_launch_dependents();
   using C = FwdCfg<HD>;
   constexpr int HH = HD / 2;  // output columns per softmax thread
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -374,6 +373,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // this block has its tensor memory: a dependent that needs some cannot take it from under it
   pdl_wait();  // the set-up above overlaps the end of the kernel in front
   const uint32_t tmem_s = tmem_base;
   const uint32_t tmem_o = tmem_base + 128;
@@ -705,7 +705,6 @@ template <int HD, bool kPacked>
 __global__ void __launch_bounds__(kFwd2Threads, 1)
 attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const AttnDev p) {
-  pdl_launch_dependents();
   using C = Fwd2Cfg<HD>;
   constexpr int S = C::kStages;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -752,6 +751,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // this block has its tensor memory: a dependent that needs some cannot take it from under it
   pdl_wait();  // the set-up above overlaps the end of the kernel in front
 
   if (warp == 8) {
@@ -1158,7 +1158,6 @@ __global__ void __launch_bounds__(bwd_threads(HD), (HD == 64 ? 2 : 1))
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                      const AttnDev p) {
-  pdl_launch_dependents();
   using C = DkvCfg<HD>;
   constexpr int NS = C::kStages, NT = C::kTiles, NP = C::kPBufs, NC = 32, MW = bwd_math_warps(HD), kSpan = 64 / (MW / 4);  // kSpan: columns of a chunk per math thread
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1227,6 +1226,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // this block has its tensor memory: a dependent that needs some cannot take it from under it
   pdl_wait();  // the set-up above overlaps the end of the kernel in front
   const uint32_t tmem_dv = tmem_base + NT * 128;  // score tile i: S^T at 128 i, dP^T at 128 i + 64
   const uint32_t tmem_dk = tmem_dv + HD;
@@ -1473,7 +1473,6 @@ __global__ void __launch_bounds__(bwd_threads(HD), (HD == 64 ? 2 : 1))
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                    const AttnDev p) {
-  pdl_launch_dependents();
   using C = DqCfg<HD>;
   constexpr int NS = C::kStages, NT = C::kTiles, NC = 32, MW = bwd_math_warps(HD), kSpan = 64 / (MW / 4);  // kSpan: columns of a chunk per math thread
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1533,6 +1532,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // this block has its tensor memory: a dependent that needs some cannot take it from under it
   pdl_wait();  // the set-up above overlaps the end of the kernel in front
   const uint32_t tmem_dq = tmem_base + NT * 128;  // score tile i: S at 128 i, dP at 128 i + 64
 
