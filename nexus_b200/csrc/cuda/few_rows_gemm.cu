@@ -154,20 +154,24 @@ __global__ void __launch_bounds__(128, M > 8 ? 2 : (M > 2 ? 3 : 5)) skinny_kerne
   }
 }
 
-// The same sums of exactly M rows with a column per warp and no prefetch of its own: many small warps per SM instead.
-template <int M, typename YT>
-__global__ void __launch_bounds__(256) skinny_wide_kernel(const FewRowsArgs a) {
+// The same sums of exactly M rows with a column per warp and no prefetch of its own: many small warps per SM instead.  kSpread: lane i
+// finishes row i, otherwise lane 0 finishes them all, which takes fewer registers for some M (M = 12 and 16: 48 against 54, so that an
+// SM holds a block more; with the arguments in a struct 16 rows of 6400 x 1600 took 32.7 us in place of 28.9).
+template <int M, bool kSpread, typename YT>
+__global__ void __launch_bounds__(256)
+skinny_wide_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const __nv_bfloat16* __restrict__ w, int64_t ldw,
+                   const __nv_bfloat16* __restrict__ bias, const YT* residual, int64_t ldr, YT* y, int64_t ldy, int n, int k, int act) {
   const int col = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  pdl_trigger();
-  pdl_dependency();
-  if (col >= a.n) return;
+  if constexpr (kSpread) {
+    pdl_trigger();
+    pdl_dependency();
+  }
+  if (col >= n) return;
   float acc[M];
 #pragma unroll
   for (int i = 0; i < M; ++i) acc[i] = 0.0f;
-  const __nv_bfloat16* __restrict__ x = a.x;
-  const int64_t ldx = a.ldx;
-  const __nv_bfloat16* wr = a.w + static_cast<int64_t>(col) * a.ldw;
-  for (int c = lane * 8; c < a.k; c += 256) {
+  const __nv_bfloat16* wr = w + static_cast<int64_t>(col) * ldw;
+  for (int c = lane * 8; c < k; c += 256) {
     float wv[8];
     unpack8(*reinterpret_cast<const uint4*>(wr + c), wv);
 #pragma unroll
@@ -180,42 +184,92 @@ __global__ void __launch_bounds__(256) skinny_wide_kernel(const FewRowsArgs a) {
       acc[i] += t;
     }
   }
-  float sum = 0.0f;
+  if constexpr (kSpread) {
+    float sum = 0.0f;
 #pragma unroll
-  for (int i = 0; i < M; ++i) {
-    float t = acc[i];
+    for (int i = 0; i < M; ++i) {
+      float t = acc[i];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == i) sum = t;
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == i) sum = t;
+    }
+    if (lane >= M) return;
+    float v = apply_act(sum + (bias != nullptr ? __bfloat162float(bias[col]) : 0.0f), act);
+    if (residual != nullptr) v += Num<YT>::load(residual + lane * ldr + col);
+    Num<YT>::store(y + lane * ldy + col, v);
+  } else {
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      float t = acc[i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      acc[i] = t;
+    }
+    if (lane != 0) return;
+    const float b = bias != nullptr ? __bfloat162float(bias[col]) : 0.0f;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      float v = apply_act(acc[i] + b, act);
+      if (residual != nullptr) v += Num<YT>::load(residual + i * ldr + col);
+      Num<YT>::store(y + i * ldy + col, v);
+    }
   }
-  if (lane >= M) return;
-  float v = apply_act(sum + (a.bias != nullptr ? __bfloat162float(a.bias[col]) : 0.0f), a.act);
-  if (a.residual != nullptr) v += Num<YT>::load(static_cast<const YT*>(a.residual) + lane * a.ldr + col);
-  Num<YT>::store(static_cast<YT*>(a.y) + lane * a.ldy + col, v);
 }
 
 template <int M, int C, typename YT>
 int launch_skinny_as(const FewRowsArgs& a, cudaStream_t st) {
   return launch_pdl(skinny_kernel<M, C, YT>, dim3(static_cast<unsigned>((a.n + 4 * C - 1) / (4 * C))), dim3(128), 0, st, a);
 }
+// Whether lanes finish a row each (1, 2, 13 and 15 rows: always; 11: never, 1 to 5 % faster).  One lane finishes them all where the
+// registers that saves end the grid a wave earlier (4800 x 1600, spread and one lane: 25.0 and 24.2 us with 16 rows; 5120 x 1600 21.8
+// and 19.7 with 12; 6400 x 1600 20.2 and 18.6 with 9), and for the row counts whose loop comes out the faster with it: 12 and 14
+// where the loop outweighs the finish (k = 3072: 2 to 8 %; at k = 768 spread is 3 to 5 % faster), 10, 14 and 16 where the blocks
+// nearly fill their one wave (5120 x 1280 with 10 rows 12.7 and 12.3, 3072 x 768 with 14 8.1 and 7.9, 3840 x 3072 with 16 33.3 and 31.7).
+template <int M, typename YT>
+bool spread_finish(unsigned blocks, int k) {
+  if ((M == 12 || M == 14) && k > 1536) return false;
+  auto per_wave = [](auto kern) {
+    int per_sm = 0;
+    const bool ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) == cudaSuccess && per_sm > 0;
+    return static_cast<unsigned>((ok ? per_sm : 4) * kNumSmsB200);
+  };
+  static const unsigned one = per_wave(skinny_wide_kernel<M, false, YT>), each = per_wave(skinny_wide_kernel<M, true, YT>);
+  const unsigned waves = (blocks + one - 1) / one;
+  if (waves < (blocks + each - 1) / each) return false;
+  return !(waves == 1 && ((M == 10 && blocks > 4 * kNumSmsB200) || (M == 14 && blocks > 2 * kNumSmsB200) || (M == 16 && k > 2048 && blocks > 400)));
+}
+template <int M, typename YT>
+int launch_wide(const FewRowsArgs& a, cudaStream_t st) {
+  const dim3 grid(static_cast<unsigned>((a.n + 7) / 8)), block(256);
+  const YT* res = static_cast<const YT*>(a.residual);
+  YT* y = static_cast<YT*>(a.y);
+  // One row alone is a dependent launch (4128 x 1024: 3.9 -> 3.5 us): with more rows the blocks that wait take warps from the grid in
+  // front (4800 x 1600, dependent and plain: 8.0 and 7.1 us with 2 rows, 27.7 and 25.5 with 16).
+  if constexpr (M == 1) {
+    return launch_pdl(skinny_wide_kernel<M, true, YT>, grid, block, 0, st, a.x, a.ldx, a.w, a.ldw, a.bias, res, a.ldr, y, a.ldy, a.n, a.k, a.act);
+  } else {
+    auto kern = skinny_wide_kernel<M, M != 11, YT>;
+    if constexpr (M != 2 && M != 11 && M != 13 && M != 15) {
+      if (!spread_finish<M, YT>(grid.x, a.k)) kern = skinny_wide_kernel<M, false, YT>;
+    }
+    kern<<<grid, block, 0, st>>>(a.x, a.ldx, a.w, a.ldw, a.bias, res, a.ldr, y, a.ldy, a.n, a.k, a.act);
+    return launch_status();
+  }
+}
 template <typename YT>
 int launch_skinny(const FewRowsArgs& a, cudaStream_t st) {
   // 3 to 8 rows: columns per warp share what a row costs besides its products, but there have to be warps enough to have most of
   // the matrix requested at once (sixteen per SM at four columns, eight at two).  8 rows, one column per warp without prefetch and
   // now: 15.5 -> 8.8 us at 768 x 3072, 31.3 -> 17.3 at 1600 x 6400, 38.7 -> 33.3 at 32000 x 1024.
+  const bool four = a.n >= 4 * 16 * kNumSmsB200, two = a.n >= 2 * 8 * kNumSmsB200;
   // 1, 2 and 9 to 16 rows: prefetch while the columns do not fill the machine with warps by themselves (one row: 6.4 -> 5.3 us at
-  // 1024 x 4096, but 15.6 without against 25.9 us at 50304 x 768; 16 rows: 26.7 -> 13.7 us at 768 x 3072, but 12.5 against 18.3 at
-  // 4128 x 1024).
-  const bool four = a.n >= 4 * 16 * kNumSmsB200, two = a.n >= 2 * 8 * kNumSmsB200, many = a.n > (a.m > 8 ? 16 : 20) * kNumSmsB200;
-  // Of the wide form one row alone is a dependent launch (4128 x 1024: 3.9 -> 3.5 us): with more rows the blocks that wait take warps
-  // from the grid in front (4800 x 1600, dependent and plain: 8.0 and 7.1 us with 2 rows, 27.7 and 25.5 with 16).
-#define NX_WIDE(M_)                                                                                                                  \
-  if (many && a.m == M_) {                                                                                                          \
-    const dim3 grid(static_cast<unsigned>((a.n + 7) / 8));                                                                          \
-    if constexpr (M_ == 1) return launch_pdl(skinny_wide_kernel<M_, YT>, grid, dim3(256), 0, st, a);                                \
-    skinny_wide_kernel<M_, YT><<<grid, 256, 0, st>>>(a);                                                                            \
-    return launch_status();                                                                                                         \
-  }
+  // 1024 x 4096, but 15.6 without against 25.9 us at 50304 x 768; 12 rows: 19.2 -> 9.0 us at 768 x 3072, but 12.4 against 14.5 at
+  // 4800 x 1024).  With 13 and more rows two of its blocks fill an SM's registers, so that it ends where a second wave would begin
+  // (columns without and with prefetch, 13 rows: 7.1 and 5.5 us at 1184 x 1024, 7.6 and 9.9 at 1600 x 1024); 16 rows of a long K
+  // bear that a little longer (17.6 -> 14.6 us at 1600 x 1600).  11 rows take the instance of 12.
+  const int alone_above = kNumSmsB200 * (a.m == 1 || a.m == 2 ? 20 : (a.m == 11 ? 12 : (a.m < 13 ? 16 : 8)));
+  const bool many = a.n > alone_above && !(a.m == 16 && a.k >= 1600 && a.n <= 1600);
+#define NX_WIDE(M_) if (many && a.m == M_) return launch_wide<M_, YT>(a, st);
   NX_WIDE(1) NX_WIDE(2) NX_WIDE(9) NX_WIDE(10) NX_WIDE(11) NX_WIDE(12) NX_WIDE(13) NX_WIDE(14) NX_WIDE(15) NX_WIDE(16)
 #undef NX_WIDE
 #define NX_SK(M_)                                                  \

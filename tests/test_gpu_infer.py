@@ -332,6 +332,29 @@ def test_few_rows_at_the_edges_of_its_tiles(n, k, dtype):
         assert (buf[:, n:] == 9.0).all()
 
 
+@pytest.mark.parametrize("n,k,dtype", [(1184, 264, "bf16"), (1185, 264, "f32"), (1600, 1600, "bf16"), (1777, 72, "bf16"), (2376, 64, "f32"),
+                                       (4737, 40, "bf16"), (3600, 2056, "f32"), (6001, 1544, "bf16")])
+def test_nine_to_sixteen_rows_in_every_form(n, k, dtype):
+    """Both sides of the lines between the forms of 9 to 16 rows: prefetch, columns alone finished by a warp's lanes or by one of them.
+    A row has the same bits in all of them, in one batch of 16 and in each smaller one; bounds as above."""
+    K, I = _mods()
+    torch.manual_seed(3)
+    x, w = torch.randn(16, k, device="cuda").bfloat16(), (torch.randn(n, k, device="cuda") * k ** -0.5).bfloat16()
+    b, res = torch.randn(n, device="cuda").bfloat16(), torch.randn(16, n, device="cuda")
+    od = {"f32": torch.float32, "bf16": torch.bfloat16}[dtype]
+    tol = 1e-4 if dtype == "f32" else 2e-2
+    one = torch.cat([I.skinny_gemm(x[i: i + 1], w, out_dtype=od) for i in range(16)])
+    assert (one.double() - x.double() @ w.double().t()).abs().max() < tol
+    for m in range(9, 17):
+        assert torch.equal(I.skinny_gemm(x[:m], w, out_dtype=od), one[:m]), m
+        buf = torch.full((m, n + 3), 9.0, device="cuda", dtype=od)
+        y = buf[:, :n]
+        y.copy_(res[:m])
+        I.skinny_gemm(x[:m], w, b, act="relu", residual=y, out=y)
+        want = torch.relu(x[:m].double() @ w.double().t() + b.double()) + res[:m].to(od).double()
+        assert (y.double() - want).abs().max() < 2 * tol and (buf[:, n:] == 9.0).all()
+
+
 def test_few_rows_refuses_what_it_cannot_address():
     K, I = _mods()
     x, w = torch.zeros(65, 64, device="cuda").bfloat16(), torch.zeros(8, 64, device="cuda").bfloat16()
