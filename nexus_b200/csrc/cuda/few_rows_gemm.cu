@@ -434,9 +434,22 @@ int launch_few(const FewRowsArgs& a, int parts, cudaStream_t st) {
   return cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess ? 0 : ((void)cudaGetLastError(), -2);
 }
 
+// CTAs of a cluster along K: enough to have the weights of the whole matrix requested at once (two CTAs per SM), at least 64 elements
+// of K each, but no more than are resident at 64 rows (three per SM): a second wave cost 12.6 us against 7.9 at 64 rows of
+// 4128 x 1024, 15.6 against 13.9 at 8192 x 1024.
+int few_rows_parts(int n, int k) {
+  const int blocks = (n + kCols - 1) / kCols;
+  int parts = 1;
+  while (parts < 8 && blocks * parts < 2 * kNumSmsB200 && 2 * blocks * parts <= 3 * kNumSmsB200 && k >= 2 * parts * 64) parts *= 2;
+  return parts;
+}
+int few_rows_chain(int k, int parts) { return ((k + parts - 1) / parts + 31) / 32 * 32; }
+
 }  // namespace
 
 extern "C" int nx_skinny_max_rows(void) { return kFewRows; }
+
+extern "C" int nx_few_rows_chain(int n, int k) { return n > 0 && k > 0 ? few_rows_chain(k, few_rows_parts(n, k)) : -1; }
 
 extern "C" int nx_skinny_gemm(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* bias, const void* residual,
                               int64_t ldr, void* y, int64_t ldy, int out_dtype, int m, int n, int k, int act, int w_const,
@@ -457,14 +470,9 @@ extern "C" int nx_skinny_gemm(const void* x, int64_t ldx, const void* w, int64_t
   const uintptr_t align = out_dtype == NX_F32 ? 15 : 7;
   a.vec = !(reinterpret_cast<uintptr_t>(y) & align) && !(ldy & 3) &&
           (residual == nullptr || (!(reinterpret_cast<uintptr_t>(residual) & align) && !(ldr & 3)));
-  const int blocks = (n + kCols - 1) / kCols;
-  if (blocks > 65535) return -1;
-  // Enough CTAs to have the weights of the whole matrix requested at once (two per SM), at least 64 elements of K each, but no more
-  // than are resident at 64 rows (three per SM): a second wave cost 12.6 us against 7.9 at 64 rows of
-  // 4128 x 1024, 15.6 against 13.9 at 8192 x 1024.
-  int parts = 1;
-  while (parts < 8 && blocks * parts < 2 * kNumSmsB200 && 2 * blocks * parts <= 3 * kNumSmsB200 && k >= 2 * parts * 64) parts *= 2;
-  a.k_per = ((k + parts - 1) / parts + 31) / 32 * 32;
+  if ((n + kCols - 1) / kCols > 65535) return -1;
+  const int parts = few_rows_parts(n, k);
+  a.k_per = few_rows_chain(k, parts);
 #define NX_FEW(MT_) return out_dtype == NX_F32 ? launch_few<MT_, float>(a, parts, st) : launch_few<MT_, __nv_bfloat16>(a, parts, st)
   if (m <= 32) NX_FEW(4);
   NX_FEW(8);

@@ -42,6 +42,8 @@ int nx_paged_attention_decode(const NxPagedArgs* args, nx_stream_t stream);
 // The reduction order of a row is fixed, so a row's result does not depend on the batch it is in (one order for up to 16 rows,
 // another above).
 int nx_skinny_max_rows(void);
+// Elements of K that a CTA of the form for more than 16 rows walks through: the length of its chain (-1: no such sizes).
+int nx_few_rows_chain(int n, int k);
 // y and residual share out_dtype (BF16 or FP32); y may alias residual.  `w_const`: no kernel that may still be running on the
 // device writes w (weights of a loaded model): they are fetched while the kernel before this one finishes.
 int nx_skinny_gemm(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* bias, const void* residual,

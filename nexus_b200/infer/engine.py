@@ -549,11 +549,16 @@ class Engine:
 
     def _few_rows(self, rows: int, n: int, k: int) -> bool:
         """Whether a product reads its weights once, straight into registers: up to 16 rows always; up to 64 where the split tcgen05
-        product with its reduction pass is slower (64 rows: 7.2 against 12.4 us at 1600 x 1600, 12.8 against 16.7 at 6400 x 1600,
-        8.7 against 10.6 at 768 x 3072) and not where it is faster (20.1 against 15.9 at 1600 x 6400; vocabularies, whose tiles
-        fill the machine unsplit: 76 against 39 at 50304 x 1600).  Its time grows with n * k (12.8 us at 10 M, 52 at 33 M), that of
-        the other hardly (16.6 and 19.7): the line lies between."""
-        return rows <= self._skinny or (rows <= 64 and k <= 3072 and n < 16384 and n * k <= 12 << 20)
+        product with its reduction pass is slower.  That is so while no block's chain along K is longer than 512 (64 rows, split and few
+        rows, us: chain 400 of 6400 x 1600 17.0 and 12.8; 512 of 12288 x 1024 19.9 and 15.0, of 4096 x 2048 14.1 and 13.3; 640 of
+        4096 x 2560 14.7 and 16.2, of 8192 x 1280 15.9 and 16.9; 768 of 4096 x 3072 15.6 and 19.1; 800 of 7168 x 1600 17.2 and 20.7).
+        Vocabularies, whose tiles fill the machine unsplit, and larger matrices stay (76 against 39 us at 50304 x 1600)."""
+        if rows <= self._skinny:
+            return True
+        if rows > 64 or k > 3072 or n >= 16384 or n * k > 12 << 20:
+            return False
+        from ..ops import _infer as I
+        return I.few_rows_chain(n, k) <= 512
 
     def _norm(self, x, w, b):
         if not self.fast:

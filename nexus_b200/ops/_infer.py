@@ -33,6 +33,11 @@ def skinny_max_rows() -> int:
     return int(K.lib().nx_skinny_max_rows())
 
 
+def few_rows_chain(n: int, k: int) -> int:
+    """Elements of K that a block of `skinny_gemm` walks through with more than 16 rows of [n, k]."""
+    return int(K.lib().nx_few_rows_chain(C.c_int(n), C.c_int(k)))
+
+
 def kv_append(k, v, slots, k_cache, v_cache, *, k_scale=None, v_scale=None, kv_kind=KV_BF16) -> None:
     """k/v: [tokens, kv_heads, D] (row-strided views allowed); slots: int32 [tokens]."""
     tokens, hk, d = k.shape

@@ -355,6 +355,17 @@ def test_nine_to_sixteen_rows_in_every_form(n, k, dtype):
         assert (y.double() - want).abs().max() < 2 * tol and (buf[:, n:] == 9.0).all()
 
 
+@pytest.mark.parametrize("n,k,few", [(6400, 1600, True), (12288, 1024, True), (4096, 2048, True), (768, 3072, True), (4096, 2560, False),
+                                     (8192, 1280, False), (4096, 3072, False), (7168, 1600, False), (50304, 768, False), (1600, 6400, False)])
+def test_products_of_more_than_sixteen_rows_take_the_faster_kernel(n, k, few):
+    """Sizes whose two kernels were timed at 17, 32, 33 and 64 rows."""
+    K, I = _mods()
+    from nexus_b200.infer import Engine
+    eng = Engine.__new__(Engine)
+    eng._skinny = 16
+    assert [eng._few_rows(r, n, k) for r in (1, 16, 17, 33, 64, 65)] == [True, True, few, few, few, False]
+
+
 def test_few_rows_refuses_what_it_cannot_address():
     K, I = _mods()
     x, w = torch.zeros(65, 64, device="cuda").bfloat16(), torch.zeros(8, 64, device="cuda").bfloat16()
