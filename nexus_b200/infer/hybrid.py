@@ -259,7 +259,8 @@ class HybridEngine(Engine):
         self._stepped = M.Segments(table, 0, single.count + short.count, max(single.max_len, short.max_len),
                                    single.total + short.total)
         self._every = M.Segments(table, 0, first, max(g.max_len for g in groups), sum(g.total for g in groups))
-        self._packed: dict = {}        # blocks of the fresh prompts, per head size, window and cap
+        self._fresh = self._fresh_prompts()
+        self._packed: dict = {}        # their blocks, per head size, window and cap
         prompt.plan(self, self._prompt_windows, self._prompt_slices)
         return self._body(dv[0], dv[1], dv[2], dv[3], dv[4], dv[5][:logit_rows], runs, nl)
 
@@ -297,7 +298,7 @@ class HybridEngine(Engine):
         if not self._many.count:
             return
         # fresh prompts take the tcgen05 flash kernel where the head size allows it, all of a step in one launch
-        fresh = self._fresh_prompts() if a.dim == a.vdim and a.dim in (64, 128) and a.scale > 0 else None
+        fresh = self._fresh if a.dim == a.vdim and a.dim in (64, 128) and a.scale > 0 else None
         if not fresh:
             M.paged_window_attention(q, *paged, self._many, **kw)
             return
@@ -314,9 +315,11 @@ class HybridEngine(Engine):
     def _fresh_prompts(self):
         """(first row, rows) of the step's long segments if every one starts at position 0."""
         single, short, long_ = self._groups
-        host, first = self._host_rows[self.INDEX_ROWS:], single.count + short.count
-        segs = [[int(v) for v in host[:3, j]] for j in range(first, first + long_.count)]
-        return [(row0, n) for row0, n, pos in segs] if all(pos == 0 for _, _, pos in segs) else None
+        if not long_.count:
+            return None
+        first = single.count + short.count
+        segs = self._host_rows[self.INDEX_ROWS:][:3, first: first + long_.count].t().tolist()
+        return [(row0, n) for row0, n, _ in segs] if all(pos == 0 for _, _, pos in segs) else None
 
     def _conv(self, x, w, bias, tail) -> torch.Tensor:
         from ..ops import _mixers as M

@@ -118,6 +118,22 @@ def test_mixed_batches_with_pages_and_slots_used_again(name, precision):
     assert e.free_blocks() == e.total_blocks() and e.sched.live_sequences() == 0
 
 
+def test_fresh_prompts_of_a_step_are_listed_once(monkeypatch):
+    """Two layers whose prompts take the packed kernel share one list, and one table of blocks."""
+    from nexus_b200.infer.hybrid import HybridEngine
+    from nexus_b200.ops import _cuda as K
+    left = {"heads": 2, "kv_heads": 1, "dim": 64, "vdim": 64, "mask": {"size": 150}, "rot": {"base": 90000.0, "dims": 64}, "scale": 0.125}
+    monkeypatch.setitem(CONFIGS, "twice", O.random_config(("parallel", "parallel"), left=left))
+    lists, tables = [], []
+    list_prompts, blocks = HybridEngine._fresh_prompts, K.PackedBlocks
+    monkeypatch.setattr(HybridEngine, "_fresh_prompts", lambda e: lists.append(list_prompts(e)) or lists[-1])
+    monkeypatch.setattr(K, "PackedBlocks", lambda *a, **k: tables.append(a[0]) or blocks(*a, **k))
+    e = _engine("twice", "bf16")
+    _feed(e, "twice", [[(0, 170), (1, 61), (2, 23)]], "bf16")
+    assert lists == tables == [[(0, 170), (170, 61), (231, 23)]]
+    del _cache["twice"]
+
+
 def test_layers_of_the_residual_stream():
     cfg, w, seqs, _ = _model("base")
     want, got = [], []
