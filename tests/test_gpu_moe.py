@@ -138,3 +138,21 @@ def test_router_logits_are_fp32_sums(N, d, E):
     x, r = torch.randn(N, d, device="cuda").bfloat16(), (torch.randn(E, d, device="cuda") * d ** -0.5).bfloat16()
     want = x.double() @ r.double().t()
     assert (G.router_logits(x, r).double() - want).norm() <= 2.4e-8 * (d / 2) ** 0.5 * want.norm()
+
+
+def test_router_delta_pieces_sum_to_the_value():
+    """Three BF16 pieces hold an FP32 gradient whole, up to the largest and down to small ones."""
+    import ctypes as C
+    from nexus_b200.ops import _cuda as K
+    big = torch.finfo(torch.float32).max
+    torch.manual_seed(14)
+    delta = torch.cat([torch.tensor([big, -big, 3.39e38, 1.0, -1.0 / 3.0, 1e-30, 0.0]), torch.randn(249) * 10.0 ** torch.randint(-20, 20, (249,))]).cuda()
+    N, E, pitch = delta.numel(), 5, 8
+    gate, dgate = torch.ones(N, 2, device="cuda"), torch.stack([delta, -delta], 1).contiguous()      # their inner sum is 0
+    expert = torch.tensor([[1, 3]], dtype=torch.int32, device="cuda").repeat(N, 1).contiguous()
+    dsel, pieces = torch.empty(N, 2, device="cuda"), torch.empty(N, 3, pitch, device="cuda", dtype=torch.bfloat16)
+    K._check(K.lib().nx_moe_router_delta(K._p(gate), K._p(dgate), K._p(expert), K._p(dsel), K._p(pieces), C.c_int(N), C.c_int(2), C.c_int(E),
+                                         C.c_int(pitch), K._stream()), "nx_moe_router_delta")
+    got = pieces.double().sum(1)
+    assert torch.equal(dsel[:, 0], delta) and torch.equal(dsel[:, 1], -delta)
+    assert torch.equal(got[:, 1], delta.double()) and torch.equal(got[:, 3], -delta.double()) and (got[:, [0, 2, 4, 5, 6, 7]] == 0).all()
