@@ -33,6 +33,15 @@ def _use_kernels(*ts: torch.Tensor) -> bool:
     return True
 
 
+def _has_storage(t: torch.Tensor) -> bool:
+    """False for the tensors of a vmap, which stand for several."""
+    try:
+        t.data_ptr()
+    except RuntimeError:
+        return False
+    return True
+
+
 def gelu_tanh(x: torch.Tensor) -> torch.Tensor:
     return F.gelu(x, approximate="tanh")
 
@@ -440,7 +449,8 @@ class _FusedCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         (g,) = ctx.saved_tensors
-        if g.is_cuda:
+        # one plain gradient: not one of a batch, none that is differentiated itself (with respect to `dloss`)
+        if g.is_cuda and not torch.is_grad_enabled() and _has_storage(dloss):
             from ..ops import _cuda as K
             return K.scale(g, dloss.float()).to(ctx.dtype).view(ctx.shape), None, None, None, None, None, None
         return (g * dloss.to(g.dtype)).to(ctx.dtype).view(ctx.shape), None, None, None, None, None, None

@@ -329,6 +329,22 @@ def test_cross_entropy_of_masked_vectors(dt, V, mask):
             assert (grad[:, :V][logits[:, :V] == mask] == 0).all()
 
 
+def test_loss_gradient_in_batches_and_differentiated():
+    """Several gradients of the loss at once, and the derivative of its gradient with respect to the factor in front of it."""
+    from nexus_b200.fused import ops
+    torch.manual_seed(15)
+    logits = torch.randn(6, 40, device="cuda", requires_grad=True)
+    targets = torch.arange(6, device="cuda")
+    loss = ops.cross_entropy(logits, targets)
+    (g,) = torch.autograd.grad(loss, logits, retain_graph=True)
+    (many,) = torch.autograd.grad(loss, logits, torch.tensor([1.0, -2.0], device="cuda"), is_grads_batched=True, retain_graph=True)
+    assert torch.allclose(many, torch.stack([g, -2 * g]))
+    factor = torch.tensor(3.0, device="cuda", requires_grad=True)
+    (scaled,) = torch.autograd.grad(loss * factor, logits, create_graph=True)
+    (back,) = torch.autograd.grad((scaled * g).sum(), factor)
+    assert torch.allclose(scaled, 3 * g) and torch.allclose(back, (g * g).sum())
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 516), (64, 1600), (3, 1028), (1300, 2048), (5, 4100), (7, 8192), (2, 8196)])
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("xdt", [torch.float32, torch.bfloat16])
