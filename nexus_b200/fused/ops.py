@@ -86,8 +86,8 @@ class _FusedLinear(torch.autograd.Function):
         from ..ops import _cuda as K
         x2, w, aux = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
+        if not dy2.is_contiguous() or dy2.data_ptr() % 16:
+            dy2 = dy2.clone(memory_format=torch.contiguous_format)
         dpre = dy2 if ctx.act == "identity" else K.act_bwd(aux, dy2.to(aux.dtype), ctx.act)
         dx = K.gemm(dpre, w, b_mn=True).view(ctx.x_shape) if ctx.needs_input_grad[0] else None
         dw = K.weight_grad(dpre, x2, w.dtype) if ctx.needs_input_grad[1] else None

@@ -345,6 +345,18 @@ def test_loss_gradient_in_batches_and_differentiated():
     assert torch.allclose(scaled, 3 * g) and torch.allclose(back, (g * g).sum())
 
 
+@pytest.mark.parametrize("rows,pitch,at", [(5, 16, 1), (1, 21, 1), (8, 16, 3)])
+def test_linear_weight_gradient_from_any_output_gradient(rows, pitch, at):
+    """Gradients that lie beside 16 bytes.  BF16 result of exact products: 2^-8."""
+    from nexus_b200.fused import ops
+    torch.manual_seed(17)
+    x, w = torch.randn(rows, 24, device="cuda").bfloat16(), torch.randn(16, 24, device="cuda").bfloat16().requires_grad_(True)
+    dy = torch.randn(rows * pitch + 8, device="cuda").bfloat16()[at:].as_strided((rows, 16), (pitch, 1))
+    (dw,) = torch.autograd.grad(ops.fused_linear(x, w), w, dy)
+    want = dy.double().t() @ x.double()
+    assert ((dw.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 516), (64, 1600), (3, 1028), (1300, 2048), (5, 4100), (7, 8192), (2, 8196)])
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("xdt", [torch.float32, torch.bfloat16])
