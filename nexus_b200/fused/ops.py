@@ -355,14 +355,14 @@ class _QkvAttention(torch.autograd.Function):
 def qkv_attention_ok(qkv, dim: int, rope=None) -> bool:
     """Whether `qkv_attention` takes these rows (and these tables [positions, half], FP32): CUDA BF16, head size 64 or 128."""
     if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 3 and qkv.is_contiguous() and dim in (64, 128)
-            and qkv.numel() > 0 and qkv.data_ptr() % 16 == 0):
+            and 0 < qkv.numel() < 1 << 34 and qkv.data_ptr() % 16 == 0):
         return False
     if rope is None:
         return _use_kernels(qkv)
     cos, sin = rope
     return (_use_kernels(qkv) and all(t.device == qkv.device and t.dtype == torch.float32 and t.is_contiguous() for t in (cos, sin))
             and cos.shape == sin.shape and cos.shape[1] % 8 == 0 and 0 < 2 * cos.shape[1] <= dim and cos.shape[0] >= qkv.shape[1]
-            and not (cos.requires_grad or sin.requires_grad))
+            and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0 and not (cos.requires_grad or sin.requires_grad))
 
 
 def qkv_attention(qkv, heads: int, kv_heads: int, dim: int, rope=None, window=0, softcap=0.0, alibi_slopes=None, dropout_p=0.0,

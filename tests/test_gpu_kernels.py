@@ -357,6 +357,14 @@ def test_linear_weight_gradient_from_any_output_gradient(rows, pitch, at):
     assert ((dw.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
 
 
+def test_packed_attention_leaves_tables_beside_16_bytes_to_the_general_form():
+    from nexus_b200.fused import ops
+    qkv = torch.randn(1, 4, 3 * 64, device="cuda").bfloat16()
+    flat = torch.randn(4 * 32 + 1, device="cuda")
+    on, off = flat[:128].view(4, 32), flat[1:].view(4, 32)
+    assert ops.qkv_attention_ok(qkv, 64, (on, on)) and not ops.qkv_attention_ok(qkv, 64, (off, on)) and not ops.qkv_attention_ok(qkv, 64, (on, off))
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 516), (64, 1600), (3, 1028), (1300, 2048), (5, 4100), (7, 8192), (2, 8196)])
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("xdt", [torch.float32, torch.bfloat16])
