@@ -1139,7 +1139,7 @@ __device__ __forceinline__ void store_row32_scaled(__nv_bfloat16* dst, const uin
 // ================================================================================================
 // backward, part 1: dK / dV.  One CTA per (kv block of 128, kv head, batch); loops over the q heads
 // of the group and over q chunks of 64 rows.  TMEM: S^T [128 kv][64 q], dP^T [128][64], dV [128][HD],
-// dK [128][HD].  The two threads of row r own kv row r.
+// dK [128][HD].  The thread (at head size 128 the two threads) of row r owns kv row r.
 // ================================================================================================
 template <int HD>
 struct DkvCfg {
@@ -1455,7 +1455,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
 // ================================================================================================
 // backward, part 2: dQ.  One CTA per (q block of 128, head, batch); loops over kv chunks of 64.
-// TMEM: S [128 q][64 kv], dP [128][64], dQ [128][HD].  The two threads of row r own q row r.
+// TMEM: S [128 q][64 kv], dP [128][64], dQ [128][HD].  The thread (at head size 128 the two threads) of row r owns q row r.
 // ================================================================================================
 template <int HD>
 struct DqCfg {
@@ -1757,11 +1757,6 @@ int make_map(CUtensorMap* m, const NxAttnView& v, int T, int H, int B, int HD, i
                                 v.head_stride, v.batch_stride, 64, box_rows, 1);
 }
 
-template <typename K>
-int set_smem(K kern, int bytes) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess ? 0 : -2;
-}
-
 AttnDev base_params(const NxAttnArgs* a) {
   AttnDev p{};
   p.lse = a->lse;
@@ -1837,11 +1832,7 @@ extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
     const int grid2 = std::min(p.items, sms);
 #define NX_FWD2(HD_)                                                                                \
   do {                                                                                              \
-    static bool once = false;                                                                       \
-    if (!once) {                                                                                    \
-      if (set_smem(attn_fwd2_kernel<HD_, false>, Fwd2Cfg<HD_>::kSmem)) return -2;                          \
-      once = true;                                                                                  \
-    }                                                                                               \
+    NX_ALLOW_SMEM((attn_fwd2_kernel<HD_, false>), Fwd2Cfg<HD_>::kSmem);                             \
     NX_PDL((attn_fwd2_kernel<HD_, false>), grid2, kFwd2Threads, Fwd2Cfg<HD_>::kSmem, st, tq, tk, tv, p);    \
   } while (0)
     if (HD == 64) NX_FWD2(64);
@@ -1851,11 +1842,7 @@ extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
   }
 #define NX_FWD(HD_, EXT_)                                                                           \
   do {                                                                                              \
-    static bool once = false;                                                                       \
-    if (!once) {                                                                                    \
-      if (set_smem(attn_fwd_kernel<HD_, EXT_, false>, FwdCfg<HD_>::kSmem)) return -2;                      \
-      once = true;                                                                                  \
-    }                                                                                               \
+    NX_ALLOW_SMEM((attn_fwd_kernel<HD_, EXT_, false>), FwdCfg<HD_>::kSmem);                         \
     NX_PDL((attn_fwd_kernel<HD_, EXT_, false>), grid, kFwdThreads, FwdCfg<HD_>::kSmem, st, tq, tk, tv, p);  \
   } while (0)
   const int mode = !ext ? 0 : (p.alibi == nullptr && p.dropout_p <= 0.0f && p.scale > 0.0f ? 2 : 1);
@@ -1897,11 +1884,7 @@ extern "C" int nx_attention_fwd_packed(const NxAttnArgs* a, const int32_t* block
     return -2;
 #define NX_PACKED(KERN_, CFG_, PER_SM_)                                                             \
   do {                                                                                              \
-    static bool once = false;                                                                       \
-    if (!once) {                                                                                    \
-      if (set_smem(KERN_, CFG_::kSmem)) return -2;                                                  \
-      once = true;                                                                                  \
-    }                                                                                               \
+    NX_ALLOW_SMEM(KERN_, CFG_::kSmem);                                                              \
     NX_PDL(KERN_, std::min(p.items, sms * PER_SM_), kFwdThreads, CFG_::kSmem, st, tq, tk, tv, p);   \
   } while (0)
   // the blocks are of nx_attention_packed_rows() query rows: two tiles where nx_attention_fwd takes the two-tile form too
@@ -1930,11 +1913,7 @@ extern "C" int nx_attention_bwd(const NxAttnArgs* a, nx_stream_t stream_) {
   int rc;
 #define NX_BWD(KERN_, CFG_, HD_, EXT_)                                                              \
   do {                                                                                              \
-    static bool once = false;                                                                       \
-    if (!once) {                                                                                    \
-      if (set_smem(KERN_<HD_, EXT_>, CFG_<HD_>::kSmem)) return -2;                                  \
-      once = true;                                                                                  \
-    }                                                                                               \
+    NX_ALLOW_SMEM((KERN_<HD_, EXT_>), CFG_<HD_>::kSmem);                                            \
     NX_PDL((KERN_<HD_, EXT_>), grid, bwd_threads(HD_), CFG_<HD_>::kSmem, st, tq, tk, tv, tdo, p);           \
   } while (0)
   // part 1: dQ (also forms dsum = rowsum(dO * O) and leaves it for part 2)

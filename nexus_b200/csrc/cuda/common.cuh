@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "once_per_device.h"
+
 namespace nx {
 
 constexpr int kNumSmsB200 = 148;
@@ -38,6 +40,19 @@ inline int launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem
   (void)cudaGetLastError();
   return -2;
 }
+// Allows a kernel `bytes` of dynamic shared memory on the current device, once; in a function that returns 0 or an error:
+// NX_ALLOW_SMEM((kernel), bytes)
+template <typename... KArgs>
+inline int allow_smem(OncePerDevice& once, void (*kern)(KArgs...), int bytes) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return -2;
+  return once(dev, [&](int) { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess ? 0 : -2; });
+}
+#define NX_ALLOW_SMEM(KERN_, BYTES_)                               \
+  do {                                                             \
+    static ::nx::OncePerDevice nx_once;                            \
+    if (::nx::allow_smem(nx_once, KERN_, BYTES_) != 0) return -2;  \
+  } while (0)
 // The launch in a function that returns 0 or an error: NX_PDL((kernel), grid, threads, shared memory, stream, arguments ...)
 #define NX_PDL(KERN_, GRID_, BLOCK_, SMEM_, ST_, ...)                                                  \
   do {                                                                                                 \

@@ -413,11 +413,7 @@ template <int MT, typename YT>
 int launch_few(const FewRowsArgs& a, int parts, cudaStream_t st) {
   constexpr int smem = std::max(kStages * MT * 8 * kPitch, MT * 8 * kRedPitch * 4);
   auto kern = few_rows_kernel<MT, YT>;
-  static bool once = false;
-  if (!once) {
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM(kern, smem);
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

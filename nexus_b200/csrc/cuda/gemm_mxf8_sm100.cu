@@ -835,10 +835,8 @@ int launch_mx_pair(const NxMxGemmArgs* a, MxParams p, const CUtensorMap& ta, cud
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  NX_ALLOW_SMEM(gemm_mxf8_pair_kernel, kPairSmemBytes);
   if (max_clusters == 0) {
-    if (cudaFuncSetAttribute(gemm_mxf8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes) !=
-        cudaSuccess)
-      return -2;
     cfg.gridDim = dim3(2 * 74);
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, gemm_mxf8_pair_kernel, &cfg) != cudaSuccess || n < 1) {
@@ -932,12 +930,7 @@ extern "C" int nx_gemm_mxf8(const NxMxGemmArgs* a, nx_stream_t stream_) {
     if (rc_pair != -3) return rc_pair;
   }
 
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_mxf8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
-      return -2;
-    attr_set = true;
-  }
+  NX_ALLOW_SMEM(gemm_mxf8_kernel, kSmemBytes);
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)

@@ -15,6 +15,7 @@
 //
 // Replaces the reference's cuBLASLt layer and its epilogues Bias / BiasGelu(+aux) / DGelu /
 // beta=1 accumulate (include/nexus/cuda/gemm.hpp:38-121, src/cuda/gemm_lt.cpp:260-360).
+#include "common.cuh"
 #include "glu.cuh"
 #include "nx_api_comm.h"
 #include "sm100_ptx.cuh"
@@ -1199,8 +1200,8 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const DevParams& p
   cfg.attrs = attr;
   static const bool no_pdl = std::getenv("NX_NO_PDL") != nullptr;  // measurement switch
   cfg.numAttrs = no_pdl ? 1 : 2;
+  NX_ALLOW_SMEM(kern, C::kSmemBytes);
   if (max_clusters == 0) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) return -2;
     cfg.gridDim = dim3(2 * 74);
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
@@ -1234,13 +1235,8 @@ int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const DevParams
                    cudaStream_t stream, const DistParam<DIST>& dist = DistParam<DIST>{}, int fmt_b = -1,
                    const CUtensorMap* t_out = nullptr, const CUtensorMap* t_aux = nullptr) {
   using C = Cfg<BN>;
-  static bool attr_set = false;
   auto kern = gemm_kernel<BN, A_MN, B_MN, DIST>;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess)
-      return -2;
-    attr_set = true;
-  }
+  NX_ALLOW_SMEM(kern, C::kSmemBytes);
   const uint32_t idesc = make_idesc(in_fmt, fmt_b < 0 ? in_fmt : static_cast<uint32_t>(fmt_b), A_MN, B_MN, kBM, BN);
   // unused store maps are passed as copies of an operand map: never dereferenced unless p.tma_store is set
   kern<<<grid, kThreads, C::kSmemBytes, stream>>>(ta, tb, p, idesc, dist, t_out ? *t_out : ta, t_aux ? *t_aux : ta);

@@ -799,12 +799,7 @@ extern "C" int nx_paged_attention_decode(const NxPagedArgs* a, nx_stream_t strea
           a->max_blocks, a->row_seq, a->ctx_len, a->heads, a->kv_heads, a->scale, splits, (__nv_bfloat16*)a->out,
           a->o_row_stride, a->part_o, a->part_ml, a->status);
     else {
-      static bool once = false;
-      if (!once) {
-        if (cudaFuncSetAttribute(paged_decode_tma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-          return -2;
-        once = true;
-      }
+      NX_ALLOW_SMEM((paged_decode_tma_kernel<128>), smem);
       NX_PDL((paged_decode_tma_kernel<128>), grid, 128, smem, st, tk, tv, (const __nv_bfloat16*)a->q, a->q_row_stride, a->block_table,
           a->max_blocks, a->row_seq, a->ctx_len, a->heads, a->kv_heads, a->scale, splits, (__nv_bfloat16*)a->out,
           a->o_row_stride, a->part_o, a->part_ml, a->status);
@@ -870,12 +865,7 @@ extern "C" int nx_sample(const float* logits, int64_t ld, int vocab, const NxSam
   // rows of up to ~55 k entries live in shared memory for the threshold searches
   const size_t row_bytes = static_cast<size_t>(vocab) * sizeof(float);
   const bool in_smem = row_bytes <= 220 * 1024;
-  static bool attr_set = false;
-  if (in_smem && !attr_set) {
-    if (cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
-      return -2;
-    attr_set = true;
-  }
+  if (in_smem) NX_ALLOW_SMEM(sample_kernel, 220 * 1024);
   sample_kernel<<<rows, 1024, in_smem ? row_bytes : 0, static_cast<cudaStream_t>(stream)>>>(
       logits, ld, vocab, params, counts_all, counts_out, count_row, offsets, work, out, in_smem ? 1 : 0);
   return launch_status();

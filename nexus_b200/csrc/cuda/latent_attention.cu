@@ -415,12 +415,7 @@ int launch(const CUtensorMap& tm, const NxLatentAttnArgs* a, cudaStream_t st) {
   const int half = (kSmemMax / 2 - 1024 - fixed) / stage;
   const int stages = std::min(4, half >= 2 ? half : (kSmemMax - 1024 - fixed) / stage);
   if (stages < 2) return -1;
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(latent_attn_kernel<MT, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax - 1024) != cudaSuccess)
-      return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((latent_attn_kernel<MT, CT>), kSmemMax - 1024);
   const int rt = std::min(a->heads, S::kRows), tq = std::max(1, S::kRows / rt);
   const dim3 grid(a->seg.total_len / tq + a->seg.count, (a->heads + rt - 1) / rt, a->splits);
   latent_attn_kernel<MT, CT><<<grid, S::kWarps * 32, fixed + stages * stage, st>>>(tm, *a, rt, tq, stages);

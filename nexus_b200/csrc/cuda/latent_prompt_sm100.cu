@@ -12,6 +12,7 @@
 // Key tiles start at the first key the block can see: with a window no tile is wasted on keys before it.  Kept first keys that
 // lie before the window come first, in tiles of their own.  Keys and values have rings of their own, since a key part of 192
 // columns leaves room for one stage of values.
+#include "common.cuh"
 #include "flash_common.cuh"
 #include "nx_api_mixers.h"
 #include "sm100_ptx.cuh"
@@ -465,11 +466,7 @@ struct Maps {
 template <int ND, int NR, int NV, bool kBias>
 int launch(const Maps& t, const Dev& p, cudaStream_t st) {
   constexpr int kSmem = Cfg<ND, NR, NV, kBias>::kSmem;
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(prompt_kernel<ND, NR, NV, kBias>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((prompt_kernel<ND, NR, NV, kBias>), kSmem);
   int sms = 0, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
   prompt_kernel<ND, NR, NV, kBias><<<std::min(p.items, sms), kThreads, kSmem, st>>>(t.q, t.qr, t.k, t.kr, t.v, p);

@@ -485,11 +485,7 @@ int padded_dim(const NxPagedWindowArgs* a) {
 template <int DP, bool kBias>
 int launch_prefill_as(const NxPagedWindowArgs* a, dim3 grid, int rt, int tq, int head_tiles, cudaStream_t st) {
   constexpr int kSmem = (kRows + 4 * kKeys) * (DP + 8) * 2;
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(paged_prefill_kernel<DP, kBias>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((paged_prefill_kernel<DP, kBias>), kSmem);
   paged_prefill_kernel<DP, kBias><<<grid, kRows * 2, kSmem, st>>>(*a, rt, tq, head_tiles);
   return launch_status();
 }
@@ -503,11 +499,7 @@ template <int DP, bool kBias>
 int launch_decode_as(const NxPagedWindowArgs* a, dim3 grid, int head_tiles, cudaStream_t st) {
   constexpr int kSmem = (16 + 4 * kKeys) * (DP + 8) * 2;
   static_assert(4 * kKeys * (DP + 8) * 2 >= 4 * 16 * DP * 4, "partial outputs reuse the stages");
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(paged_decode_mma_kernel<DP, kBias>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((paged_decode_mma_kernel<DP, kBias>), kSmem);
   NX_PDL((paged_decode_mma_kernel<DP, kBias>), grid, 128, kSmem, st, *a, head_tiles);
   return launch_status();
 }

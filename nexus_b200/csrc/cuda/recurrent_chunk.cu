@@ -307,13 +307,8 @@ __global__ void ssd_span_scan_kernel(const NxSsdArgs a) {
 template <int NP>
 int launch_ssd(const NxSsdArgs* a, cudaStream_t st) {
   constexpr int kBytes = SsdSmem<NP>::kBytes;
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(ssd_chunk_kernel<NP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(ssd_chunk_kernel<NP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess)
-      return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((ssd_chunk_kernel<NP, false>), kBytes);
+  NX_ALLOW_SMEM((ssd_chunk_kernel<NP, true>), kBytes);
   const int col_tiles = (a->vdim + kCols - 1) / kCols;
   dim3 grid(a->heads * col_tiles, a->parts, a->seg.count);
   if (a->parts > 1) {
@@ -726,11 +721,7 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 2 : 1) delta_chunk_kernel(con
 template <int DP, int COLS>
 int launch_delta_chunks(const NxDeltaArgs* a, int chunks, cudaStream_t st) {
   constexpr int kBytes = DeltaSmem<DP, COLS>::kBytes;
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(delta_chunk_kernel<DP, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess) return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((delta_chunk_kernel<DP, COLS>), kBytes);
   const int col_tiles = (a->vdim + COLS - 1) / COLS;
   delta_chunk_kernel<DP, COLS><<<dim3(a->heads * col_tiles, a->seg.count), 256, kBytes, st>>>(*a, chunks, col_tiles);
   return launch_status();
@@ -739,11 +730,7 @@ int launch_delta_chunks(const NxDeltaArgs* a, int chunks, cudaStream_t st) {
 template <int DP>
 int launch_delta(const NxDeltaArgs* a, cudaStream_t st) {
   constexpr int kPrep = prep_front<DP>() + kQ * (kQ + 4) * 4;
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(delta_prep_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrep) != cudaSuccess) return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((delta_prep_kernel<DP>), kPrep);
   const int chunks = (a->seg.max_len + kQ - 1) / kQ;
   delta_prep_kernel<DP><<<dim3(chunks, a->heads, a->seg.count), 128, kPrep, st>>>(*a, chunks);
   // the chunks of a segment are a chain: while the blocks do not fill the GPU, narrower column tiles shorten every link

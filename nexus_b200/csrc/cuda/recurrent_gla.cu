@@ -421,13 +421,8 @@ template <int NP>
 int launch(const NxGlaArgs* a, cudaStream_t st) {
   constexpr int kBytes = Smem<NP>::kBytes;
   static_assert(kBytes <= 227 * 1024 - 64, "shared memory");
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(gla_chunk_kernel<NP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(gla_chunk_kernel<NP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess)
-      return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((gla_chunk_kernel<NP, false>), kBytes);
+  NX_ALLOW_SMEM((gla_chunk_kernel<NP, true>), kBytes);
   const int col_tiles = (a->vdim + kCols - 1) / kCols;
   dim3 grid(a->heads * col_tiles, a->parts, a->seg.count);
   if (a->parts > 1) {

@@ -8,6 +8,7 @@
 // issues the products Q K^T up to four tiles ahead, another P V.  Both groups add to one O, so they share the row maxima that O is scaled
 // by: tile j passes them on to tile j + 1, between the two warps that own the same 32 rows.  O is rescaled only when a row's maximum has
 // grown by 2^8.  A head's table of biases (in units of log2, extended to both sides) arrives by bulk copy beside its queries.
+#include "common.cuh"
 #include "flash_common.cuh"
 #include "nx_api_mixers.h"
 #include "sm100_ptx.cuh"
@@ -480,11 +481,7 @@ int head_map(CUtensorMap* m, const void* base, int cols, int heads, int rows, in
 
 template <int ND>
 int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const Dev& p, cudaStream_t st) {
-  static bool once = false;
-  if (!once) {
-    if (cudaFuncSetAttribute(talk_prompt_kernel<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<ND>::kSmem) != cudaSuccess) return -2;
-    once = true;
-  }
+  NX_ALLOW_SMEM((talk_prompt_kernel<ND>), Cfg<ND>::kSmem);
   int sms = 0, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
   talk_prompt_kernel<ND><<<std::min(p.items, sms), kThreads, Cfg<ND>::kSmem, st>>>(q, k, v, p);
