@@ -94,16 +94,12 @@ __global__ void __launch_bounds__(128, M > 8 ? 2 : (M > 2 ? 3 : 5)) skinny_kerne
   for (int s = 0; s < kX; ++s)
 #pragma unroll
     for (int i = 0; i < M; ++i) xr[s][i] = load_x(i, s * 256);
-  // lane i * C + c finishes row i of column c (and row i + 32 / C): its residual is on the way while the products run
-  constexpr int kRes = M * C > 32 ? 2 : 1;
+  // lane i * C + c finishes row i of column c: its residual is on the way while the products run
+  static_assert(M * C <= 32, "a lane per result");
   const int my_row = lane / C, my_col = col0 + lane % C;
+  const bool mine = my_row < a.m && my_col < a.n;
   const float bias = a.bias != nullptr && my_col < a.n ? __bfloat162float(a.bias[my_col]) : 0.0f;
-  float res[kRes];
-#pragma unroll
-  for (int h = 0; h < kRes; ++h) {
-    const int row = my_row + h * (32 / C);
-    res[h] = a.residual != nullptr && row < a.m && my_col < a.n ? Num<YT>::load(static_cast<const YT*>(a.residual) + row * a.ldr + my_col) : 0.0f;
-  }
+  const float res = a.residual != nullptr && mine ? Num<YT>::load(static_cast<const YT*>(a.residual) + my_row * a.ldr + my_col) : 0.0f;
   float acc[M][C];
 #pragma unroll
   for (int i = 0; i < M; ++i)
@@ -134,7 +130,7 @@ __global__ void __launch_bounds__(128, M > 8 ? 2 : (M > 2 ? 3 : 5)) skinny_kerne
       }
     }
   }
-  float sum[kRes];
+  float sum = 0.0f;
 #pragma unroll
   for (int i = 0; i < M; ++i)
 #pragma unroll
@@ -142,16 +138,12 @@ __global__ void __launch_bounds__(128, M > 8 ? 2 : (M > 2 ? 3 : 5)) skinny_kerne
       float t = acc[i][c];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == (i * C + c) % 32) sum[(i * C + c) / 32] = t;
+      if (lane == i * C + c) sum = t;
     }
-#pragma unroll
-  for (int h = 0; h < kRes; ++h) {
-    const int row = my_row + h * (32 / C);
-    if (row >= a.m || my_col >= a.n) continue;
-    float v = apply_act(sum[h] + bias, a.act);
-    if (a.residual != nullptr) v += res[h];
-    Num<YT>::store(static_cast<YT*>(a.y) + row * a.ldy + my_col, v);
-  }
+  if (!mine) return;
+  float v = apply_act(sum + bias, a.act);
+  if (a.residual != nullptr) v += res;
+  Num<YT>::store(static_cast<YT*>(a.y) + my_row * a.ldy + my_col, v);
 }
 
 // The same sums of exactly M rows with a column per warp and no prefetch of its own: many small warps per SM instead.  kSpread: lane i
