@@ -1091,18 +1091,622 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 }
 
 // ================================================================================================
-// backward.  Both kernels are bound by the row math (conversions, exponentials, stores of P and dS) and by the hand-overs between
-// it and the tensor core, so the score products of chunk i + 1 are issued ahead of the gradient products of chunk i:
-//   head_dim 128, one CTA per SM: into a second pair of score tiles, while the math of chunk i runs;
-//   head_dim 64, two CTAs per SM with 256 TMEM columns each: into the same tiles, as soon as the math of chunk i has read them.
-// At head_dim 128 two threads (warps w and w + 4) share a row, 32 of a chunk's 64 columns each; at 64, where the other CTA's warps
-// fill the gaps, one thread has it (two per row took 112 us for dQ on 16 x 12 x 1024 x 64, against 103 before this scheme).  The
-// factor `scale` of dS goes to the results.
-// On 2 x 32 (8) x 4096 x 128, causal, dK / dV takes 542 us and dQ 510; with four math warps and the four steps in turn it was 797
-// and 759, the tensor cores busy for a quarter of that.  At head_dim 64 two CTAs per SM had hidden most of it already.
+// backward.  Bound by the row math (conversions, exponentials, stores of P and dS) and by the hand-overs between it and the tensor
+// core.
+//
+// Head size 64: two CTAs per SM with 256 TMEM columns each cover each other's waits, one thread has a row, a chunk's steps follow one
+// another.  Score products a chunk ahead, as below, cost more there than they hid (dQ, dK and dV, us, in turn and ahead: 16 x 12 x
+// 1024 229 and 247, with soft-capping 403 and 457; 1 x 16 (4) x 4096 456 and 505 to 570; 4 x 32 (4) x 1024 252 and 279).
 // ================================================================================================
-constexpr int bwd_math_warps(int hd) { return hd == 64 ? 4 : 8; }  // row quarter = warp & 3, column half = warp >> 2
-constexpr int bwd_threads(int hd) { return (bwd_math_warps(hd) + 2) * 32; }  // then one warp for TMA, one for MMA + TMEM
+constexpr int kBwd64Threads = 192;  // warps 0-3: row math, warp 4: TMA, warp 5: MMA + TMEM
+
+// ================================================================================================
+// backward at head size 64, part 1: dK / dV.  One CTA per (kv block of 128, kv head, batch); loops over the q heads
+// of the group and over q chunks of 64 rows.  TMEM: S^T [128 kv][64 q], dP^T [128][64], dV [128][HD],
+// dK [128][HD].  Thread r owns kv row r.
+// ================================================================================================
+struct Dkv64Cfg {
+  static constexpr int HD = 64;
+  static constexpr int kKVBytes = 128 * HD * 2;   // K and V tiles (resident)
+  static constexpr int kQBytes = 64 * HD * 2;     // Q / dO chunk
+  static constexpr int kPBytes = 128 * 64 * 2;    // P^T and dS^T
+  static constexpr int kSmem = 2 * kKVBytes + 4 * kQBytes + 2 * kPBytes + 2 * 2 * 64 * 4 + 128;
+  static constexpr int kTmemCols = 256;  // 64 + 64 + 2 * HD
+};
+
+template <bool EXT>  // EXT: soft-capping / ALiBi / dropout row math (a build of its own)
+__global__ void __launch_bounds__(kBwd64Threads, 2)
+attn_bwd64_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                     const AttnDev p) {
+  using C = Dkv64Cfg;
+  constexpr int HD = C::HD;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1 KiB aligned base; uniform early exit
+    if (threadIdx.x == 0) atomicCAS(p.status, 0, kStatusBadArgument);
+    return;
+  }
+  uint8_t* sK = smem;
+  uint8_t* sV = sK + C::kKVBytes;
+  uint8_t* sQ = sV + C::kKVBytes;        // 2 stages
+  uint8_t* sDO = sQ + 2 * C::kQBytes;    // 2 stages
+  uint8_t* sPT = sDO + 2 * C::kQBytes;   // [128 kv][64 q] bf16
+  uint8_t* sDST = sPT + C::kPBytes;      // [128 kv][64 q] bf16
+  float* sLse = reinterpret_cast<float*>(sDST + C::kPBytes);  // [2][64] (log2 domain)
+  float* sDsum = sLse + 2 * 64;                               // [2][64]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sDsum + 2 * 64);
+  uint64_t* kv_full = bars;
+  uint64_t* q_full = bars + 1;    // [2]
+  uint64_t* q_empty = bars + 3;   // [2]
+  uint64_t* s_full = bars + 5;    // S^T and dP^T ready
+  uint64_t* p_full = bars + 6;    // P^T and dS^T written
+  uint64_t* acc_done = bars + 7;  // dV/dK MMAs of this chunk retired (P^T/dS^T reusable)
+  uint64_t* stat_full = bars + 8;  // per-q statistics of the chunk staged in shared memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // 1-D grid in cost order: under a causal mask the early kv blocks are seen by the most queries, and
+  // CTAs are handed out in block-index order, so the long ones start first
+  const int per_blk = p.Hkv * p.B;
+  const int kb = blockIdx.x / per_blk, hk = (blockIdx.x % per_blk) % p.Hkv, b = (blockIdx.x % per_blk) / p.Hkv;
+  const int k0 = kb * 128;
+  const int group = p.H / p.Hkv;
+  const int off = p.Tk - p.Tq;
+
+  // q rows that can see this kv block: q >= k0 - off (causal), q <= k0 + 127 - off + window - 1 (window)
+  int q_lo = 0, q_hi = p.Tq;
+  if (p.causal) q_lo = max(0, k0 - off);
+  if (p.window > 0) q_hi = min(p.Tq, k0 + 127 - off + p.window);
+  const int cb = q_lo / 64;
+  const int ce = q_hi > q_lo ? (q_hi + 63) / 64 : cb;
+  const int nchunk = ce - cb;
+  const int iters = nchunk * group;
+
+  if (threadIdx.x == 0) {
+    mbar_init(kv_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], 1);
+      mbar_init(&q_empty[s], 1);
+    }
+    mbar_init(s_full, 1);
+    mbar_init(p_full, 4);  // one arrival per math warp
+    mbar_init(acc_done, 1);
+    mbar_init(stat_full, 2);  // warps 0 and 1 stage the statistics
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 5) {
+    tmem_alloc(tmem_slot, C::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // this block has its tensor memory
+  pdl_wait();
+  const uint32_t tmem_st = tmem_base;         // S^T   64 cols
+  const uint32_t tmem_dpt = tmem_base + 64;   // dP^T  64 cols
+  const uint32_t tmem_dv = tmem_base + 128;   // dV    HD cols
+  const uint32_t tmem_dk = tmem_base + 128 + HD;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      mbar_arrive_expect_tx(kv_full, 2 * C::kKVBytes);
+      load_tile<HD>(sK, &tm_k, kv_full, 128, k0, hk, b, p.hfirst);
+      load_tile<HD>(sV, &tm_v, kv_full, 128, k0, hk, b, p.hfirst);
+      for (int it = 0; it < iters; ++it) {
+        const int s = it & 1;
+        const int hq = hk * group + it / nchunk;
+        const int c0 = (cb + it % nchunk) * 64;
+        if (!mbar_wait_bounded(&q_empty[s], ((it >> 1) & 1) ^ 1u, abort_flag)) {
+          atomicCAS(p.status, 0, kStatusTimeoutProducer);
+          break;
+        }
+        mbar_arrive_expect_tx(&q_full[s], 2 * C::kQBytes);
+        load_tile<HD>(sQ + s * C::kQBytes, &tm_q, &q_full[s], 64, c0, hq, b, p.hfirst);
+        load_tile<HD>(sDO + s * C::kQBytes, &tm_do, &q_full[s], 64, c0, hq, b, p.hfirst);
+      }
+    }
+  } else if (warp == 5) {
+    // the whole warp walks the loop (descriptors stay in uniform registers); one elected lane issues
+    {
+      const bool leader = elect_one();
+      const uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, false, false, 128, 64);   // K Q^T, V dO^T
+      const uint32_t idesc_g = make_idesc(kFmtBF16, kFmtBF16, false, true, 128, HD);    // P^T dO, dS^T Q
+      bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(kv_full, 0, abort_flag));
+      if (!ok && leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
+      const uint64_t dK = desc_kmajor(smem_u32(sK), 128, 0), dV = desc_kmajor(smem_u32(sV), 128, 0);
+      const uint64_t dPT = desc_kmajor(smem_u32(sPT), 128, 0), dDST = desc_kmajor(smem_u32(sDST), 128, 0);
+      for (int it = 0; it < iters && ok; ++it) {
+        const int s = it & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&q_full[s], (it >> 1) & 1, abort_flag))) {
+          if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t aQ = smem_u32(sQ + s * C::kQBytes), aDO = smem_u32(sDO + s * C::kQBytes);
+        const uint64_t dQk = desc_kmajor(aQ, 64, 0), dDOk = desc_kmajor(aDO, 64, 0);
+        const uint64_t dQm = desc_mnmajor(aQ, 64, 0), dDOm = desc_mnmajor(aDO, 64, 0);
+        if (leader) {
+#pragma unroll
+          for (int ks = 0; ks < HD / 16; ++ks)
+            umma_f16_ss(tmem_st, dK + kstep_kmajor(128, ks), dQk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
+#pragma unroll
+          for (int ks = 0; ks < HD / 16; ++ks)
+            umma_f16_ss(tmem_dpt, dV + kstep_kmajor(128, ks), dDOk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
+          umma_commit(s_full);
+        }
+        __syncwarp();
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(p_full, it & 1, abort_flag))) {
+          if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
+          break;
+        }
+        tc_fence_after_sync();
+        // dV += P^T dO ; dK += dS^T Q   (reduction over the 64 q rows of the chunk: 4 k-steps)
+        if (leader) {
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_f16_ss(tmem_dv, dPT + kstep_kmajor(128, ks), dDOm + kstep_mnmajor(ks), idesc_g,
+                        (it > 0 || ks > 0) ? 1u : 0u);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_f16_ss(tmem_dk, dDST + kstep_kmajor(128, ks), dQm + kstep_mnmajor(ks), idesc_g,
+                        (it > 0 || ks > 0) ? 1u : 0u);
+          umma_commit(&q_empty[s]);
+          umma_commit(acc_done);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    const int r = warp * 32 + lane;  // kv row inside the block == TMEM lane
+    const int k = k0 + r;
+    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
+    const float sc = p.scale * kLog2e;
+    // queries that may attend to key k:  k - off <= q (causal),  q <= k - off + window - 1 (window)
+    int q_row_lo = p.causal ? k - off : 0;
+    int q_row_hi = p.Tq - 1;
+    if (p.window > 0) q_row_hi = min(q_row_hi, k - off + p.window - 1);
+    if (k >= p.Tk) q_row_lo = 0x3fffffff;  // key out of range: nothing valid
+    bool ok = true;
+    for (int it = 0; it < iters; ++it) {
+      const int hq = hk * group + it / nchunk;
+      const int c0 = (cb + it % nchunk) * 64;
+      // stage the per-q statistics of this chunk (double-buffered by iteration parity)
+      float* lse_s = sLse + (it & 1) * 64;
+      float* ds_s = sDsum + (it & 1) * 64;
+      if (r < 64) {
+        const int q = c0 + r;
+        const int64_t idx = (static_cast<int64_t>(b) * p.H + hq) * p.Tq + q;
+        float l = q < p.Tq ? p.lse[idx] : INFINITY;
+        if (l == -INFINITY) l = INFINITY;  // row that saw no key: probabilities are zero
+        lse_s[r] = l * kLog2e;
+        ds_s[r] = q < p.Tq ? p.dsum[idx] : 0.0f;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(stat_full);
+      }
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(stat_full, it & 1, abort_flag));
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait_bounded(s_full, it & 1, abort_flag));
+      if (ok && it > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_done, (it - 1) & 1, abort_flag));
+      if (!ok) {
+        if (lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
+        break;
+      }
+      tc_fence_after_sync();
+      const bool need_mask = (k0 + 128 > p.Tk) || (c0 + 64 > p.Tq) || (p.causal && (k0 + 127 > c0 + off)) ||
+                             (p.window > 0 && (k0 < c0 + 63 + off - p.window + 1));
+      constexpr bool ext_on = EXT;
+      const ScoreExt ext = EXT ? make_ext(p, hq, b) : ScoreExt{};
+      auto body = [&](auto mask_tag, auto ext_tag) {
+        constexpr bool kMask = decltype(mask_tag)::value;
+        constexpr bool kExt = decltype(ext_tag)::value;
+#pragma unroll 1
+        for (int cc = 0; cc < 2; ++cc) {
+          uint32_t sv[32], dv[32];
+          tmem_ld_32x32b_x32(tmem_st + lane_addr + cc * 32, sv);
+          tmem_ld_32x32b_x32(tmem_dpt + lane_addr + cc * 32, dv);
+          tmem_ld_wait();
+          const int clo = q_row_lo - c0 - cc * 32, chi = q_row_hi - c0 - cc * 32;  // valid iff clo <= c <= chi
+          float pr[32], dsv[32];
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            const int qi = cc * 32 + c;
+            float sraw = __uint_as_float(sv[c]), dfac = 1.0f;
+            if (kExt) sraw = score_ext(ext, sraw, k - (c0 + qi + off), dfac);
+            float e = ex2f(fmaf(sraw, sc, -lse_s[qi]));
+            if (kMask && (c < clo || c > chi)) e = 0.0f;
+            float dp = __uint_as_float(dv[c]), keep = 1.0f;
+            if (kExt && ext.drop_p > 0.0f) {
+              keep = drop_scale_qk(ext, c0 + qi, k);
+              dp *= keep;
+            }
+            pr[c] = e * keep;  // what met V in the forward pass
+            dsv[c] = e * (dp - ds_s[qi]) * p.scale;
+            if (kExt) dsv[c] *= dfac;
+          }
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint4 w, z;
+            w.x = pack_bf16x2(pr[8 * g + 0], pr[8 * g + 1]);
+            w.y = pack_bf16x2(pr[8 * g + 2], pr[8 * g + 3]);
+            w.z = pack_bf16x2(pr[8 * g + 4], pr[8 * g + 5]);
+            w.w = pack_bf16x2(pr[8 * g + 6], pr[8 * g + 7]);
+            z.x = pack_bf16x2(dsv[8 * g + 0], dsv[8 * g + 1]);
+            z.y = pack_bf16x2(dsv[8 * g + 2], dsv[8 * g + 3]);
+            z.z = pack_bf16x2(dsv[8 * g + 4], dsv[8 * g + 5]);
+            z.w = pack_bf16x2(dsv[8 * g + 6], dsv[8 * g + 7]);
+            const uint32_t o = sw128_off(r, cc * 4 + g);
+            *reinterpret_cast<uint4*>(sPT + o) = w;
+            *reinterpret_cast<uint4*>(sDST + o) = z;
+          }
+        }
+      };
+      if (ext_on) {
+        if (need_mask) body(std::true_type{}, std::true_type{});
+        else body(std::false_type{}, std::true_type{});
+      } else {
+        if (need_mask) body(std::true_type{}, std::false_type{});
+        else body(std::false_type{}, std::false_type{});
+      }
+      fence_proxy_async_smem();  // this thread's tile writes -> visible to the tensor core's reads
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+    }
+    // drain: wait for the last accumulation, then write dK / dV rows
+    if (ok && iters > 0) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_done, (iters - 1) & 1, abort_flag));
+      if (!ok && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
+    }
+    if (ok) {  // warp-uniform: the TMEM loads below are warp-collective, only the stores are per row
+      tc_fence_after_sync();
+      const bool row_ok = k < p.Tk;
+      __nv_bfloat16* dk = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(b) * p.o_batch +
+                          static_cast<int64_t>(k) * p.o_row + static_cast<int64_t>(hk) * p.o_head;
+      __nv_bfloat16* dvp = reinterpret_cast<__nv_bfloat16*>(p.out2) + static_cast<int64_t>(b) * p.o2_batch +
+                           static_cast<int64_t>(k) * p.o2_row + static_cast<int64_t>(hk) * p.o2_head;
+#pragma unroll 1
+      for (int cc = 0; cc < HD / 32; ++cc) {
+        uint32_t a[32], c[32];
+        if (iters > 0) {
+          tmem_ld_32x32b_x32(tmem_dk + lane_addr + cc * 32, a);
+          tmem_ld_32x32b_x32(tmem_dv + lane_addr + cc * 32, c);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) a[i] = c[i] = 0u;
+        }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint4 w, z;
+          w.x = pack_bf16x2(__uint_as_float(a[8 * g + 0]), __uint_as_float(a[8 * g + 1]));
+          w.y = pack_bf16x2(__uint_as_float(a[8 * g + 2]), __uint_as_float(a[8 * g + 3]));
+          w.z = pack_bf16x2(__uint_as_float(a[8 * g + 4]), __uint_as_float(a[8 * g + 5]));
+          w.w = pack_bf16x2(__uint_as_float(a[8 * g + 6]), __uint_as_float(a[8 * g + 7]));
+          z.x = pack_bf16x2(__uint_as_float(c[8 * g + 0]), __uint_as_float(c[8 * g + 1]));
+          z.y = pack_bf16x2(__uint_as_float(c[8 * g + 2]), __uint_as_float(c[8 * g + 3]));
+          z.z = pack_bf16x2(__uint_as_float(c[8 * g + 4]), __uint_as_float(c[8 * g + 5]));
+          z.w = pack_bf16x2(__uint_as_float(c[8 * g + 6]), __uint_as_float(c[8 * g + 7]));
+          if (row_ok) {
+            reinterpret_cast<uint4*>(dk + cc * 32)[g] = w;
+            reinterpret_cast<uint4*>(dvp + cc * 32)[g] = z;
+          }
+        }
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag != 0) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(2000);
+    __syncthreads();
+  }
+  if (warp == 5) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, C::kTmemCols);
+  }
+}
+
+// ================================================================================================
+// backward at head size 64, part 2: dQ.  One CTA per (q block of 128, head, batch); loops over kv chunks of 64.
+// TMEM: S [128 q][64 kv], dP [128][64], dQ [128][HD].  Thread r owns q row r.
+// ================================================================================================
+struct Dq64Cfg {
+  static constexpr int HD = 64;
+  static constexpr int kQBytes = 128 * HD * 2;   // Q and dO tiles (resident)
+  static constexpr int kKVBytes = 64 * HD * 2;   // K / V chunk
+  static constexpr int kPBytes = 128 * 64 * 2;   // dS
+  static constexpr int kStages = 2;  // K / V chunk stages (a third one measured no faster)
+  static constexpr int kSmem = 2 * kQBytes + 2 * kStages * kKVBytes + kPBytes + 256;
+  static constexpr int kTmemCols = 256;  // 64 + 64 + HD
+};
+
+template <bool EXT>  // EXT: soft-capping / ALiBi / dropout row math (a build of its own)
+__global__ void __launch_bounds__(kBwd64Threads, 2)
+attn_bwd64_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                   const AttnDev p) {
+  using C = Dq64Cfg;
+  constexpr int HD = C::HD;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1 KiB aligned base; uniform early exit
+    if (threadIdx.x == 0) atomicCAS(p.status, 0, kStatusBadArgument);
+    return;
+  }
+  uint8_t* sQ = smem;
+  uint8_t* sDO = sQ + C::kQBytes;
+  constexpr int NS = C::kStages;
+  uint8_t* sK = sDO + C::kQBytes;        // NS stages
+  uint8_t* sV = sK + NS * C::kKVBytes;   // NS stages
+  uint8_t* sDS = sV + NS * C::kKVBytes;  // [128 q][64 kv] bf16
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + C::kPBytes);
+  uint64_t* q_full = bars;
+  uint64_t* kv_full = bars + 1;        // [NS]
+  uint64_t* kv_empty = kv_full + NS;   // [NS]
+  uint64_t* s_full = kv_empty + NS;
+  uint64_t* p_full = s_full + 1;
+  uint64_t* acc_done = p_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // 1-D grid in cost order (late q blocks see the most keys under a causal mask)
+  const int per_blk = p.H * p.B;
+  const int qb = p.nqb - 1 - blockIdx.x / per_blk;
+  const int h = (blockIdx.x % per_blk) % p.H, b = (blockIdx.x % per_blk) / p.H;
+  const int hk = h / (p.H / p.Hkv);
+  const int q0 = qb * 128;
+
+  int kv_lo, kv_hi;
+  kv_range(p, p.Tq, p.Tk, q0, min(128, p.Tq - q0), kv_lo, kv_hi);
+  const int jb = kv_lo / 64;
+  const int je = kv_hi > kv_lo ? (kv_hi + 63) / 64 : jb;
+  const int iters = je - jb;
+
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int s = 0; s < NS; ++s) {
+      mbar_init(&kv_full[s], 1);
+      mbar_init(&kv_empty[s], 1);
+    }
+    mbar_init(s_full, 1);
+    mbar_init(p_full, 4);  // one arrival per math warp
+    mbar_init(acc_done, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 5) {
+    tmem_alloc(tmem_slot, C::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // this block has its tensor memory
+  pdl_wait();
+  const uint32_t tmem_s = tmem_base;
+  const uint32_t tmem_dp = tmem_base + 64;
+  const uint32_t tmem_dq = tmem_base + 128;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      mbar_arrive_expect_tx(q_full, 2 * C::kQBytes);
+      load_tile<HD>(sQ, &tm_q, q_full, 128, q0, h, b, p.hfirst);
+      load_tile<HD>(sDO, &tm_do, q_full, 128, q0, h, b, p.hfirst);
+      for (int it = 0; it < iters; ++it) {
+        const int s = it % NS;
+        if (!mbar_wait_bounded(&kv_empty[s], ((it / NS) & 1) ^ 1u, abort_flag)) {
+          atomicCAS(p.status, 0, kStatusTimeoutProducer);
+          break;
+        }
+        mbar_arrive_expect_tx(&kv_full[s], 2 * C::kKVBytes);
+        load_tile<HD>(sK + s * C::kKVBytes, &tm_k, &kv_full[s], 64, (jb + it) * 64, hk, b, p.hfirst);
+        load_tile<HD>(sV + s * C::kKVBytes, &tm_v, &kv_full[s], 64, (jb + it) * 64, hk, b, p.hfirst);
+      }
+    }
+  } else if (warp == 5) {
+    // the whole warp walks the loop (descriptors stay in uniform registers); one elected lane issues
+    {
+      const bool leader = elect_one();
+      const uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, false, false, 128, 64);  // Q K^T, dO V^T
+      const uint32_t idesc_g = make_idesc(kFmtBF16, kFmtBF16, false, true, 128, HD);   // dS K
+      bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(q_full, 0, abort_flag));
+      if (!ok && leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
+      const uint64_t dQ = desc_kmajor(smem_u32(sQ), 128, 0), dDO = desc_kmajor(smem_u32(sDO), 128, 0);
+      const uint64_t dDS = desc_kmajor(smem_u32(sDS), 128, 0);
+      for (int it = 0; it < iters && ok; ++it) {
+        const int s = it % NS;
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(&kv_full[s], (it / NS) & 1, abort_flag))) {
+          if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t aK = smem_u32(sK + s * C::kKVBytes), aV = smem_u32(sV + s * C::kKVBytes);
+        const uint64_t dKk = desc_kmajor(aK, 64, 0), dVk = desc_kmajor(aV, 64, 0), dKm = desc_mnmajor(aK, 64, 0);
+        if (leader) {
+#pragma unroll
+          for (int ks = 0; ks < HD / 16; ++ks)
+            umma_f16_ss(tmem_s, dQ + kstep_kmajor(128, ks), dKk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
+#pragma unroll
+          for (int ks = 0; ks < HD / 16; ++ks)
+            umma_f16_ss(tmem_dp, dDO + kstep_kmajor(128, ks), dVk + kstep_kmajor(64, ks), idesc_s, ks > 0 ? 1u : 0u);
+          umma_commit(s_full);
+        }
+        __syncwarp();
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(p_full, it & 1, abort_flag))) {
+          if (leader) atomicCAS(p.status, 0, kStatusTimeoutMma);
+          break;
+        }
+        tc_fence_after_sync();
+        if (leader) {
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_f16_ss(tmem_dq, dDS + kstep_kmajor(128, ks), dKm + kstep_mnmajor(ks), idesc_g,
+                        (it > 0 || ks > 0) ? 1u : 0u);
+          umma_commit(&kv_empty[s]);
+          umma_commit(acc_done);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    const int r = warp * 32 + lane;
+    const int q = q0 + r;
+    const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
+    const float sc = p.scale * kLog2e;
+    const int off = p.Tk - p.Tq;
+    const int64_t sidx = (static_cast<int64_t>(b) * p.H + h) * p.Tq + q;
+    float lse_n = q < p.Tq ? p.lse[sidx] : INFINITY;
+    if (lse_n == -INFINITY) lse_n = INFINITY;  // row that saw no key: probabilities are zero
+    const float lse2 = lse_n * kLog2e;
+    // dsum = rowsum(dO * O) of this thread's row, straight from global memory (the loads overlap the first tiles'
+    // TMA traffic); published for the dK/dV kernel
+    float dsum = 0.0f;
+    if (q < p.Tq) {
+      const uint4* orow = reinterpret_cast<const uint4*>(p.o_in + static_cast<int64_t>(b) * p.oi_batch +
+                                                         static_cast<int64_t>(q) * p.oi_row + static_cast<int64_t>(h) * p.oi_head);
+      const uint4* grow = reinterpret_cast<const uint4*>(p.do_in + static_cast<int64_t>(b) * p.di_batch +
+                                                         static_cast<int64_t>(q) * p.di_row + static_cast<int64_t>(h) * p.di_head);
+      float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll
+      for (int i = 0; i < HD / 8; ++i) {
+        const uint4 ov = orow[i], gv = grow[i];
+        const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float x0, x1, y0, y1;
+          unpack_bf16x2(ow[j], x0, x1);
+          unpack_bf16x2(gw[j], y0, y1);
+          a0 = fmaf(x0, y0, a0);
+          a1 = fmaf(x1, y1, a1);
+        }
+      }
+      dsum = a0 + a1;
+      p.dsum_out[sidx] = dsum;
+    }
+    int row_lo, row_hi;
+    row_limits(p, p.Tq, p.Tk, q, row_lo, row_hi);
+    if (q >= p.Tq) row_lo = 0x3fffffff;
+    constexpr bool ext_on = EXT;
+    const ScoreExt ext = EXT ? make_ext(p, h, b) : ScoreExt{};
+    bool ok = true;
+    for (int it = 0; it < iters; ++it) {
+      const int k0 = (jb + it) * 64;
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(s_full, it & 1, abort_flag));
+      if (ok && it > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_done, (it - 1) & 1, abort_flag));
+      if (!ok) {
+        if (lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
+        break;
+      }
+      tc_fence_after_sync();
+      const bool need_mask = (k0 + 64 > p.Tk) || (q0 + 128 > p.Tq) || (p.causal && (k0 + 63 > q0 + off)) ||
+                             (p.window > 0 && (k0 < q0 + 127 + off - p.window + 1));
+      auto body = [&](auto mask_tag, auto ext_tag) {
+        constexpr bool kMask = decltype(mask_tag)::value;
+        constexpr bool kExt = decltype(ext_tag)::value;
+#pragma unroll 1
+        for (int cc = 0; cc < 2; ++cc) {
+          uint32_t sv[32], dv[32];
+          tmem_ld_32x32b_x32(tmem_s + lane_addr + cc * 32, sv);
+          tmem_ld_32x32b_x32(tmem_dp + lane_addr + cc * 32, dv);
+          tmem_ld_wait();
+          const int clo = row_lo - k0 - cc * 32, chi = row_hi - k0 - cc * 32;
+          float dsv[32];
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            float sraw = __uint_as_float(sv[c]), dfac = 1.0f;
+            if (kExt) sraw = score_ext(ext, sraw, k0 + cc * 32 + c - (q + off), dfac);
+            float e = ex2f(fmaf(sraw, sc, -lse2));
+            if (kMask && (c < clo || c > chi)) e = 0.0f;
+            float dp = __uint_as_float(dv[c]);
+            if (kExt && ext.drop_p > 0.0f) dp *= drop_scale_qk(ext, q, k0 + cc * 32 + c);
+            dsv[c] = e * (dp - dsum) * p.scale;
+            if (kExt) dsv[c] *= dfac;
+          }
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint4 z;
+            z.x = pack_bf16x2(dsv[8 * g + 0], dsv[8 * g + 1]);
+            z.y = pack_bf16x2(dsv[8 * g + 2], dsv[8 * g + 3]);
+            z.z = pack_bf16x2(dsv[8 * g + 4], dsv[8 * g + 5]);
+            z.w = pack_bf16x2(dsv[8 * g + 6], dsv[8 * g + 7]);
+            *reinterpret_cast<uint4*>(sDS + sw128_off(r, cc * 4 + g)) = z;
+          }
+        }
+      };
+      if (ext_on) {
+        if (need_mask) body(std::true_type{}, std::true_type{});
+        else body(std::false_type{}, std::true_type{});
+      } else {
+        if (need_mask) body(std::true_type{}, std::false_type{});
+        else body(std::false_type{}, std::false_type{});
+      }
+      fence_proxy_async_smem();  // this thread's tile writes -> visible to the tensor core's reads
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+    }
+    if (ok && iters > 0) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(acc_done, (iters - 1) & 1, abort_flag));
+      if (!ok && lane == 0) atomicCAS(p.status, 0, kStatusTimeoutEpilogue);
+    }
+    if (ok) {  // warp-uniform: the TMEM loads below are warp-collective, only the stores are per row
+      tc_fence_after_sync();
+      const bool row_ok = q < p.Tq;
+      __nv_bfloat16* dq = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<int64_t>(b) * p.o_batch +
+                          static_cast<int64_t>(q) * p.o_row + static_cast<int64_t>(h) * p.o_head;
+#pragma unroll 1
+      for (int cc = 0; cc < HD / 32; ++cc) {
+        uint32_t a[32];
+        if (iters > 0) {
+          tmem_ld_32x32b_x32(tmem_dq + lane_addr + cc * 32, a);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) a[i] = 0u;
+        }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint4 w;
+          w.x = pack_bf16x2(__uint_as_float(a[8 * g + 0]), __uint_as_float(a[8 * g + 1]));
+          w.y = pack_bf16x2(__uint_as_float(a[8 * g + 2]), __uint_as_float(a[8 * g + 3]));
+          w.z = pack_bf16x2(__uint_as_float(a[8 * g + 4]), __uint_as_float(a[8 * g + 5]));
+          w.w = pack_bf16x2(__uint_as_float(a[8 * g + 6]), __uint_as_float(a[8 * g + 7]));
+          if (row_ok) reinterpret_cast<uint4*>(dq + cc * 32)[g] = w;
+        }
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag != 0) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(2000);
+    __syncthreads();
+  }
+  if (warp == 5) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, C::kTmemCols);
+  }
+}
+
+// ================================================================================================
+// backward at head size 128, one CTA per SM: the score products of chunk i + 1 are issued ahead of the gradient products of chunk i, into a
+// second pair of score tiles, while the math of chunk i runs.  Two threads (warps w and w + 4) share a row, 32 of a chunk's 64 columns
+// each.  The factor `scale` of dS goes to the results.
+// On 2 x 32 (8) x 4096 x 128, causal, dK / dV takes 542 us and dQ 510; with four math warps and the four steps in turn it was 797
+// and 759, the tensor cores busy for a quarter of that.
+// ================================================================================================
+constexpr int kBwdMathWarps = 8;  // row quarter = warp & 3, column half = warp >> 2
+constexpr int kBwdThreads = (kBwdMathWarps + 2) * 32;  // then one warp for TMA, one for MMA + TMEM
 
 // NC score columns and as many of dP, one wait
 template <int NC>
@@ -1137,29 +1741,29 @@ __device__ __forceinline__ void store_row32_scaled(__nv_bfloat16* dst, const uin
 }
 
 // ================================================================================================
-// backward, part 1: dK / dV.  One CTA per (kv block of 128, kv head, batch); loops over the q heads
+// part 1: dK / dV.  One CTA per (kv block of 128, kv head, batch); loops over the q heads
 // of the group and over q chunks of 64 rows.  TMEM: S^T [128 kv][64 q], dP^T [128][64], dV [128][HD],
-// dK [128][HD].  The thread (at head size 128 the two threads) of row r owns kv row r.
+// dK [128][HD].  The two threads of row r own kv row r.
 // ================================================================================================
 template <int HD>
 struct DkvCfg {
   static constexpr int kKVBytes = 128 * HD * 2;   // K and V tiles (resident)
   static constexpr int kQBytes = 64 * HD * 2;     // Q / dO chunk
   static constexpr int kPBytes = 128 * 64 * 2;    // P^T and dS^T
-  static constexpr int kTiles = (HD == 64) ? 1 : 2;   // score tiles in TMEM
-  static constexpr int kStages = (HD == 64) ? 2 : 3;  // Q / dO chunks
-  static constexpr int kPBufs = (HD == 64) ? 1 : 2;   // P^T / dS^T buffers (two CTAs per SM leave room for one)
+  static constexpr int kTiles = 2;   // score tiles in TMEM
+  static constexpr int kStages = 3;  // Q / dO chunks
+  static constexpr int kPBufs = 2;   // P^T / dS^T buffers
   static constexpr int kSmem = 2 * kKVBytes + 2 * kStages * kQBytes + 2 * kPBufs * kPBytes + 4 * 2 * 64 * 4 + 192;
-  static constexpr int kTmemCols = (HD == 64) ? 256 : 512;  // kTiles * 128 + 2 * HD
+  static constexpr int kTmemCols = 512;  // kTiles * 128 + 2 * HD
 };
 
 template <int HD, bool EXT>  // EXT: soft-capping / ALiBi / dropout row math (a build of its own)
-__global__ void __launch_bounds__(bwd_threads(HD), (HD == 64 ? 2 : 1))
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                      const AttnDev p) {
   using C = DkvCfg<HD>;
-  constexpr int NS = C::kStages, NT = C::kTiles, NP = C::kPBufs, NC = 32, MW = bwd_math_warps(HD), kSpan = 64 / (MW / 4);  // kSpan: columns of a chunk per math thread
+  constexpr int NS = C::kStages, NT = C::kTiles, NP = C::kPBufs, NC = 32, MW = kBwdMathWarps, kSpan = 64 / (MW / 4);  // kSpan: columns of a chunk per math thread
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1 KiB aligned base; uniform early exit
@@ -1276,9 +1880,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     };
     if (iters > 0) scores(0);
     for (int it = 0; it < iters && ok; ++it) {
-      if (NT == 2 && it + 1 < iters) scores(it + 1);
+      if (it + 1 < iters) scores(it + 1);
       ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&p_full[it & 1], (it >> 1) & 1, abort_flag));
-      if (NT == 1 && it + 1 < iters) scores(it + 1);
       if (!ok) break;
       tc_fence_after_sync();
       // dV += P^T dO ; dK += dS^T Q   (reduction over the 64 q rows of the chunk: 4 k-steps)
@@ -1455,26 +2058,26 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 
 // ================================================================================================
 // backward, part 2: dQ.  One CTA per (q block of 128, head, batch); loops over kv chunks of 64.
-// TMEM: S [128 q][64 kv], dP [128][64], dQ [128][HD].  The thread (at head size 128 the two threads) of row r owns q row r.
+// TMEM: S [128 q][64 kv], dP [128][64], dQ [128][HD].  The two threads of row r own q row r.
 // ================================================================================================
 template <int HD>
 struct DqCfg {
   static constexpr int kQBytes = 128 * HD * 2;   // Q and dO tiles (resident)
   static constexpr int kKVBytes = 64 * HD * 2;   // K / V chunk
   static constexpr int kPBytes = 128 * 64 * 2;   // dS
-  static constexpr int kTiles = (HD == 64) ? 1 : 2;  // score tiles in TMEM
+  static constexpr int kTiles = 2;  // score tiles in TMEM
   static constexpr int kStages = 3;
   static constexpr int kSmem = 2 * kQBytes + 2 * kStages * kKVBytes + 2 * kPBytes + 192;
-  static constexpr int kTmemCols = (HD == 64) ? 256 : 512;  // kTiles * 128 + HD
+  static constexpr int kTmemCols = 512;  // kTiles * 128 + HD
 };
 
 template <int HD, bool EXT>  // EXT: soft-capping / ALiBi / dropout row math (a build of its own)
-__global__ void __launch_bounds__(bwd_threads(HD), (HD == 64 ? 2 : 1))
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                    const AttnDev p) {
   using C = DqCfg<HD>;
-  constexpr int NS = C::kStages, NT = C::kTiles, NC = 32, MW = bwd_math_warps(HD), kSpan = 64 / (MW / 4);  // kSpan: columns of a chunk per math thread
+  constexpr int NS = C::kStages, NT = C::kTiles, NC = 32, MW = kBwdMathWarps, kSpan = 64 / (MW / 4);  // kSpan: columns of a chunk per math thread
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // the swizzled tiles need a 1 KiB aligned base; uniform early exit
@@ -1579,9 +2182,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     };
     if (iters > 0) scores(0);
     for (int it = 0; it < iters && ok; ++it) {
-      if (NT == 2 && it + 1 < iters) scores(it + 1);
+      if (it + 1 < iters) scores(it + 1);
       ok = ok && __all_sync(0xffffffffu, mbar_wait_bounded(&p_full[it & 1], (it >> 1) & 1, abort_flag));
-      if (NT == 1 && it + 1 < iters) scores(it + 1);
       if (!ok) break;
       tc_fence_after_sync();
       const int s = it % NS;
@@ -1634,13 +2236,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
       dsum = a0 + a1;
     }
-    if constexpr (MW == 8) {
-      float* sX = reinterpret_cast<float*>(sDS);  // [2][128]
-      sX[half * 128 + r] = dsum;
-      softmax_bar();
-      dsum = sX[r] + sX[128 + r];
-      softmax_bar();
-    }
+    float* sX = reinterpret_cast<float*>(sDS);  // [2][128]
+    sX[half * 128 + r] = dsum;
+    softmax_bar();
+    dsum = sX[r] + sX[128 + r];
+    softmax_bar();
     if (half == 0 && q < p.Tq) p.dsum_out[sidx] = dsum;
     int row_lo, row_hi;
     row_limits(p, p.Tq, p.Tk, q, row_lo, row_hi);
@@ -1795,6 +2395,12 @@ int check_args(const NxAttnArgs* a) {
   return 0;
 }
 
+// Whether a kernel of head size 64 is launched to begin while the one in front drains.  Its blocks then go where room comes first, two
+// to an SM, and the long ones, which lead the grid, share SMs while others have one or none: 1 x 16 (4) x 4096 forward, dependent and
+// plain, 99.2 and 88.2 us, soft-capped 198 and 161, 8 x 12 x 512 22.5 and 18.9; dK / dV of the first 32 us more.  Short sequences gain
+// the launch (3 x 4 x 203: 7.7 and 8.4).  At head size 128 an SM holds one block either way.
+bool dependent64(const NxAttnArgs* a) { return a->tq <= 256 && a->tk <= 256; }
+
 }  // namespace
 
 extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
@@ -1843,7 +2449,10 @@ extern "C" int nx_attention_fwd(const NxAttnArgs* a, nx_stream_t stream_) {
 #define NX_FWD(HD_, EXT_)                                                                           \
   do {                                                                                              \
     NX_ALLOW_SMEM((attn_fwd_kernel<HD_, EXT_, false>), FwdCfg<HD_>::kSmem);                         \
-    NX_PDL((attn_fwd_kernel<HD_, EXT_, false>), grid, kFwdThreads, FwdCfg<HD_>::kSmem, st, tq, tk, tv, p);  \
+    if (HD_ == 128 || dependent64(a))                                                               \
+      NX_PDL((attn_fwd_kernel<HD_, EXT_, false>), grid, kFwdThreads, FwdCfg<HD_>::kSmem, st, tq, tk, tv, p);\
+    else                                                                                            \
+      attn_fwd_kernel<HD_, EXT_, false><<<grid, kFwdThreads, FwdCfg<HD_>::kSmem, st>>>(tq, tk, tv, p);      \
   } while (0)
   const int mode = !ext ? 0 : (p.alibi == nullptr && p.dropout_p <= 0.0f && p.scale > 0.0f ? 2 : 1);
   if (HD == 64) {
@@ -1911,10 +2520,16 @@ extern "C" int nx_attention_bwd(const NxAttnArgs* a, nx_stream_t stream_) {
   const int HD = a->head_dim;
   const bool ext = a->softcap > 0.0f || a->alibi_slopes != nullptr || a->dropout_p > 0.0f;
   int rc;
+#define NX_BWD64(KERN_, CFG_, EXT_)                                                                 \
+  do {                                                                                              \
+    NX_ALLOW_SMEM(KERN_<EXT_>, CFG_::kSmem);                                                        \
+    if (dependent64(a)) NX_PDL(KERN_<EXT_>, grid, kBwd64Threads, CFG_::kSmem, st, tq, tk, tv, tdo, p);      \
+    else KERN_<EXT_><<<grid, kBwd64Threads, CFG_::kSmem, st>>>(tq, tk, tv, tdo, p);                 \
+  } while (0)
 #define NX_BWD(KERN_, CFG_, HD_, EXT_)                                                              \
   do {                                                                                              \
     NX_ALLOW_SMEM((KERN_<HD_, EXT_>), CFG_<HD_>::kSmem);                                            \
-    NX_PDL((KERN_<HD_, EXT_>), grid, bwd_threads(HD_), CFG_<HD_>::kSmem, st, tq, tk, tv, tdo, p);           \
+    NX_PDL((KERN_<HD_, EXT_>), grid, kBwdThreads, CFG_<HD_>::kSmem, st, tq, tk, tv, tdo, p);                \
   } while (0)
   // part 1: dQ (also forms dsum = rowsum(dO * O) and leaves it for part 2)
   {
@@ -1940,8 +2555,8 @@ extern "C" int nx_attention_bwd(const NxAttnArgs* a, nx_stream_t stream_) {
     p.dsum_out = a->dsum;
     const unsigned grid = static_cast<unsigned>(p.nqb * a->heads * a->batch);
     if (HD == 64) {
-      if (ext) NX_BWD(attn_bwd_dq_kernel, DqCfg, 64, true);
-      else NX_BWD(attn_bwd_dq_kernel, DqCfg, 64, false);
+      if (ext) NX_BWD64(attn_bwd64_dq_kernel, Dq64Cfg, true);
+      else NX_BWD64(attn_bwd64_dq_kernel, Dq64Cfg, false);
     } else {
       if (ext) NX_BWD(attn_bwd_dq_kernel, DqCfg, 128, true);
       else NX_BWD(attn_bwd_dq_kernel, DqCfg, 128, false);
@@ -1965,14 +2580,15 @@ extern "C" int nx_attention_bwd(const NxAttnArgs* a, nx_stream_t stream_) {
     p.o2_batch = a->dv.batch_stride;
     const unsigned grid = static_cast<unsigned>(((a->tk + 127) / 128) * a->kv_heads * a->batch);
     if (HD == 64) {
-      if (ext) NX_BWD(attn_bwd_dkdv_kernel, DkvCfg, 64, true);
-      else NX_BWD(attn_bwd_dkdv_kernel, DkvCfg, 64, false);
+      if (ext) NX_BWD64(attn_bwd64_dkdv_kernel, Dkv64Cfg, true);
+      else NX_BWD64(attn_bwd64_dkdv_kernel, Dkv64Cfg, false);
     } else {
       if (ext) NX_BWD(attn_bwd_dkdv_kernel, DkvCfg, 128, true);
       else NX_BWD(attn_bwd_dkdv_kernel, DkvCfg, 128, false);
     }
     if (cudaGetLastError() != cudaSuccess) return -2;
   }
+#undef NX_BWD64
 #undef NX_BWD
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

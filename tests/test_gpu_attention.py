@@ -280,3 +280,22 @@ def test_backward_in_a_thread_that_made_no_runtime_call_yet():
     th.start()
     th.join()
     assert out and all(torch.equal(a, b) for a, b in zip(out[0], want))
+
+
+@pytest.mark.parametrize("Tq,Tk", [(256, 256), (257, 257), (256, 257), (40, 300)])
+@pytest.mark.parametrize("softcap", [0.0, 20.0])
+def test_head_size_64_in_both_launch_forms(Tq, Tk, softcap):
+    """Sequences of up to 256 are dependent launches, longer ones plain: forward and gradients one after another on one stream, against
+    the FP32 form.  BF16 results of sums of values of order one: 2^-8 of the largest, twice for the rounded operands."""
+    from nexus_b200.fused import ops
+    torch.manual_seed(18)
+    q, do = (torch.randn(2, Tq, 4, 64, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(2, Tk, 2, 64, device="cuda").bfloat16() for _ in range(2))
+    for _ in range(3):
+        leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        o = ops.attention(*leaves, softcap=softcap)
+        got = (o, *torch.autograd.grad(o, leaves, do))
+    ref = [t.float().requires_grad_(True) for t in (q, k, v)]
+    w = ops.attention_reference(*ref, softcap=softcap)
+    for a, b in zip(got, (w, *torch.autograd.grad(w, ref, do.float()))):
+        assert (a.float() - b).abs().max() < 2.0 ** -7 * b.abs().max()
