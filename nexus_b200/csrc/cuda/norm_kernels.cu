@@ -125,10 +125,12 @@ __global__ void norm_fwd_kernel(const XT* __restrict__ x, const XT* __restrict__
 }
 
 // Rows of 128 * VPL columns (kTail: of up to that many): a warp keeps its row in registers (VPL vectors of four per lane), so the row is read
-// from memory once with all of its loads in flight together, and gamma / beta are loaded once per warp.  Same
+// from memory once with all of its loads in flight together.  gamma / beta are loaded once per warp up to 1024 columns, longer ones with
+// every row: beside the row they took 192 registers and more, so that few rows were on the way at once (16384 rows of 1600 in BF16:
+// 47 us, 37 a row read three times by many warps).  Same
 // arithmetic and summation order as norm_fwd_kernel.
 template <typename XT, typename PT, typename YT, bool kRms, int VPL, bool kTail>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(VPL > 8 ? 128 : 256)
 norm_fwd_reg_kernel(const XT* __restrict__ x, const XT* __restrict__ res, XT* __restrict__ sum_out,
                     const PT* __restrict__ gamma, const PT* __restrict__ beta, YT* __restrict__ y,
                     float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols, float eps) {
@@ -137,16 +139,19 @@ norm_fwd_reg_kernel(const XT* __restrict__ x, const XT* __restrict__ res, XT* __
   const int kCols = kTail ? cols : 128 * VPL, nvec = kCols >> 2;
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
-  float g[VPL][4], b[VPL][4];
+  constexpr bool kKeep = VPL <= 8;   // gamma and beta beside the row in registers
+  float g[kKeep ? VPL : 1][4], b[kKeep ? VPL : 1][4];
+  if constexpr (kKeep) {
 #pragma unroll
-  for (int i = 0; i < VPL; ++i) {
-    const bool in = !kTail || lane + 32 * i < nvec;
-    if (in) Vec4<PT>::load(gamma + 4 * (lane + 32 * i), g[i]);
-    if (!kRms && beta && in) {
-      Vec4<PT>::load(beta + 4 * (lane + 32 * i), b[i]);
-    } else {
+    for (int i = 0; i < VPL; ++i) {
+      const bool in = !kTail || lane + 32 * i < nvec;
+      if (in) Vec4<PT>::load(gamma + 4 * (lane + 32 * i), g[i]);
+      if (!kRms && beta && in) {
+        Vec4<PT>::load(beta + 4 * (lane + 32 * i), b[i]);
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[i][j] = 0.0f;
+        for (int j = 0; j < 4; ++j) b[i][j] = 0.0f;
+      }
     }
   }
   for (int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps_per_block) {
@@ -219,12 +224,17 @@ norm_fwd_reg_kernel(const XT* __restrict__ x, const XT* __restrict__ res, XT* __
     for (int i = 0; i < VPL; ++i) {
       if (kTail && lane + 32 * i >= nvec) continue;
       float o[4];
+      if constexpr (!kKeep) {
+        Vec4<PT>::load(gamma + 4 * (lane + 32 * i), g[0]);
+        if (!kRms && beta) Vec4<PT>::load(beta + 4 * (lane + 32 * i), b[0]);
+      }
+      const int at = kKeep ? i : 0;
       if (!kRms && beta) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] = (v[i][j] - mean) * rstd * g[i][j] + b[i][j];
+        for (int j = 0; j < 4; ++j) o[j] = (v[i][j] - mean) * rstd * g[at][j] + b[at][j];
       } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] = (v[i][j] - mean) * rstd * g[i][j];
+        for (int j = 0; j < 4; ++j) o[j] = (v[i][j] - mean) * rstd * g[at][j];
       }
       Vec4<YT>::store(yr + 4 * (lane + 32 * i), o);
     }
@@ -427,8 +437,9 @@ int launch_fwd(bool rms, const void* x, const void* res, void* sum_out, const vo
   static const bool no_reg = std::getenv("NX_NORM_FWD_GENERIC") != nullptr;  // measurement switch
   // A warp per row; few rows go to as many SMs as there are (64 rows of 1600: 10.4 us by eight blocks of the generic kernel,
   // 3.1 us now; 4096 rows of 2048 in BF16: 11.5 and 7.3 us).
-  const int few_wpb = std::max(1, std::min(wpb, rows / kNumSmsB200)), few_blocks = std::min((rows + few_wpb - 1) / few_wpb, kNumSmsB200 * 8);
-  if (!no_reg && ((cols % 128 == 0 && cols <= 1024) || (cols > 1024 && cols <= 2048))) {
+  // Rows of more than 1024 columns leave room for fewer warps: blocks of four, which fill an SM's registers more evenly.
+  const int few_wpb = std::max(1, std::min(cols > 1024 ? 4 : wpb, rows / kNumSmsB200)), few_blocks = std::min((rows + few_wpb - 1) / few_wpb, kNumSmsB200 * 8);
+  if (!no_reg && (cols % 128 == 0 || cols > 512) && cols <= 2048) {
 #define NX_FWD_REG(V_, TAIL_)                                                                                                  \
   {                                                                                                                            \
     if (rms)                                                                                                                   \
@@ -441,6 +452,7 @@ int launch_fwd(bool rms, const void* x, const void* res, void* sum_out, const vo
   }
     if (cols > 1536) NX_FWD_REG(16, true)
     if (cols > 1024) NX_FWD_REG(12, true)
+    if (cols % 128 != 0) NX_FWD_REG(8, true)
     switch (cols / 128) {
       case 1: NX_FWD_REG(1, false)
       case 2: NX_FWD_REG(2, false)
@@ -453,8 +465,8 @@ int launch_fwd(bool rms, const void* x, const void* res, void* sum_out, const vo
     }
 #undef NX_FWD_REG
   }
-  // Shorter rows leave most of a block's threads without work (a warp per row stays), longer ones do not fit its registers.
-  if (!no_reg && cols > 512 && cols <= 8192) {
+  // Longer rows do not fit a block's registers either.
+  if (!no_reg && cols > 2048 && cols <= 8192) {
     const int grid = std::min(rows, kNumSmsB200 * 8);
 #define NX_FWD_BLOCK(V_)                                                                                                       \
   {                                                                                                                            \
@@ -467,7 +479,6 @@ int launch_fwd(bool rms, const void* x, const void* res, void* sum_out, const vo
     return launch_status();                                                                                                    \
   }
     const int vec = (cols / 4 + threads - 1) / threads;
-    if (vec <= 1) NX_FWD_BLOCK(1)
     if (vec <= 4) NX_FWD_BLOCK(4)
     NX_FWD_BLOCK(8)
 #undef NX_FWD_BLOCK
