@@ -125,12 +125,11 @@ __global__ void norm_fwd_kernel(const XT* __restrict__ x, const XT* __restrict__
 }
 
 // Rows of 128 * VPL columns (kTail: of up to that many): a warp keeps its row in registers (VPL vectors of four per lane), so the row is read
-// from memory once with all of its loads in flight together.  gamma / beta are loaded once per warp up to 1024 columns, longer ones with
-// every row: beside the row they took 192 registers and more, so that few rows were on the way at once (16384 rows of 1600 in BF16:
-// 47 us, 37 a row read three times by many warps).  Same
+// from memory once with all of its loads in flight together.  kKeep: so are gamma and beta, loaded once per warp before the statistics;
+// otherwise they are loaded with every row after them (see launch_fwd).  Same
 // arithmetic and summation order as norm_fwd_kernel.
-template <typename XT, typename PT, typename YT, bool kRms, int VPL, bool kTail>
-__global__ void __launch_bounds__(VPL > 8 ? 128 : 256)
+template <typename XT, typename PT, typename YT, bool kRms, int VPL, bool kTail, bool kKeep>
+__global__ void __launch_bounds__(kKeep ? 256 : 128)
 norm_fwd_reg_kernel(const XT* __restrict__ x, const XT* __restrict__ res, XT* __restrict__ sum_out,
                     const PT* __restrict__ gamma, const PT* __restrict__ beta, YT* __restrict__ y,
                     float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols, float eps) {
@@ -139,7 +138,6 @@ norm_fwd_reg_kernel(const XT* __restrict__ x, const XT* __restrict__ res, XT* __
   const int kCols = kTail ? cols : 128 * VPL, nvec = kCols >> 2;
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
-  constexpr bool kKeep = VPL <= 8;   // gamma and beta beside the row in registers
   float g[kKeep ? VPL : 1][4], b[kKeep ? VPL : 1][4];
   if constexpr (kKeep) {
 #pragma unroll
@@ -437,31 +435,37 @@ int launch_fwd(bool rms, const void* x, const void* res, void* sum_out, const vo
   static const bool no_reg = std::getenv("NX_NORM_FWD_GENERIC") != nullptr;  // measurement switch
   // A warp per row; few rows go to as many SMs as there are (64 rows of 1600: 10.4 us by eight blocks of the generic kernel,
   // 3.1 us now; 4096 rows of 2048 in BF16: 11.5 and 7.3 us).
-  // Rows of more than 1024 columns leave room for fewer warps: blocks of four, which fill an SM's registers more evenly.
-  const int few_wpb = std::max(1, std::min(cols > 1024 ? 4 : wpb, rows / kNumSmsB200)), few_blocks = std::min((rows + few_wpb - 1) / few_wpb, kNumSmsB200 * 8);
+  // Rows of more than 1024 columns with gamma and beta in registers (up to 255 a thread) leave an SM eight rows on the way.  That is
+  // enough for few rows, and the loads overlap (64 rows of 1600 in FP32: 2.5 us, 4.7 with the loads behind the statistics; 609: 3.1 and
+  // 5.2; 1200 in BF16: 6.4 and 5.6); many
+  // rows take them from the cache in blocks of four warps (16384 rows of 1600 in BF16: 47.5 and 28.3 us, 37 by the general kernel).
+  const bool keep = cols <= 1024 || rows <= 6 * kNumSmsB200;
+  const int few_wpb = std::max(1, std::min(keep ? wpb : 4, rows / kNumSmsB200)), few_blocks = std::min((rows + few_wpb - 1) / few_wpb, kNumSmsB200 * 8);
   if (!no_reg && (cols % 128 == 0 || cols > 512) && cols <= 2048) {
-#define NX_FWD_REG(V_, TAIL_)                                                                                                  \
+#define NX_FWD_REG(V_, TAIL_, KEEP_)                                                                                                  \
   {                                                                                                                            \
     if (rms)                                                                                                                   \
-      NX_PDL((norm_fwd_reg_kernel<XT, PT, YT, true, V_, TAIL_>), few_blocks, 32 * few_wpb, 0, st, \
+      NX_PDL((norm_fwd_reg_kernel<XT, PT, YT, true, V_, TAIL_, KEEP_>), few_blocks, 32 * few_wpb, 0, st, \
           (const XT*)x, (const XT*)res, (XT*)sum_out, (const PT*)gamma, (const PT*)beta, (YT*)y, mean, rstd, rows, cols, eps); \
     else                                                                                                                       \
-      NX_PDL((norm_fwd_reg_kernel<XT, PT, YT, false, V_, TAIL_>), few_blocks, 32 * few_wpb, 0, st, \
+      NX_PDL((norm_fwd_reg_kernel<XT, PT, YT, false, V_, TAIL_, KEEP_>), few_blocks, 32 * few_wpb, 0, st, \
           (const XT*)x, (const XT*)res, (XT*)sum_out, (const PT*)gamma, (const PT*)beta, (YT*)y, mean, rstd, rows, cols, eps); \
     return launch_status();                                                                                                    \
   }
-    if (cols > 1536) NX_FWD_REG(16, true)
-    if (cols > 1024) NX_FWD_REG(12, true)
-    if (cols % 128 != 0) NX_FWD_REG(8, true)
+    if (cols > 1536 && keep) NX_FWD_REG(16, true, true)
+    if (cols > 1536) NX_FWD_REG(16, true, false)
+    if (cols > 1024 && keep) NX_FWD_REG(12, true, true)
+    if (cols > 1024) NX_FWD_REG(12, true, false)
+    if (cols % 128 != 0) NX_FWD_REG(8, true, true)
     switch (cols / 128) {
-      case 1: NX_FWD_REG(1, false)
-      case 2: NX_FWD_REG(2, false)
-      case 3: NX_FWD_REG(3, false)
-      case 4: NX_FWD_REG(4, false)
-      case 5: NX_FWD_REG(5, false)
-      case 6: NX_FWD_REG(6, false)
-      case 7: NX_FWD_REG(7, false)
-      default: NX_FWD_REG(8, false)
+      case 1: NX_FWD_REG(1, false, true)
+      case 2: NX_FWD_REG(2, false, true)
+      case 3: NX_FWD_REG(3, false, true)
+      case 4: NX_FWD_REG(4, false, true)
+      case 5: NX_FWD_REG(5, false, true)
+      case 6: NX_FWD_REG(6, false, true)
+      case 7: NX_FWD_REG(7, false, true)
+      default: NX_FWD_REG(8, false, true)
     }
 #undef NX_FWD_REG
   }
