@@ -168,10 +168,11 @@ def test_mx_linear_gradients_close_to_fp32():
     K.check_status()
 
 
-@pytest.mark.parametrize("rows,cols,ld", [(1, 8, 8), (127, 129, 136), (128, 128, 128), (300, 264, 272), (1040, 33, 40), (31, 4096, 4096)])
+@pytest.mark.parametrize("rows,cols,ld", [(1, 8, 8), (127, 129, 136), (128, 128, 128), (300, 264, 272), (1040, 33, 40), (31, 4096, 4096),
+                                          (48, 144, 152), (32, 129, 136), (64, 33, 40), (1040, 1016, 1024), (1041, 3873, 3880), (1040, 3873, 3880)])
 def test_mx_quantize_both_forms_from_one_read(rows, cols, ld):
-    """Edges of the 128 x 128 tiles, odd widths inside a wider pitch, NaN and infinities: the bytes of the reference in both forms; rows
-    that lie on no 16 bytes take the general kernel and give the same."""
+    """Edges of the 128 x 128 tiles, odd widths inside a wider pitch, sizes on both sides of the lines between the kernels, NaN and
+    infinities: the bytes of the reference in both forms; rows that lie on no 16 bytes take the general kernel and give the same."""
     from nexus_b200.ops import _lowp as L
     torch.manual_seed(5)
     x = (torch.randn(rows, ld, device="cuda") * torch.logspace(-4, 4, ld, device="cuda")).bfloat16()[:, :cols]
